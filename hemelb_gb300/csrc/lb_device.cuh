@@ -282,36 +282,121 @@ __device__ __forceinline__ double feq64_one(double rho, double mx, double my, do
                         3. * mde);
 }
 
-__device__ __forceinline__ void collide64(const StepArgs& a, const double* f, double& rho,
-                                          double& mx, double& my, double& mz, double* fpost,
-                                          double omega, double omega_minus) {
+// The collision term by term, for states the fast form below does not take (a
+// density or momentum that is not finite, a density that is not positive): every
+// product by a lattice velocity component is formed, so a NaN or an infinity
+// spreads exactly as in the reference.
+static __device__ __noinline__ void collide64_general(int kernel, const double* f, double* mom, double* fpost,
+                                                      double omega, double omega_minus) {
   double r = 0.0, x = 0.0, y = 0.0, z = 0.0;
-#pragma unroll
   for (int i = 0; i < Q; ++i) {
     r += f[i];
-    x += (double)Lat::cx(i) * f[i];
-    y += (double)Lat::cy(i) * f[i];
-    z += (double)Lat::cz(i) * f[i];
+    x += (double)c_cx[i] * f[i];
+    y += (double)c_cy[i] * f[i];
+    z += (double)c_cz[i] * f[i];
+  }
+  mom[0] = r;
+  mom[1] = x;
+  mom[2] = y;
+  mom[3] = z;
+  if (kernel == 0) {
+    for (int i = 0; i < Q; ++i) fpost[i] = f[i] + (f[i] - feq64_one(r, x, y, z, i)) * omega;
+  } else {
+    fpost[0] = f[0] + omega * (f[0] - feq64_one(r, x, y, z, 0));
+    for (int i = 1; i < Q; i += 2) {
+      const double ni = f[i] - feq64_one(r, x, y, z, i), nb = f[i + 1] - feq64_one(r, x, y, z, i + 1);
+      const double sym = 0.5 * omega * (ni + nb);
+      const double asym = 0.5 * omega_minus * (ni - nb);
+      fpost[i] = f[i] + sym + asym;
+      fpost[i + 1] = f[i + 1] + sym - asym;
+    }
+  }
+}
+
+// Density and momentum in the reference's summation order without the terms whose
+// lattice velocity component is zero: for finite f such a term adds a zero to a sum
+// that is never -0 and leaves its bits alone (a sum of zeros only may differ in the
+// sign of zero, which no later result keeps).
+__device__ __forceinline__ void moments64(const double* f, double& rho, double& mx, double& my, double& mz) {
+  double r = f[0], x = f[1] - f[2], y = f[3] - f[4], z = f[5] - f[6];
+#pragma unroll
+  for (int i = 1; i < Q; ++i) r += f[i];
+#pragma unroll
+  for (int i = 7; i < Q; ++i) {
+    if (Lat::cx(i) > 0) x += f[i];
+    if (Lat::cx(i) < 0) x -= f[i];
+    if (Lat::cy(i) > 0) y += f[i];
+    if (Lat::cy(i) < 0) y -= f[i];
+    if (Lat::cz(i) > 0) z += f[i];
+    if (Lat::cz(i) < 0) z -= f[i];
   }
   rho = r;
   mx = x;
   my = y;
   mz = z;
-  double feq[Q];
-  feq64(rho, mx, my, mz, feq);
-  if (a.kernel == 0) {
+}
+
+// Whether the fast FP64 form takes a state: 0 < rho and rho, |m|^2 finite, tested on
+// the high words by the integer unit.
+__device__ __forceinline__ bool plain_state64(double rho, double m2) {
+  const int hr = __double2hiint(rho);
+  return hr > 0 && hr < 0x7ff00000 && (unsigned)__double2hiint(m2) < 0x7ff00000u;
+}
+
+// The same results bit for bit with about half the FP64 instructions.  GB300 issues
+// an FP64 warp instruction per SM only every 16 cycles or so (1.25 TFLOP/s nominal),
+// so this form is bound by their count: 200 a site for LBGK instead of 385 (moments
+// 45 instead of 103, equilibrium 97 instead of 225, relaxation 57; TRT 236 instead of
+// 421).  Opposite directions share c.m up to its sign, (4.5/rho)(c.m)^2, the sum with
+// rho - 1.5 m^2/rho and 3 c.m, each rounded as the reference rounds it; a product by
+// +-1 and a sum with a zero term are exact.
+__device__ __forceinline__ void collide64(const StepArgs& a, const double* f, double& rho,
+                                          double& mx, double& my, double& mz, double* fpost,
+                                          double omega, double omega_minus) {
+  moments64(f, rho, mx, my, mz);
+  const double m2 = mx * mx + my * my + mz * mz;
+  if (!plain_state64(rho, m2)) {  // copies, so that f and fpost stay in registers on the other path
+    double tf[Q], tp[Q], mom[4];
 #pragma unroll
-    for (int i = 0; i < Q; ++i) fpost[i] = f[i] + (f[i] - feq[i]) * omega;
-  } else {
-    fpost[0] = f[0] + omega * (f[0] - feq[0]);
+    for (int i = 0; i < Q; ++i) tf[i] = f[i];
+    collide64_general(a.kernel, tf, mom, tp, omega, omega_minus);
 #pragma unroll
-    for (int i = 1; i < Q; i += 2) {
-      const int ib = i + 1;
-      const double ni = f[i] - feq[i], nb = f[ib] - feq[ib];
-      const double sym = 0.5 * omega * (ni + nb);
-      const double asym = 0.5 * omega_minus * (ni - nb);
+    for (int i = 0; i < Q; ++i) fpost[i] = tp[i];
+    rho = mom[0];
+    mx = mom[1];
+    my = mom[2];
+    mz = mom[3];
+    return;
+  }
+  const double density_1 = 1. / rho;
+  const double base = rho - (3. / 2.) * m2 * density_1;
+  const double c45 = (9. / 2.) * density_1;
+  const bool lbgk = a.kernel == 0;
+  const double half_p = 0.5 * omega, half_m = 0.5 * omega_minus;
+  fpost[0] = f[0] + (f[0] - weight_d(0) * base) * omega;
+#pragma unroll
+  for (int i = 1; i < Q; i += 2) {
+    double mde = 0.0;
+    if (i == 1) mde = mx;
+    if (i == 3) mde = my;
+    if (i == 5) mde = mz;
+    if (i == 7) mde = mx + my;
+    if (i == 9) mde = mx - my;
+    if (i == 11) mde = mx + mz;
+    if (i == 13) mde = mx - mz;
+    if (i == 15) mde = my + mz;
+    if (i == 17) mde = my - mz;
+    const double even = base + c45 * mde * mde;
+    const double odd = 3. * mde;
+    const double ni = f[i] - weight_d(i) * (even + odd), nb = f[i + 1] - weight_d(i) * (even - odd);
+    if (lbgk) {
+      fpost[i] = f[i] + ni * omega;
+      fpost[i + 1] = f[i + 1] + nb * omega;
+    } else {
+      const double sym = half_p * (ni + nb);
+      const double asym = half_m * (ni - nb);
       fpost[i] = f[i] + sym + asym;
-      fpost[ib] = f[ib] + sym - asym;
+      fpost[i + 1] = f[i + 1] + sym - asym;
     }
   }
 }
