@@ -162,7 +162,6 @@ struct hlbg_ctx {
   uint64_t* d_b_links = nullptr;  // 3-bit link code per direction (see lb_device.cuh)
   float* d_b_normal = nullptr;      // wall normal per record
   double* d_wss = nullptr;          // wall shear stress output, allocated on first use
-  int32_t* d_rec_slot = nullptr;  // slot of each record
   std::vector<int32_t> h_new_of_old;  // device block index of each input block
   std::vector<uint16_t> h_site2slot;  // in-block slot of each local site (built by hlbg_halo_offsets)
   int32_t* d_halo_err = nullptr;      // out-of-range offsets seen by the halo pack / unpack
@@ -175,8 +174,9 @@ struct hlbg_ctx {
     }
   };
   std::map<GraphKey, cudaGraphExec_t> graphs;
-  int32_t* d_io_rec = nullptr;    // records with at least one iolet link
-  int64_t n_io_rec = 0;
+  int32_t* d_io_slot = nullptr;   // iolet links (StepArgs::io_slot, io_meta)
+  int32_t* d_io_meta = nullptr;
+  int64_t n_io_links = 0;
   int32_t* d_ref2slot = nullptr;
   int32_t* d_ps_slot = nullptr;
   int8_t* d_ps_dir = nullptr;
@@ -286,6 +286,9 @@ void fill_args(hlbg_ctx* ctx, StepArgs& a) {
   a.b_cut = ctx->d_b_cut;
   a.b_links = ctx->d_b_links;
   a.blk_omega = ctx->d_blk_omega;
+  a.io_slot = ctx->d_io_slot;
+  a.io_meta = ctx->d_io_meta;
+  a.n_io_links = ctx->n_io_links;
   a.iolets = ctx->d_iolets;
   a.n_in = (int32_t)ctx->inlets.size();
   a.kernel = ctx->params.kernel;
@@ -334,15 +337,6 @@ int launch_collide(hlbg_ctx* ctx, StepArgs& a, cudaStream_t st) {
     default: launch_stream_collide_2(a, ctx->d_block_xyz, st, ctx->sc_variant); break;
   }
   CK(cudaGetLastError());
-  // the all-slots kernel leaves iolet links to k_iolet_links; the list kernel does them itself
-  if (!a.list && ctx->n_io_rec > 0) {
-    switch (ctx->prec) {
-      case 0: launch_iolet_links_0(a, ctx->d_io_rec, ctx->d_rec_slot, ctx->n_io_rec, ctx->d_block_xyz, st); break;
-      case 1: launch_iolet_links_1(a, ctx->d_io_rec, ctx->d_rec_slot, ctx->n_io_rec, ctx->d_block_xyz, st); break;
-      default: launch_iolet_links_2(a, ctx->d_io_rec, ctx->d_rec_slot, ctx->n_io_rec, ctx->d_block_xyz, st); break;
-    }
-    CK(cudaGetLastError());
-  }
   return HLBG_OK;
 }
 
@@ -818,17 +812,20 @@ int build_layout(hlbg_ctx* ctx, const hlbg_geometry* g) {
   if (want_cut && (rc = upload(ctx, &ctx->d_b_cut, rcut))) return rc;
   if ((rc = upload(ctx, &ctx->d_b_links, rlinks))) return rc;
   if ((rc = upload(ctx, &ctx->d_b_normal, rnorm))) return rc;
-  if ((rc = upload(ctx, &ctx->d_rec_slot, ctx->h_rec_slot))) return rc;
   {
-    std::vector<int32_t> io_rec;
+    std::vector<int32_t> io_slot, io_meta;
+    if (ctx->inlets.size() + ctx->outlets.size() >= (size_t)1 << 26) return fail(ctx, HLBG_ERR_INVAL, "too many iolets");
     for (int64_t r = 0; r < ctx->nrec; ++r)
       for (int d = 1; d < 19; ++d)
         if (((rlinks[r] >> (3 * d)) & 7u) == HLBG_LC_IOLET) {
-          io_rec.push_back((int32_t)r);
-          break;
+          const bool inlet = rtype[r] == 2 || rtype[r] == 4;
+          const int32_t gi = inlet ? rid[r] : (int32_t)ctx->inlets.size() + rid[r];
+          io_slot.push_back(ctx->h_rec_slot[r]);
+          io_meta.push_back((int32_t)((uint32_t)gi << 5) | d);
         }
-    ctx->n_io_rec = (int64_t)io_rec.size();
-    if ((rc = upload(ctx, &ctx->d_io_rec, io_rec))) return rc;
+    ctx->n_io_links = (int64_t)io_slot.size();
+    if ((rc = upload(ctx, &ctx->d_io_slot, io_slot))) return rc;
+    if ((rc = upload(ctx, &ctx->d_io_meta, io_meta))) return rc;
   }
   if ((rc = upload(ctx, &ctx->d_ref2slot, ctx->h_ref2slot))) return rc;
   if ((rc = upload(ctx, &ctx->d_ps_slot, ctx->h_ps_slot))) return rc;
@@ -1078,7 +1075,7 @@ void hlbg_destroy(hlbg_ctx* ctx) {
   void* ptrs[] = {ctx->f[0],        ctx->f[1],        ctx->d_block_nbr, ctx->d_block_xyz,
                   ctx->d_site_code, ctx->d_block_bulk, ctx->d_b_wall,   ctx->d_b_iolet,
                   ctx->d_b_ioid,    ctx->d_b_type,    ctx->d_b_cut,     ctx->d_ref2slot, ctx->d_b_links,
-                  ctx->d_rec_slot,  ctx->d_io_rec,
+                  ctx->d_io_slot,   ctx->d_io_meta,
                   ctx->d_ps_slot,   ctx->d_ps_dir,    ctx->d_ps_q,      ctx->d_iolets,
                   ctx->d_io_tab,    ctx->d_stage,     ctx->d_stage_rho, ctx->d_stage_u,
                   ctx->d_list,      ctx->d_part,      ctx->d_part_bad,  ctx->d_steady,
@@ -1160,7 +1157,9 @@ int64_t hlbg_site_count(const hlbg_ctx* ctx) { return ctx ? ctx->nsites : 0; }
 int64_t hlbg_slot_count(const hlbg_ctx* ctx) { return ctx ? ctx->nslot : 0; }
 int32_t hlbg_launches_per_step(const hlbg_ctx* ctx) {
   if (!ctx) return 0;
-  return 1 + (ctx->n_io_rec > 0 ? 1 : 0) + (ctx->params.wall == HLBG_WALL_BFL && ctx->n_ps > 0 ? 1 : 0);
+  // the staged launches leave the iolet links to a launch of their own
+  const bool staged = ctx->prec != 0 && (ctx->sc_variant == 4 || ctx->sc_variant == 8) && ctx->d_pipe_desc;
+  return 1 + (staged && ctx->n_io_links > 0 ? 1 : 0) + (ctx->params.wall == HLBG_WALL_BFL && ctx->n_ps > 0 ? 1 : 0);
 }
 size_t hlbg_device_bytes(const hlbg_ctx* ctx) { return ctx ? ctx->dev_bytes : 0; }
 

@@ -178,6 +178,13 @@ struct StepArgs {
   const uint64_t* b_links;  // [nrec] 3-bit link code per direction (HLBG_LC_*)
   const int32_t* list;  // optional slot list (per-range drop-in), null = all slots
   int64_t list_count;
+  // Iolet links (Nash / Ladd), one thread each: link k belongs to the site in slot
+  // io_slot[k], direction io_meta[k] & 31, iolet io_meta[k] >> 5 (inlets first).  The
+  // first io_ctas CTAs of a stream-and-collide launch take them.
+  const int32_t* io_slot;
+  const int32_t* io_meta;
+  int64_t n_io_links;
+  uint32_t io_ctas;
   const IoletDev* iolets;     // [n_in + n_out]
   const double* iolet_rho;    // [n_in + n_out] ghost density for this step (Nash)
   const double* iolet_umax;   // [n_in + n_out] peak speed for this step (Ladd)

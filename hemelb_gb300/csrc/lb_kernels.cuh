@@ -34,12 +34,11 @@ struct Calc<0> {
 
 // ---------------------------------------------------------------------------
 // Value an iolet link writes into the site's own inverse-direction slot:
-// Nash (NashZerothOrderPressure.h:388-421) or Ladd (LaddIolet.h:465-502).  Out of
-// line with scalar arguments: iolet links are a fraction of a percent of links.
+// Nash (NashZerothOrderPressure.h:388-421) or Ladd (LaddIolet.h:465-502).
 // m0 is the density (FP64 form) or the density deviation (FP32 / FP16 forms).
 // ---------------------------------------------------------------------------
 template <int P>
-__device__ __noinline__ typename Calc<P>::T iolet_link_value(
+__device__ __forceinline__ typename Calc<P>::T iolet_link_value(
     const StepArgs& a, int gi, int model, int d, typename Calc<P>::T fpost_d,
     typename Calc<P>::T m0, typename Calc<P>::T mx, typename Calc<P>::T my,
     typename Calc<P>::T mz, int gx, int gy, int gz) {
@@ -69,6 +68,15 @@ __device__ __noinline__ typename Calc<P>::T iolet_link_value(
   } else {
     return fpost_d - ladd_correction32(io, (float)a.iolet_umax[gi], 1.f + m0, gx, gy, gz, d);
   }
+}
+
+// The same out of line, for the per-site dispatch of BoundaryAll (19 call sites).
+template <int P>
+__device__ __noinline__ typename Calc<P>::T iolet_link_value_call(
+    const StepArgs& a, int gi, int model, int d, typename Calc<P>::T fpost_d,
+    typename Calc<P>::T m0, typename Calc<P>::T mx, typename Calc<P>::T my,
+    typename Calc<P>::T mz, int gx, int gy, int gz) {
+  return iolet_link_value<P>(a, gi, model, d, fpost_d, m0, mx, my, mz, gx, gy, gz);
 }
 
 // Entry k of the 27-block table around a site's block (neighbour block index,
@@ -142,7 +150,7 @@ struct BoundaryAll {
       const int gi = is_inlet ? ioid : a.n_in + ioid;
       const int model = is_inlet ? a.inlet_model : a.outlet_model;
       const int64_t b = s >> 9;
-      const T v = iolet_link_value<P>(a, gi, model, D, fpost[D], m0, mx, my, mz,
+      const T v = iolet_link_value_call<P>(a, gi, model, D, fpost[D], m0, mx, my, mz,
                                       block_xyz[3 * b] * 8 + x, block_xyz[3 * b + 1] * 8 + y,
                                       block_xyz[3 * b + 2] * 8 + z);
       Store<P>::store(fn + own, inv * kSites + l, v, a);
@@ -264,7 +272,7 @@ struct PushMixed {
           const T q = (T)a.b_cut[r * (Q - 1) + D - 1];
           v = (fpost[D] + ((T)2.0 * q - (T)1) * fpost[inv]) / ((T)2.0 * q);
         }
-        if (lc == HLBG_LC_IOLET) st = false;  // written by k_iolet_links
+        if (lc == HLBG_LC_IOLET) st = false;  // written by iolet_link
       }
     }
     if (st) Store<P>::store(fn, off, v, a);
@@ -477,31 +485,31 @@ __device__ __forceinline__ MonAccT<P> mon_neutral_t() {
 // 32-bit words [sum (rho-1) | max |du| | min f | min (rho-1) | max (rho-1) | max |u|
 // | count | unstable] in the same buffer, converted to FP64 by the second stage.
 template <int P>
-__device__ __forceinline__ void mon_write_partial(const StepArgs& a, const MonAccT<P>& acc) {
+__device__ __forceinline__ void mon_write_partial(const StepArgs& a, const MonAccT<P>& acc, unsigned cta) {
   const int64_t n = a.mon_nparts;
   if constexpr (P == 0) {
     const MonAcc r = mon_block(acc);
     if (threadIdx.x == 0) {
-      a.mon_part[blockIdx.x] = r.mass;
-      a.mon_part[n + blockIdx.x] = r.maxdu;
-      a.mon_part[2 * n + blockIdx.x] = r.minf;
-      a.mon_part[3 * n + blockIdx.x] = (double)r.bad;
-      a.mon_part[4 * n + blockIdx.x] = r.rmin;
-      a.mon_part[5 * n + blockIdx.x] = r.rmax;
-      a.mon_part[6 * n + blockIdx.x] = r.umax;
+      a.mon_part[cta] = r.mass;
+      a.mon_part[n + cta] = r.maxdu;
+      a.mon_part[2 * n + cta] = r.minf;
+      a.mon_part[3 * n + cta] = (double)r.bad;
+      a.mon_part[4 * n + cta] = r.rmin;
+      a.mon_part[5 * n + cta] = r.rmax;
+      a.mon_part[6 * n + cta] = r.umax;
     }
   } else {
     const MonAccF r = mon_block_f(acc);
     if (threadIdx.x == 0) {
       float* p = reinterpret_cast<float*>(a.mon_part);
-      p[blockIdx.x] = r.dm;
-      p[n + blockIdx.x] = sqrtf(r.maxdu);
-      p[2 * n + blockIdx.x] = r.minf;
-      p[3 * n + blockIdx.x] = r.dmin;
-      p[4 * n + blockIdx.x] = r.dmax;
-      p[5 * n + blockIdx.x] = sqrtf(r.umax);
-      p[6 * n + blockIdx.x] = __uint_as_float(r.count);
-      p[7 * n + blockIdx.x] = __uint_as_float(r.bad);
+      p[cta] = r.dm;
+      p[n + cta] = sqrtf(r.maxdu);
+      p[2 * n + cta] = r.minf;
+      p[3 * n + cta] = r.dmin;
+      p[4 * n + cta] = r.dmax;
+      p[5 * n + cta] = sqrtf(r.umax);
+      p[6 * n + cta] = __uint_as_float(r.count);
+      p[7 * n + cta] = __uint_as_float(r.bad);
     }
   }
 }
@@ -533,6 +541,58 @@ __device__ __forceinline__ void site_update(const StepArgs& a, const B& base,
   const int64_t r = code - 2;
   BoundaryAll<P, 0>::run(fn, a, base, s, l >> 6, (l >> 3) & 7, l & 7, a.b_wall[r], a.b_iolet[r],
                          (int)a.b_type[r], a.b_ioid[r], r, fpost, m0, mx, my, mz, block_xyz);
+}
+
+// One iolet link (Nash / Ladd): the value streamed into the site's own inverse-
+// direction slot, from the site's state in f_old with the arithmetic of the
+// collision.  The slot has no other writer, so links may run before, after or beside
+// the update's other CTAs: they are the first CTAs of its launch.  One thread per
+// link (about five links a site), because a site's links in one thread are a serial
+// chain of FP64 operations on a handful of SMs: as a launch of its own with one thread
+// per site this took 36 us beside 38 us of the pipe's update (25k sites, FP64) and 20
+// beside 569 us of the 16.9M-site tree's (FP32).  A Nash link needs the moments only.
+template <int P>
+__device__ __forceinline__ void iolet_link(const StepArgs& a, int64_t i, const int32_t* __restrict__ block_xyz) {
+  using St = Store<P>;
+  using S = typename St::S;
+  using T = typename Calc<P>::T;
+  if (i >= a.n_io_links) return;
+  const int64_t s = __ldg(a.io_slot + i);
+  const int meta = __ldg(a.io_meta + i);
+  const int d = meta & 31, gi = meta >> 5;
+  const int64_t b = s >> 9;
+  const int j = (int)(s & (kSites - 1));
+  const S* fo = static_cast<const S*>(a.f_old) + b * (Q * kSites) + j;
+  S* fn = static_cast<S*>(a.f_new) + b * (Q * kSites) + j;
+  const int ls = site_of_slot(a, s, (__ldg(a.block_nbr + b * 27 + 13) & kPackedBit) != 0);
+  const int gx = block_xyz[3 * b] * 8 + (ls >> 6), gy = block_xyz[3 * b + 1] * 8 + ((ls >> 3) & 7),
+            gz = block_xyz[3 * b + 2] * 8 + (ls & 7);
+  T f[Q], fpost[Q];
+#pragma unroll
+  for (int k = 0; k < Q; ++k) f[k] = St::load(fo, k * kSites, a);
+  T m0, mx, my, mz, fp = (T)0;
+  const int model = gi < a.n_in ? a.inlet_model : a.outlet_model;
+  bool full = true;
+  if constexpr (P == 0) {
+    if (model == 0) {
+      moments64(f, m0, mx, my, mz);
+      full = !plain_state64(m0, mx * mx + my * my + mz * mz);
+    }
+  }
+  if (full) {
+    collide_any<P>(a, b, f, m0, mx, my, mz, fpost);
+#pragma unroll
+    for (int k = 1; k < Q; ++k)
+      if (k == d) fp = fpost[k];
+  }
+  const T v = iolet_link_value<P>(a, gi, model, d, fp, m0, mx, my, mz, gx, gy, gz);
+  St::store(fn, c_inv[d] * kSites, v, a);
+}
+
+// Iolet links as a launch of their own, beside the staged launches (indices 4 and 8).
+template <int P>
+__global__ void __launch_bounds__(128) k_iolet_links(StepArgs a, const int32_t* __restrict__ block_xyz) {
+  iolet_link<P>(a, (int64_t)blockIdx.x * 128 + threadIdx.x, block_xyz);
 }
 
 // One warp's 32 slots of one block (a warp never spans two blocks).  Lanes 0..26
@@ -675,11 +735,16 @@ __device__ __forceinline__ void collide_listed_warp(const StepArgs& a, int64_t w
 
 template <int P, int THREADS, int MINB, bool MON>
 __global__ void __launch_bounds__(THREADS, MINB) k_stream_collide_listed(StepArgs a, const int32_t* block_xyz) {
+  if (blockIdx.x < a.io_ctas) {  // whole CTA
+    iolet_link<P>(a, (int64_t)blockIdx.x * THREADS + threadIdx.x, block_xyz);
+    return;
+  }
+  const unsigned cta = blockIdx.x - a.io_ctas;
   MonAccT<P> acc = mon_neutral_t<P>();
   bool check = false;
   if constexpr (MON) check = *a.mon_state != 0;
-  collide_listed_warp<P, MON>(a, ((int64_t)blockIdx.x * THREADS + threadIdx.x) >> 5, block_xyz, acc, check);
-  if constexpr (MON) mon_write_partial<P>(a, acc);
+  collide_listed_warp<P, MON>(a, ((int64_t)cta * THREADS + threadIdx.x) >> 5, block_xyz, acc, check);
+  if constexpr (MON) mon_write_partial<P>(a, acc, cta);
 }
 
 // ---------------------------------------------------------------------------
@@ -1044,7 +1109,15 @@ void launch_pipe(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
 template <int P, int THREADS, int MINB, bool MON>
 void launch_listed(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
   const int64_t g = (a.n_warps * 32 + THREADS - 1) / THREADS;
-  if (g) k_stream_collide_listed<P, THREADS, MINB, MON><<<(unsigned)g, THREADS, 0, st>>>(a, bxyz);
+  StepArgs b = a;
+  b.io_ctas = (uint32_t)((a.n_io_links + THREADS - 1) / THREADS);
+  if (g) k_stream_collide_listed<P, THREADS, MINB, MON><<<(unsigned)g + b.io_ctas, THREADS, 0, st>>>(b, bxyz);
+}
+
+template <int P>
+void launch_iolets(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
+  const unsigned g = (unsigned)((a.n_io_links + 127) / 128);
+  if (g) k_iolet_links<P><<<g, 128, 0, st>>>(a, bxyz);
 }
 
 // Fluid-list shape of launch variant 7: 64-thread CTAs, 16 per SM (the 32
@@ -1059,11 +1132,16 @@ void launch_listed(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
 template <int P, int THREADS, int MINB, bool MON>
 __global__ void __launch_bounds__(THREADS, MINB)
     k_stream_collide(StepArgs a, const int32_t* block_xyz) {
+  if (blockIdx.x < a.io_ctas) {  // whole CTA
+    iolet_link<P>(a, (int64_t)blockIdx.x * THREADS + threadIdx.x, block_xyz);
+    return;
+  }
+  const unsigned cta = blockIdx.x - a.io_ctas;
   MonAccT<P> acc = mon_neutral_t<P>();
   bool check = false;
   if constexpr (MON) check = *a.mon_state != 0;
-  collide_slot<P, MON>(a, (int64_t)blockIdx.x * THREADS + threadIdx.x, block_xyz, acc, check);
-  if constexpr (MON) mon_write_partial<P>(a, acc);
+  collide_slot<P, MON>(a, (int64_t)cta * THREADS + threadIdx.x, block_xyz, acc, check);
+  if constexpr (MON) mon_write_partial<P>(a, acc, cta);
 }
 
 // Second stage of the fused StabilityTester's reduction: CTA c folds partials
@@ -1145,51 +1223,6 @@ __global__ void __launch_bounds__(256) k_stream_collide_list(StepArgs a, const i
   if (code == 0) return;
   const int32_t* tab = a.block_nbr + b * 27;
   site_update<P>(a, GlobalBase{tab}, tab, s, code, block_xyz);
-}
-
-// Iolet links (Nash / Ladd) of the sites listed in `rec`: the site's collision is
-// recomputed from f_old with the same arithmetic as k_stream_collide, and each iolet
-// link writes the site's own inverse-direction slot.  These slots have no other
-// writer, so this launch and k_stream_collide may run in either order.
-template <int P>
-__global__ void __launch_bounds__(128) k_iolet_links(StepArgs a, const int32_t* __restrict__ rec,
-                                                     const int32_t* __restrict__ rec_slot, int64_t n,
-                                                     const int32_t* __restrict__ block_xyz) {
-  using St = Store<P>;
-  using S = typename St::S;
-  using T = typename Calc<P>::T;
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int64_t r = rec[i];
-  const int64_t s = rec_slot[r];
-  const int64_t b = s >> 9;
-  const int l = (int)(s & (kSites - 1));
-  const S* fo = static_cast<const S*>(a.f_old) + b * (Q * kSites) + l;
-  S* fn = static_cast<S*>(a.f_new) + b * (Q * kSites) + l;
-  T f[Q], fpost[Q];
-#pragma unroll
-  for (int d = 0; d < Q; ++d) f[d] = St::load(fo, d * kSites, a);
-  T m0, mx, my, mz;
-  collide_any<P>(a, b, f, m0, mx, my, mz, fpost);
-  const uint64_t links = a.b_links[r];
-  const int type = a.b_type[r];
-  const int ioid = a.b_ioid[r];
-  const bool is_inlet = (type == 2 || type == 4);
-  const int gi = is_inlet ? ioid : a.n_in + ioid;
-  const int model = is_inlet ? a.inlet_model : a.outlet_model;
-  const int ls = site_of_slot(a, s, (__ldg(a.block_nbr + b * 27 + 13) & kPackedBit) != 0);
-  const int gx = block_xyz[3 * b] * 8 + (ls >> 6), gy = block_xyz[3 * b + 1] * 8 + ((ls >> 3) & 7),
-            gz = block_xyz[3 * b + 2] * 8 + (ls & 7);
-#pragma unroll 1
-  for (int d = 1; d < Q; ++d) {
-    if (((links >> (3 * d)) & 7u) != HLBG_LC_IOLET) continue;
-    T fp = fpost[0];
-#pragma unroll
-    for (int e = 1; e < Q; ++e)
-      if (e == d) fp = fpost[e];
-    const T v = iolet_link_value<P>(a, gi, model, d, fp, m0, mx, my, mz, gx, gy, gz);
-    St::store(fn, c_inv[d] * kSites, v, a);
-  }
 }
 
 // BouzidiFirdaousLallemandLink::PostStepLink (BouzidiFirdaousLallemand.h:336-357)
@@ -1576,7 +1609,9 @@ namespace hlbg {
 template <int P, int THREADS, int MINB, bool MON = false>
 void launch_sc(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
   const unsigned g = (unsigned)(a.nslot / THREADS);
-  if (g) k_stream_collide<P, THREADS, MINB, MON><<<g, THREADS, 0, st>>>(a, bxyz);
+  StepArgs b = a;
+  b.io_ctas = (uint32_t)((a.n_io_links + THREADS - 1) / THREADS);
+  if (g) k_stream_collide<P, THREADS, MINB, MON><<<g + b.io_ctas, THREADS, 0, st>>>(b, bxyz);
 }
 }  // namespace hlbg
 
@@ -1631,6 +1666,7 @@ __global__ void k_halo_unpack(void* f, const int64_t* off, int64_t n, int64_t li
       if constexpr (P != 0) {                                                                   \
         if (a.blk_runs) {                                                                       \
           launch_block_staged<P, 256, 4>(a, bxyz, st);                                          \
+          launch_iolets<P>(a, bxyz, st);                                                        \
           return;                                                                               \
         }                                                                                       \
       }                                                                                         \
@@ -1640,6 +1676,7 @@ __global__ void k_halo_unpack(void* f, const int64_t* off, int64_t n, int64_t li
       if constexpr (P != 0) {                                                                   \
         if (a.pipe_desc && !a.mon_u) {                                                          \
           launch_pipe<P, HLBG_PIPE_NCW, (P == 1 ? HLBG_PIPE_STAGES : 2 * HLBG_PIPE_STAGES)>(a, bxyz, st); \
+          launch_iolets<P>(a, bxyz, st);                                                        \
           return;                                                                               \
         }                                                                                       \
       }                                                                                         \
@@ -1696,11 +1733,6 @@ __global__ void k_halo_unpack(void* f, const int64_t* off, int64_t n, int64_t li
     const int64_t per = (nparts + n2 - 1) / n2;                                                 \
     k_mon_stage2<<<(unsigned)n2, 256, 0, st>>>(part, nparts, per, part2, n2, P != 0);           \
     k_mon_final<<<1, 256, 0, st>>>(part2, n2, mon_state, result, sa, steady);                   \
-  }                                                                                             \
-  void launch_iolet_links_##P(const StepArgs& a, const int32_t* rec, const int32_t* rec_slot,    \
-                              int64_t n, const int32_t* bxyz, cudaStream_t st) {                \
-    unsigned g = (unsigned)((n + 127) / 128);                                                   \
-    if (g) k_iolet_links<P><<<g, 128, 0, st>>>(a, rec, rec_slot, n, bxyz);                      \
   }                                                                                             \
   void launch_post_step_##P(const PostArgs& p, cudaStream_t st) {                               \
     unsigned g = (unsigned)((p.count + 255) / 256);                                             \

@@ -211,7 +211,8 @@ const char *hlbg_last_error(const hlbg_ctx *ctx);
 
 int64_t hlbg_site_count(const hlbg_ctx *ctx);   /* fluid sites N */
 int64_t hlbg_slot_count(const hlbg_ctx *ctx);   /* device slots (n_blocks * 512) */
-/* Kernel launches one hlbg_step time step makes (stream-collide, iolet links, BFL PostStep). */
+/* Kernel launches one hlbg_step time step makes: stream-collide (the iolet links are its
+ * first CTAs; a launch of their own beside the staged shapes 4 and 8), BFL PostStep. */
 int32_t hlbg_launches_per_step(const hlbg_ctx *ctx);
 int hlbg_collision_counts(const hlbg_ctx *ctx, int64_t counts[6]);
 size_t hlbg_device_bytes(const hlbg_ctx *ctx);
