@@ -135,6 +135,15 @@ def bias_grad(dy, db):
     _ok(_lib().hlbg_nn_bias_grad(_p(dy), _p(db), dy.numel() // c, c, _stream()), "hlbg_nn_bias_grad")
 
 
+def relu_bias_backward(dy, y, db):
+    """relu_backward and bias_grad in one pass over dy."""
+    _need(dy, _BF16, "relu dy")
+    _need(y, _BF16, "relu y")
+    _need(db, _F32, "bias gradient")
+    c = dy.shape[-1]
+    _ok(_lib().hlbg_nn_relu_bias_bwd(_p(dy), _p(y), _p(db), dy.numel() // c, c, _stream()), "hlbg_nn_relu_bias_bwd")
+
+
 def pool2(x, y):
     _need(x, _BF16, "pool input")
     _need(y, _BF16, "pool output")
@@ -147,6 +156,53 @@ def pool2_backward(dy, dx):
     _need(dy, _BF16, "pool dy")
     _need(dx, _BF16, "pool dx")
     _ok(_lib().hlbg_nn_pool2(_p(dy), _p(dx), n, d, h, w, c, 1, _stream()), "hlbg_nn_pool2")
+
+
+def _fused(c, d, h, w, *tensors):
+    """Shapes the fused up/down-sampling passes take."""
+    return (all(k % 8 == 0 for k in c) and d % 2 == h % 2 == w % 2 == 0
+            and all(t.data_ptr() % 16 == 0 and 0 < t.numel() < 1 << 33 for t in tensors))
+
+
+def pool2_backward_add(dy, acc):
+    """acc += the gradient of pool2 (rounded to BF16, then added)."""
+    n, d, h, w, c = acc.shape
+    _need(dy, _BF16, "pool dy")
+    _need(acc, _BF16, "pool sum")
+    if not _fused((c,), d, h, w, dy, acc):
+        tmp = torch.empty(acc.shape, dtype=_BF16, device=acc.device)
+        pool2_backward(dy, tmp)
+        add_(acc, tmp)
+        return
+    _ok(_lib().hlbg_nn_pool2_bwd_add(_p(dy), _p(acc), n, d, h, w, c, _stream()), "hlbg_nn_pool2_bwd_add")
+
+
+def up2_concat(x, skip, y):
+    """y = [up2(x) | skip] in one pass."""
+    n, d, h, w, cb = skip.shape
+    ca = x.shape[-1]
+    for t, what in ((x, "upsample input"), (skip, "concat skip"), (y, "concat y")):
+        _need(t, _BF16, what)
+    if not _fused((ca, cb), d, h, w, x, skip, y):
+        u = torch.empty((n, d, h, w, ca), dtype=_BF16, device=x.device)
+        up2(x, u)
+        concat(u, skip, y)
+        return
+    _ok(_lib().hlbg_nn_up2_concat(_p(x), ca, _p(skip), cb, _p(y), n, d, h, w, _stream()), "hlbg_nn_up2_concat")
+
+
+def up2_split(dy, dx, dskip):
+    """The gradient of up2_concat: dx = up2_backward of dy's first channels, dskip the rest."""
+    n, d, h, w, cb = dskip.shape
+    ca = dx.shape[-1]
+    for t, what in ((dy, "split y"), (dx, "upsample dx"), (dskip, "split skip")):
+        _need(t, _BF16, what)
+    if not _fused((ca, cb), d, h, w, dy, dx, dskip):
+        g = torch.empty((n, d, h, w, ca), dtype=_BF16, device=dy.device)
+        split(dy, g, dskip)
+        up2_backward(g, dx)
+        return
+    _ok(_lib().hlbg_nn_up2_split(_p(dy), _p(dx), ca, _p(dskip), cb, n, d, h, w, _stream()), "hlbg_nn_up2_split")
 
 
 def up2(x, y):

@@ -241,8 +241,9 @@ class Conv:
 
     def backward(self, dy, need_dx=True):
         if self.relu:
-            nn.relu_backward(dy, self.y)
-        nn.bias_grad(dy, self.gb)
+            nn.relu_bias_backward(dy, self.y, self.gb)
+        else:
+            nn.bias_grad(dy, self.gb)
         nn.conv3d_weight_grad(self.x, dy, self.gw)
         dx = None
         if need_dx:
@@ -305,10 +306,8 @@ class UNet:
     @staticmethod
     def _up_cat(x, skip):
         n, d, h, w, c = skip.shape
-        u = torch.empty((n, d, h, w, x.shape[-1]), dtype=torch.bfloat16, device=x.device)
-        nn.up2(x, u)
         y = torch.empty((n, d, h, w, x.shape[-1] + c), dtype=torch.bfloat16, device=x.device)
-        nn.concat(u, skip, y)
+        nn.up2_concat(x, skip, y)
         return y
 
     def forward(self, x):
@@ -327,18 +326,9 @@ class UNet:
     @staticmethod
     def _split_up(g, x_shape, skip_grad):
         """Gradient of concat(up2(x), skip): returns dx and writes the skip part."""
-        n, d, h, w, _ = skip_grad.shape
-        gu = torch.empty((n, d, h, w, x_shape[-1]), dtype=torch.bfloat16, device=g.device)
-        nn.split(g, gu, skip_grad)
         gx = torch.empty(x_shape, dtype=torch.bfloat16, device=g.device)
-        nn.up2_backward(gu, gx)
+        nn.up2_split(g, gx, skip_grad)
         return gx
-
-    @staticmethod
-    def _pool_back_add(g, acc):
-        tmp = torch.empty(acc.shape, dtype=torch.bfloat16, device=g.device)
-        nn.pool2_backward(g, tmp)
-        nn.add_(acc, tmp)
 
     def backward(self, dout):
         """dout: BF16 gradient of the loss w.r.t. the FP32 output; accumulates the
@@ -355,11 +345,11 @@ class UNet:
         ge2 = torch.empty_like(e2)
         g = self._split_up(g, b.shape, ge2)
         g = L["ba"].backward(L["bb"].backward(g))
-        self._pool_back_add(g, ge2)
+        nn.pool2_backward_add(g, ge2)
         g = L["e2a"].backward(L["e2b"].backward(ge2))
-        self._pool_back_add(g, ge1)
+        nn.pool2_backward_add(g, ge1)
         g = L["e1a"].backward(L["e1b"].backward(ge1))
-        self._pool_back_add(g, ge0)
+        nn.pool2_backward_add(g, ge0)
         L["e0a"].backward(L["e0b"].backward(ge0), need_dx=False)
         self._saved = None
 

@@ -41,6 +41,8 @@ int hlbg_nn_flip_transpose(const void *w, void *wt, int32_t cout, int32_t cin, i
                            void *stream);
 int hlbg_nn_relu_bwd(void *dy, const void *y, int64_t n, void *stream);
 int hlbg_nn_bias_grad(const void *dy, float *db, int64_t m, int32_t c, void *stream);
+/* The two above in one pass over dy: dy *= (y > 0), then db[c] += sum_m dy[m, c]. */
+int hlbg_nn_relu_bias_bwd(void *dy, const void *y, float *db, int64_t m, int32_t c, void *stream);
 /* 2x average pooling; backward: x = dy (coarse), y = dx (fine), sizes fine */
 int hlbg_nn_pool2(const void *x, void *y, int32_t n, int32_t d, int32_t h, int32_t w, int32_t c,
                   int32_t backward, void *stream);
@@ -51,6 +53,16 @@ int hlbg_nn_concat(const void *a, int32_t ca, const void *b, int32_t cb, void *y
                    void *stream);
 int hlbg_nn_split(const void *y, void *da, int32_t ca, void *db, int32_t cb, int64_t m,
                   int32_t accumulate_b, void *stream);
+/* Upsampling and concatenation in one pass, y = [up2(x) | skip], and its gradient
+ * (dx = sum of the 8 copies, dskip); and acc += pool2 gradient of dy.  d, h, w are the
+ * fine sizes, even; channel counts are multiples of 8 and every buffer is 16-byte
+ * aligned, else 1 (the single passes above and below take every shape). */
+int hlbg_nn_up2_concat(const void *x, int32_t ca, const void *skip, int32_t cb, void *y, int32_t n,
+                       int32_t d, int32_t h, int32_t w, void *stream);
+int hlbg_nn_up2_split(const void *dy, void *dx, int32_t ca, void *dskip, int32_t cb, int32_t n,
+                      int32_t d, int32_t h, int32_t w, void *stream);
+int hlbg_nn_pool2_bwd_add(const void *dy, void *acc, int32_t n, int32_t d, int32_t h, int32_t w,
+                          int32_t c, void *stream);
 int hlbg_nn_add(void *a, const void *b, int64_t n, void *stream);
 /* masked MSE: loss += sum (mask (pred - target))^2, dpred = 2 mask (pred - target) * inv_count */
 int hlbg_nn_mse(const float *pred, const float *target, const float *mask, void *dpred, float *loss,
