@@ -208,6 +208,7 @@ struct hlbg_ctx {
   void* d_mon_u = nullptr;
   double* d_mon_part = nullptr;
   double* d_mon_part2 = nullptr;
+  uint32_t* d_mon_tick = nullptr;
   int32_t* d_mon_state = nullptr;
   double* d_mon_result = nullptr;
   double* h_mon_result = nullptr;  // pinned
@@ -218,7 +219,7 @@ struct hlbg_ctx {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   size_t dev_bytes = 0;
   float fp16_scale = 1024.f;
-  int sc_variant = 0;  // chosen by hlbg_autotune
+  int sc_variant = 6;  // launch shape (default_variant; hlbg_set_launch_variant, hlbg_autotune)
   bool initialised = false;
 };
 
@@ -834,9 +835,9 @@ int build_layout(hlbg_ctx* ctx, const hlbg_geometry* g) {
   return HLBG_OK;
 }
 
-constexpr int64_t kMonStage2 = 1024;
 constexpr int kMonFields = 7;  // partials: mass, max |du|, min f, unstable, min rho, max rho, max |u|
 constexpr int kMonResult = 8;  // the same plus the valid flag
+constexpr int64_t kMonGroupCtas = 64;  // CTAs per group of the reduction (mon_finish)
 
 // Buffers of the fused StabilityTester, allocated on first use.
 int mon_prepare(hlbg_ctx* ctx) {
@@ -846,11 +847,14 @@ int mon_prepare(hlbg_ctx* ctx) {
   int rc = dev_alloc(ctx, &u, 3 * (size_t)ctx->nslot * es);
   if (rc) return rc;
   ctx->d_mon_u = u;
-  // one partial per CTA of 128 or more threads, for every launch shape: all slots,
-  // or the fluid list (whose padded warps can outnumber a block's 16)
-  const int64_t max_ctas = (std::max(ctx->nslot, ctx->n_warps * 32) + 127) / 128;
+  // one partial per CTA, for every launch shape: all slots in CTAs of 128 or more
+  // threads, or the fluid list (FP64: one warp per CTA, else four)
+  const int64_t max_ctas = std::max((ctx->nslot + 127) / 128, ctx->prec == 0 ? ctx->n_warps : (ctx->n_warps + 3) / 4);
+  const int64_t max_groups = (max_ctas + kMonGroupCtas - 1) / kMonGroupCtas;
   if ((rc = dev_alloc(ctx, &ctx->d_mon_part, kMonFields * (size_t)max_ctas))) return rc;
-  if ((rc = dev_alloc(ctx, &ctx->d_mon_part2, kMonFields * (size_t)kMonStage2))) return rc;
+  if ((rc = dev_alloc(ctx, &ctx->d_mon_part2, kMonFields * (size_t)max_groups))) return rc;
+  if ((rc = dev_alloc(ctx, &ctx->d_mon_tick, (size_t)max_groups + 1))) return rc;
+  CK(cudaMemsetAsync(ctx->d_mon_tick, 0, ((size_t)max_groups + 1) * sizeof(uint32_t), ctx->stream));
   if ((rc = dev_alloc(ctx, &ctx->d_mon_state, 1))) return rc;
   if ((rc = dev_alloc(ctx, &ctx->d_mon_result, kMonResult))) return rc;
   CK(cudaMemsetAsync(ctx->d_mon_result, 0, kMonResult * sizeof(double), ctx->stream));  // no check yet
@@ -878,26 +882,19 @@ int64_t monitored_grid(const hlbg_ctx* ctx) {
   }
 }
 
-// Monitor fields of a step's arguments (the kernel then records velocities and
-// writes one partial per CTA).
-void mon_args(hlbg_ctx* ctx, StepArgs& a) {
+// Monitor fields of a step's arguments: the kernel records velocities and, with
+// `fold`, compares and reduces them (steady: counts the check).
+void mon_args(hlbg_ctx* ctx, StepArgs& a, bool fold, bool steady) {
   a.mon_u = ctx->d_mon_u;
   a.mon_part = ctx->d_mon_part;
   a.mon_nparts = monitored_grid(ctx);
+  a.mon_part2 = ctx->d_mon_part2;
+  a.mon_tick = ctx->d_mon_tick;
   a.mon_state = ctx->d_mon_state;
-}
-
-// The two reduction stages after a monitored step (steady: count the check).
-int mon_reduce(hlbg_ctx* ctx, const StepArgs& a, bool steady, cudaStream_t st) {
-  const int64_t n2 = std::min<int64_t>(kMonStage2, a.mon_nparts);
-  SteadyArgs sa{ctx->d_steady, ctx->d_steady ? ctx->d_steady + 1 : nullptr, ctx->d_steady_n};
-  switch (ctx->prec) {
-    case 0: launch_mon_reduce_0(a.mon_part, a.mon_nparts, ctx->d_mon_part2, n2, ctx->d_mon_state, ctx->d_mon_result, sa, steady, st); break;
-    case 1: launch_mon_reduce_1(a.mon_part, a.mon_nparts, ctx->d_mon_part2, n2, ctx->d_mon_state, ctx->d_mon_result, sa, steady, st); break;
-    default: launch_mon_reduce_2(a.mon_part, a.mon_nparts, ctx->d_mon_part2, n2, ctx->d_mon_state, ctx->d_mon_result, sa, steady, st); break;
-  }
-  CK(cudaGetLastError());
-  return HLBG_OK;
+  a.mon_result = ctx->d_mon_result;
+  a.mon_fold = fold;
+  a.mon_steady = steady;
+  a.steady = SteadyArgs{ctx->d_steady, ctx->d_steady ? ctx->d_steady + 1 : nullptr, ctx->d_steady_n};
 }
 
 int run_post(hlbg_ctx* ctx, cudaStream_t st, const int32_t* slot, const int8_t* dir, const float* q,
@@ -957,11 +954,10 @@ int graph_steps(hlbg_ctx* ctx, int n, bool check) {
       fill_args(ctx, a);
       a.iolet_rho = ctx->d_io_tab + (size_t)k * 2 * ctx->n_io;
       a.iolet_umax = a.iolet_rho + ctx->n_io;
-      if (check) mon_args(ctx, a);
+      if (check) mon_args(ctx, a, true, true);
       rc = launch_collide(ctx, a, ctx->stream);
       if (!rc) rc = run_post(ctx, ctx->stream, ctx->d_ps_slot, ctx->d_ps_dir, ctx->d_ps_q, ctx->n_ps);
       ctx->cur ^= 1;
-      if (!rc && check) rc = mon_reduce(ctx, a, true, ctx->stream);
     }
     ctx->cur = cur0;
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
@@ -988,6 +984,12 @@ int graph_steps(hlbg_ctx* ctx, int n, bool check) {
 }  // namespace
 
 namespace {
+
+// Launch shape of a new context: the fluid list, whose warps hold fluid sites only.
+// All slots (index 0) was the default before: on the 1.46M-site bifurcation, where 38 %
+// of the slots are solid, FP64 takes 670 us a step against 786, FP32 63 against 75.
+// FP16 takes 128 x 9 (its list keeps bulk and boundary sites apart).
+int default_variant(int prec) { return prec == HLBG_FP16 ? 5 : 6; }
 
 // Iolet parameters of a context: the models must match the streamers (Nash reads
 // a density, Ladd a velocity), and the warm-up start density is the smallest iolet
@@ -1080,7 +1082,7 @@ void hlbg_destroy(hlbg_ctx* ctx) {
                   ctx->d_io_tab,    ctx->d_stage,     ctx->d_stage_rho, ctx->d_stage_u,
                   ctx->d_list,      ctx->d_part,      ctx->d_part_bad,  ctx->d_steady,
                   ctx->d_steady_n,  ctx->d_slot2site, ctx->d_site2slot, ctx->d_mon_u,
-                  ctx->d_mon_part,  ctx->d_mon_part2, ctx->d_mon_state, ctx->d_mon_result,
+                  ctx->d_mon_part,  ctx->d_mon_part2, ctx->d_mon_tick, ctx->d_mon_state, ctx->d_mon_result,
                   ctx->d_warp_block, ctx->d_lane_slot, ctx->d_b_normal, ctx->d_wss,
                   ctx->d_blk_fluid, ctx->d_blk_bnd, ctx->d_blk_run_off, ctx->d_blk_runs, ctx->d_pipe_desc, ctx->d_stage_err,
                   ctx->d_flux_slot, ctx->d_flux_gi, ctx->d_flux, ctx->d_halo_err};
@@ -1121,6 +1123,7 @@ int hlbg_create(const hlbg_geometry* g, const hlbg_params* p, const hlbg_iolet* 
     return fail(ctx, HLBG_ERR_INVAL, "bad iolet arrays");
   ctx->params = *p;
   ctx->prec = p->precision;
+  ctx->sc_variant = default_variant(ctx->prec);
   ctx->elem = p->precision == HLBG_FP64 ? 8 : (p->precision == HLBG_FP32DEV ? 4 : 2);
   int rc = set_iolet_params(ctx, inlets, n_inlets, outlets, n_outlets);
   if (rc) return rc;
@@ -1414,7 +1417,7 @@ int hlbg_step_monitored(hlbg_ctx* ctx, int32_t nsteps, hlbg_stats* out) {
       fill_args(ctx, a);
       a.iolet_rho = ctx->d_io_tab + (size_t)k * 2 * ctx->n_io;
       a.iolet_umax = a.iolet_rho + ctx->n_io;
-      if (check || record) mon_args(ctx, a);
+      if (check || record) mon_args(ctx, a, check, false);
       // a record-only step compares nothing: the velocities on record are older
       if (record) CK(cudaMemsetAsync(ctx->d_mon_state, 0, sizeof(int32_t), st));
       if ((rc = launch_collide(ctx, a, st))) return rc;
@@ -1422,7 +1425,6 @@ int hlbg_step_monitored(hlbg_ctx* ctx, int32_t nsteps, hlbg_stats* out) {
       ctx->cur ^= 1;
       ctx->t1++;
       if (check) {
-        if ((rc = mon_reduce(ctx, a, false, st))) return rc;
         ctx->mon_checked_t = (int64_t)t;
       } else if (record) {
         // the next step's check is valid (any nonzero word marks the record present)

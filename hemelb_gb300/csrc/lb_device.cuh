@@ -133,6 +133,16 @@ __host__ __device__ __forceinline__ int local_of_slot(int j) {
 }
 __host__ __device__ __forceinline__ int slot_of_local(int l) { return slot_in_block(l >> 6, (l >> 3) & 7, l & 7); }
 
+// Steady-state detection after every step (StabilityTester with its convergence
+// check, Code/lb/StabilityTester.h:91-183): the end of the fused monitor's
+// reduction counts checks and records the first check whose max |u_new - u_old|
+// is within the threshold (tol * U_ref), and the first unstable one.
+struct SteadyArgs {
+  const double* threshold;  // tol * U_ref
+  double* last_du;          // max |du| of the latest check
+  long long* counters;      // [checks done, first converged check or -1, first unstable check or -1]
+};
+
 struct StepArgs {
   const void* f_old;
   void* f_new;
@@ -143,12 +153,20 @@ struct StepArgs {
   const uint16_t* site2slot;  // [nslot] slot of each local site (packed blocks)
   // Fused StabilityTester (monitored steps only): each site's velocity at its last
   // update, u[(block * 3 + c) * 512 + slot] (double for FP64, float otherwise); the
-  // per-CTA partials [mass | max |du| | min f | unstable] with stride mon_nparts;
-  // mon_state 0 while no velocity has been recorded since the state was set.
+  // per-CTA partials (mon_finish, stride mon_nparts), those of groups of CTAs, and the
+  // arrival counters (groups arrived, then CTAs arrived per group; zero between
+  // launches); mon_state 0 while no velocity has been recorded since the state was
+  // set.  mon_fold 0: record the velocities only.
   void* mon_u;
   double* mon_part;
   int64_t mon_nparts;
-  const int32_t* mon_state;
+  double* mon_part2;
+  uint32_t* mon_tick;
+  int32_t* mon_state;
+  double* mon_result;
+  SteadyArgs steady;
+  int32_t mon_fold;
+  int32_t mon_steady;  // count this check for steady-state detection
   // Fluid-list launch: warp w works on block warp_block[w] & 0x7fffffff, lane k on
   // its slot lane_slot[32 w + k] & 511 (0xffff: idle; kListBoundary set for a site
   // with a boundary record); a negative warp_block marks a warp that only writes

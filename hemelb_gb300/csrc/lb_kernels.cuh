@@ -291,60 +291,83 @@ struct PushMixed<P, Q> {
 
 // StabilityTester::PostSendToParent (Code/lb/StabilityTester.h:91-149) and
 // ComputeRelativeDifference (:160-183) plus total mass: one slot per thread, one
-// partial per CTA, reduced by k_monitor_final in a fixed order (deterministic).
+// partial per CTA, reduced in a fixed order (deterministic): by k_monitor_final, or by
+// mon_finish in the fused form.
 // The fused monitor also tracks IncompressibilityChecker's quantities
 // (Code/lb/IncompressibilityChecker.hpp:157-199): smallest and largest density and
 // largest velocity magnitude over the sites.
+// FP64 comparisons run on the FP64 unit (a warp instruction every 16 cycles or so per
+// SM), so everything but the mass is kept in 64-bit integers whose order is that of
+// the values: the unsigned bits of a squared speed (never negative; a NaN sorts above
+// infinity, so the maximum propagates it as !(x <= max) does) and, for densities and
+// distributions, ordered_key.  |du| and |u| stay squared until the last stage: the
+// square root is monotonic and correctly rounded, so the maximum is the same.
 struct MonAcc {
-  double mass, maxdu, minf;
-  unsigned long long bad;
-  double rmin, rmax, umax;
+  double mass;
+  unsigned long long maxdu, umax, bad;
+  long long minf, rmin, rmax;
 };
 
+// Signed integer with the order of the doubles (NaN excluded by the callers).
+__device__ __forceinline__ long long ordered_key(double v) {
+  const long long b = __double_as_longlong(v);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double ordered_value(long long k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
+}
+__device__ __forceinline__ bool is_nan64(double v) {
+  return (__double_as_longlong(v) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+}
+
 __device__ __forceinline__ MonAcc mon_neutral() {
-  return MonAcc{0.0, 0.0, 1.0e300, 0ull, 1.0e300, -1.0e300, 0.0};
+  return MonAcc{0.0, 0ull, 0ull, 0ull, ordered_key(1.0e300), ordered_key(1.0e300), ordered_key(-1.0e300)};
 }
 
 __device__ __forceinline__ void mon_combine(MonAcc& a, const MonAcc& b) {
   a.mass += b.mass;
-  if (!(b.maxdu <= a.maxdu)) a.maxdu = b.maxdu;  // NaN-propagating max
-  a.minf = fmin(a.minf, b.minf);
+  a.maxdu = a.maxdu > b.maxdu ? a.maxdu : b.maxdu;
+  a.umax = a.umax > b.umax ? a.umax : b.umax;
   a.bad += b.bad;
-  a.rmin = fmin(a.rmin, b.rmin);
-  a.rmax = fmax(a.rmax, b.rmax);
-  if (!(b.umax <= a.umax)) a.umax = b.umax;
+  a.minf = a.minf < b.minf ? a.minf : b.minf;
+  a.rmin = a.rmin < b.rmin ? a.rmin : b.rmin;
+  a.rmax = a.rmax > b.rmax ? a.rmax : b.rmax;
 }
 
 __device__ __forceinline__ MonAcc mon_shfl(const MonAcc& v, int off) {
   MonAcc o;
   o.mass = __shfl_down_sync(0xffffffffu, v.mass, off);
   o.maxdu = __shfl_down_sync(0xffffffffu, v.maxdu, off);
-  o.minf = __shfl_down_sync(0xffffffffu, v.minf, off);
+  o.umax = __shfl_down_sync(0xffffffffu, v.umax, off);
   o.bad = __shfl_down_sync(0xffffffffu, v.bad, off);
+  o.minf = __shfl_down_sync(0xffffffffu, v.minf, off);
   o.rmin = __shfl_down_sync(0xffffffffu, v.rmin, off);
   o.rmax = __shfl_down_sync(0xffffffffu, v.rmax, off);
-  o.umax = __shfl_down_sync(0xffffffffu, v.umax, off);
   return o;
+}
+
+__device__ __forceinline__ MonAcc mon_warp(MonAcc v) {  // result valid in lane 0
+  for (int off = 16; off > 0; off >>= 1) mon_combine(v, mon_shfl(v, off));
+  return v;
 }
 
 // CTA-wide reduction (up to 1024 threads) in a fixed order; result valid in thread 0.
 __device__ __forceinline__ MonAcc mon_block(MonAcc v) {
+  v = mon_warp(v);
+  if (blockDim.x == 32) return v;
   __shared__ MonAcc sh[32];
-  for (int off = 16; off > 0; off >>= 1) mon_combine(v, mon_shfl(v, off));
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) sh[w] = v;
   __syncthreads();
-  if (w == 0) {
-    v = lane < (int)(blockDim.x >> 5) ? sh[lane] : mon_neutral();
-    for (int off = 16; off > 0; off >>= 1) mon_combine(v, mon_shfl(v, off));
-  }
+  if (threadIdx.x == 0)
+    for (int k = 1; k < (int)(blockDim.x >> 5); ++k) mon_combine(v, sh[k]);
   return v;
 }
 
 // The FP32 forms accumulate their monitor values in FP32 and integers up to the
 // CTA's partial (min / max are exact in any precision; the mass is a count plus
-// the sum of the density deviations, which are small); only the second reduction
-// stage works in FP64: GB300's FP64 rate would otherwise make every monitored CTA
+// the sum of the density deviations, which are small); only the mass of a group of
+// CTAs is summed in FP64: GB300's FP64 rate would otherwise make every monitored CTA
 // an FP64 workload.
 struct MonAccF {
   float dm, maxdu, minf, dmin, dmax, umax;  // dm: sum of rho - 1; dmin/dmax: of rho - 1;
@@ -419,22 +442,36 @@ __device__ __forceinline__ void mon_site(const StepArgs& a, int64_t s, const dou
   const double ux = mx / m0, uy = my / m0, uz = mz / m0;
   if (check) {
     const double dx = ux - uo.x, dy = uy - uo.y, dz = uz - uo.z;
-    const double du = sqrt(dot3d(dx, dy, dz, dx, dy, dz));
-    if (!(du <= acc.maxdu)) acc.maxdu = du;
+    const unsigned long long du2 = (unsigned long long)__double_as_longlong(dot3d(dx, dy, dz, dx, dy, dz));
+    acc.maxdu = du2 > acc.maxdu ? du2 : acc.maxdu;
     acc.mass += m0;
-    acc.rmin = fmin(acc.rmin, m0);
-    acc.rmax = fmax(acc.rmax, m0);
-    const double um = sqrt(dot3d(ux, uy, uz, ux, uy, uz));
-    if (!(um <= acc.umax)) acc.umax = um;
-    bool bad = false;
-    double mn = f[0];
-#pragma unroll
-    for (int d = 0; d < Q; ++d) {
-      bad |= !(f[d] > 0.0);
-      mn = fmin(mn, f[d]);
+    if (!is_nan64(m0)) {  // fmin / fmax pass over a NaN
+      const long long k = ordered_key(m0);
+      acc.rmin = k < acc.rmin ? k : acc.rmin;
+      acc.rmax = k > acc.rmax ? k : acc.rmax;
     }
-    acc.minf = fmin(acc.minf, mn);
-    acc.bad += bad ? 1ull : 0ull;
+    const unsigned long long um2 = (unsigned long long)__double_as_longlong(dot3d(ux, uy, uz, ux, uy, uz));
+    acc.umax = um2 > acc.umax ? um2 : acc.umax;
+    // bits of positive doubles are positive integers in the same order; any f <= 0
+    // (or -0) makes the smallest of them non-positive, a NaN makes the density NaN
+    long long mn = __double_as_longlong(f[0]);
+#pragma unroll
+    for (int d = 1; d < Q; ++d) {
+      const long long v = __double_as_longlong(f[d]);
+      mn = v < mn ? v : mn;
+    }
+    if (mn <= 0 || is_nan64(m0)) {
+      bool bad = false;
+      mn = ordered_key(1.0e300);
+#pragma unroll
+      for (int d = 0; d < Q; ++d) {
+        const long long k = ordered_key(f[d]);
+        bad |= k <= 0 || is_nan64(f[d]);
+        if (!is_nan64(f[d])) mn = k < mn ? k : mn;
+      }
+      acc.bad += bad ? 1ull : 0ull;
+    }
+    acc.minf = mn < acc.minf ? mn : acc.minf;
   }
   u[ui] = ux;
   u[ui + kSites] = uy;
@@ -480,38 +517,140 @@ template <int P>
 __device__ __forceinline__ MonAccT<P> mon_neutral_t() {
   if constexpr (P == 0) return mon_neutral(); else return mon_neutral_f();
 }
-// One CTA's monitor partial: FP64 form as 7 doubles [mass | max |du| | min f |
-// unstable | min rho | max rho | max |u|], stride mon_nparts; FP32 forms as 8
-// 32-bit words [sum (rho-1) | max |du| | min f | min (rho-1) | max (rho-1) | max |u|
-// | count | unstable] in the same buffer, converted to FP64 by the second stage.
+// One CTA's monitor partial: FP64 form as 7 64-bit words (the fields of MonAcc, stride
+// mon_nparts); FP32 forms as 8 32-bit words [sum (rho-1) | max |du|^2 | min f | min
+// (rho-1) | max (rho-1) | max |u|^2 | count | unstable] in the same buffer.
+constexpr int kMonWords = 7;
+__device__ __forceinline__ void mon_store(double* part, int64_t n, int64_t i, const MonAcc& r) {
+  long long* p = reinterpret_cast<long long*>(part);
+  part[i] = r.mass;
+  p[n + i] = (long long)r.maxdu;
+  p[2 * n + i] = (long long)r.umax;
+  p[3 * n + i] = (long long)r.bad;
+  p[4 * n + i] = r.minf;
+  p[5 * n + i] = r.rmin;
+  p[6 * n + i] = r.rmax;
+}
+// (written by other SMs earlier in the same launch: past L1)
+__device__ __forceinline__ MonAcc mon_load(const double* part, int64_t n, int64_t i) {
+  const long long* p = reinterpret_cast<const long long*>(part);
+  return MonAcc{__ldcg(part + i),
+                (unsigned long long)__ldcg(p + n + i),
+                (unsigned long long)__ldcg(p + 2 * n + i),
+                (unsigned long long)__ldcg(p + 3 * n + i),
+                __ldcg(p + 4 * n + i),
+                __ldcg(p + 5 * n + i),
+                __ldcg(p + 6 * n + i)};
+}
 template <int P>
-__device__ __forceinline__ void mon_write_partial(const StepArgs& a, const MonAccT<P>& acc, unsigned cta) {
+__device__ __forceinline__ MonAcc mon_load_cta(const StepArgs& a, int64_t i) {
   const int64_t n = a.mon_nparts;
   if constexpr (P == 0) {
+    return mon_load(a.mon_part, n, i);
+  } else {
+    const float* p = reinterpret_cast<const float*>(a.mon_part);
+    const unsigned count = __float_as_uint(__ldcg(p + 6 * n + i));
+    if (count == 0) return mon_neutral();  // a CTA of idle lanes only
+    const double du = (double)sqrtf(__ldcg(p + n + i)), um = (double)sqrtf(__ldcg(p + 5 * n + i));
+    MonAcc r;
+    r.mass = (double)count + (double)__ldcg(p + i);
+    r.maxdu = (unsigned long long)__double_as_longlong(du);
+    r.umax = (unsigned long long)__double_as_longlong(um);
+    r.bad = __float_as_uint(__ldcg(p + 7 * n + i));
+    r.minf = ordered_key((double)__ldcg(p + 2 * n + i));
+    r.rmin = ordered_key(1.0 + (double)__ldcg(p + 3 * n + i));
+    r.rmax = ordered_key(1.0 + (double)__ldcg(p + 4 * n + i));
+    return r;
+  }
+}
+
+// End of a monitored CTA: its partial, and the reduction of all of them in the same
+// launch.  The CTAs form groups of kMonGroup; the last CTA of a group to arrive folds
+// the group's partials in index order, and the last group's folds the groups' -- a
+// fixed tree, so the result does not depend on the order of arrival -- and writes the
+// result [mass, max |du|, min f, unstable, valid, min rho, max rho, max |u|], where
+// valid is 0 for the first step after the state was set (it only recorded
+// velocities).  With mon_steady a valid check is also counted for steady-state
+// detection.  Every step then marks the recorded velocities as present.  As two
+// launches after the update this took 19 + 10 us beside 59 us of a 34k-site FP64
+// step (seven FP64 comparisons and additions per shuffle level in every thread); the
+// whole monitored step is 32 us now.
+constexpr int kMonGroup = 64;
+template <int P>
+__device__ __forceinline__ void mon_finish(const StepArgs& a, const MonAccT<P>& acc, unsigned cta) {
+  const int64_t n = a.mon_nparts;
+  const unsigned groups = (unsigned)((n + kMonGroup - 1) / kMonGroup), g = cta / kMonGroup;
+  const int lane = threadIdx.x & 31;
+  int last = 0;
+  if constexpr (P == 0) {
     const MonAcc r = mon_block(acc);
-    if (threadIdx.x == 0) {
-      a.mon_part[cta] = r.mass;
-      a.mon_part[n + cta] = r.maxdu;
-      a.mon_part[2 * n + cta] = r.minf;
-      a.mon_part[3 * n + cta] = (double)r.bad;
-      a.mon_part[4 * n + cta] = r.rmin;
-      a.mon_part[5 * n + cta] = r.rmax;
-      a.mon_part[6 * n + cta] = r.umax;
-    }
+    if (threadIdx.x == 0) mon_store(a.mon_part, n, cta, r);
   } else {
     const MonAccF r = mon_block_f(acc);
     if (threadIdx.x == 0) {
       float* p = reinterpret_cast<float*>(a.mon_part);
       p[cta] = r.dm;
-      p[n + cta] = sqrtf(r.maxdu);
+      p[n + cta] = r.maxdu;
       p[2 * n + cta] = r.minf;
       p[3 * n + cta] = r.dmin;
       p[4 * n + cta] = r.dmax;
-      p[5 * n + cta] = sqrtf(r.umax);
+      p[5 * n + cta] = r.umax;
       p[6 * n + cta] = __uint_as_float(r.count);
       p[7 * n + cta] = __uint_as_float(r.bad);
     }
   }
+  if (threadIdx.x >= 32) return;
+  if (lane == 0) {
+    const unsigned size = (unsigned)(n - (int64_t)g * kMonGroup < kMonGroup ? n - (int64_t)g * kMonGroup : kMonGroup);
+    __threadfence();
+    last = atomicAdd(a.mon_tick + 1 + g, 1u) == size - 1;
+  }
+  if (!__shfl_sync(0xffffffffu, last, 0)) return;
+  __threadfence();
+  MonAcc v = mon_neutral();
+#pragma unroll
+  for (int k = 0; k < kMonGroup; k += 32) {
+    const int64_t i = (int64_t)g * kMonGroup + k + lane;
+    if (i < n) mon_combine(v, mon_load_cta<P>(a, i));
+  }
+  v = mon_warp(v);
+  if (lane == 0) {
+    mon_store(a.mon_part2, groups, g, v);
+    a.mon_tick[1 + g] = 0;
+    __threadfence();
+    last = atomicAdd(a.mon_tick, 1u) == groups - 1;
+  }
+  if (!__shfl_sync(0xffffffffu, last, 0)) return;
+  __threadfence();
+  v = mon_neutral();
+#pragma unroll 4
+  for (unsigned i = lane; i < groups; i += 32) mon_combine(v, mon_load(a.mon_part2, groups, i));
+  v = mon_warp(v);
+  if (lane != 0) return;
+  a.mon_tick[0] = 0;
+  const int valid = *a.mon_state != 0;
+  double du = __longlong_as_double((long long)v.maxdu), um = __longlong_as_double((long long)v.umax);
+  if constexpr (P == 0) {
+    du = sqrt(du);
+    um = sqrt(um);
+  }
+  double* result = a.mon_result;
+  result[0] = v.mass;
+  result[1] = du;
+  result[2] = ordered_value(v.minf);
+  result[3] = (double)v.bad;
+  result[4] = valid;
+  result[5] = ordered_value(v.rmin);
+  result[6] = ordered_value(v.rmax);
+  result[7] = um;
+  if (a.mon_steady && valid) {
+    const long long k = a.steady.counters[0] + 1;
+    a.steady.counters[0] = k;
+    *a.steady.last_du = du;
+    if (v.bad && a.steady.counters[2] < 0) a.steady.counters[2] = k;
+    if (du <= *a.steady.threshold && a.steady.counters[1] < 0) a.steady.counters[1] = k;
+  }
+  *a.mon_state = 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -744,7 +883,9 @@ __global__ void __launch_bounds__(THREADS, MINB) k_stream_collide_listed(StepArg
   bool check = false;
   if constexpr (MON) check = *a.mon_state != 0;
   collide_listed_warp<P, MON>(a, ((int64_t)cta * THREADS + threadIdx.x) >> 5, block_xyz, acc, check);
-  if constexpr (MON) mon_write_partial<P>(a, acc, cta);
+  if constexpr (MON) {
+    if (a.mon_fold) mon_finish<P>(a, acc, cta);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1106,6 +1247,11 @@ void launch_pipe(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
 #define HLBG_LIST_MINB 8
 #endif
 
+// FP64 fluid list, every shape: one warp per CTA.  The form is bound by the FP64 unit
+// of each SM, so what counts is that the SMs get equal numbers of warps: on a
+// 25k-site pipe (5 warps a SM) 128-thread CTAs leave some SMs with 8.
+constexpr int kListThreads64 = 32, kListMinb64 = 16;
+
 template <int P, int THREADS, int MINB, bool MON>
 void launch_listed(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
   const int64_t g = (a.n_warps * 32 + THREADS - 1) / THREADS;
@@ -1141,75 +1287,8 @@ __global__ void __launch_bounds__(THREADS, MINB)
   bool check = false;
   if constexpr (MON) check = *a.mon_state != 0;
   collide_slot<P, MON>(a, (int64_t)cta * THREADS + threadIdx.x, block_xyz, acc, check);
-  if constexpr (MON) mon_write_partial<P>(a, acc, cta);
-}
-
-// Second stage of the fused StabilityTester's reduction: CTA c folds partials
-// [c * per, (c + 1) * per) in a fixed order into out[c] (same layout, stride n_out).
-// fp32 != 0: the partials are the FP32 forms' 32-bit words (mon_write_partial).
-static __global__ void __launch_bounds__(256) k_mon_stage2(const double* __restrict__ in, int64_t n_in,
-                                                           int64_t per, double* __restrict__ out,
-                                                           int64_t n_out, int fp32) {
-  MonAcc acc = mon_neutral();
-  const int64_t lo = (int64_t)blockIdx.x * per, hi = lo + per < n_in ? lo + per : n_in;
-  const float* inf = reinterpret_cast<const float*>(in);
-  for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-    if (fp32) {
-      const unsigned count = __float_as_uint(inf[6 * n_in + i]);
-      if (count == 0) continue;  // a CTA of idle lanes only
-      mon_combine(acc, MonAcc{(double)count + (double)inf[i], (double)inf[n_in + i], (double)inf[2 * n_in + i],
-                              (unsigned long long)__float_as_uint(inf[7 * n_in + i]), 1.0 + (double)inf[3 * n_in + i],
-                              1.0 + (double)inf[4 * n_in + i], (double)inf[5 * n_in + i]});
-    } else {
-      mon_combine(acc, MonAcc{in[i], in[n_in + i], in[2 * n_in + i], (unsigned long long)in[3 * n_in + i],
-                              in[4 * n_in + i], in[5 * n_in + i], in[6 * n_in + i]});
-    }
-  }
-  __syncthreads();
-  acc = mon_block(acc);
-  if (threadIdx.x == 0) {
-    out[blockIdx.x] = acc.mass;
-    out[n_out + blockIdx.x] = acc.maxdu;
-    out[2 * n_out + blockIdx.x] = acc.minf;
-    out[3 * n_out + blockIdx.x] = (double)acc.bad;
-    out[4 * n_out + blockIdx.x] = acc.rmin;
-    out[5 * n_out + blockIdx.x] = acc.rmax;
-    out[6 * n_out + blockIdx.x] = acc.umax;
-  }
-}
-
-// Last stage: result = [mass, max |du|, min f, unstable, valid, min rho, max rho,
-// max |u|]; valid is 0 for the
-// first step after the state was set (it only recorded velocities).  With sa, a
-// valid check is also counted for steady-state detection.
-// Every step then marks the recorded velocities as present.
-static __global__ void __launch_bounds__(256) k_mon_final(const double* __restrict__ part, int64_t n,
-                                                          int32_t* mon_state, double* result,
-                                                          SteadyArgs sa, int steady) {
-  MonAcc acc = mon_neutral();
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x)
-    mon_combine(acc, MonAcc{part[i], part[n + i], part[2 * n + i], (unsigned long long)part[3 * n + i],
-                            part[4 * n + i], part[5 * n + i], part[6 * n + i]});
-  __syncthreads();
-  acc = mon_block(acc);
-  if (threadIdx.x == 0) {
-    const int valid = *mon_state != 0;
-    result[0] = acc.mass;
-    result[1] = acc.maxdu;
-    result[2] = acc.minf;
-    result[3] = (double)acc.bad;
-    result[4] = valid;
-    result[5] = acc.rmin;
-    result[6] = acc.rmax;
-    result[7] = acc.umax;
-    if (steady && valid) {
-      const long long k = sa.counters[0] + 1;
-      sa.counters[0] = k;
-      *sa.last_du = acc.maxdu;
-      if (acc.bad && sa.counters[2] < 0) sa.counters[2] = k;
-      if (acc.maxdu <= *sa.threshold && sa.counters[1] < 0) sa.counters[1] = k;
-    }
-    *mon_state = 1;
+  if constexpr (MON) {
+    if (a.mon_fold) mon_finish<P>(a, acc, cta);
   }
 }
 
@@ -1405,6 +1484,7 @@ __global__ void __launch_bounds__(256) k_monitor(MonitorArgs ma) {
     const S* fc = static_cast<const S*>(ma.f_cur) + off;
     const S* fp = static_cast<const S*>(ma.f_prev) + off;
     bool bad = false;
+    long long mn = ordered_key(1.0e300);
     double rn, dx, dy, dz;
     if constexpr (P == 0) {
       // Lattice::CalculateDensityAndMomentum (scalar order) on fNew and fOld
@@ -1414,8 +1494,9 @@ __global__ void __launch_bounds__(256) k_monitor(MonitorArgs ma) {
       for (int d = 0; d < Q; ++d) {
         const double vn = St::load(fc, d * kSites, a);
         const double vo = St::load(fp, d * kSites, a);
-        if (!(vn > 0.0)) bad = true;
-        acc.minf = fmin(acc.minf, vn);
+        const long long k = ordered_key(vn);
+        bad |= k <= 0 || is_nan64(vn);
+        if (!is_nan64(vn)) mn = k < mn ? k : mn;
         rn += vn;
         xn += (double)Lat::cx(d) * vn;
         yn += (double)Lat::cy(d) * vn;
@@ -1431,16 +1512,16 @@ __global__ void __launch_bounds__(256) k_monitor(MonitorArgs ma) {
     } else {
       // deviation form: FP32 on g = f - w; only the mass accumulates in FP64
       float gn[Q], go[Q];
-      float mn = 1.0e30f;
+      float mnf = 1.0e30f;
 #pragma unroll
       for (int d = 0; d < Q; ++d) {
         gn[d] = St::load(fc, d * kSites, a);
         go[d] = St::load(fp, d * kSites, a);
         const float fv = gn[d] + weight_f(d);
         if (!(fv > 0.f)) bad = true;
-        mn = fminf(mn, fv);
+        mnf = fminf(mnf, fv);
       }
-      acc.minf = (double)mn;
+      mn = ordered_key((double)mnf);
       float drn, mxn, myn, mzn, dro, mxo, myo, mzo;
       moments_dev(gn, drn, mxn, myn, mzn);
       moments_dev(go, dro, mxo, myo, mzo);
@@ -1452,30 +1533,38 @@ __global__ void __launch_bounds__(256) k_monitor(MonitorArgs ma) {
     }
     acc.bad = bad ? 1ull : 0ull;
     acc.mass = rn;
-    acc.maxdu = sqrt(dot3d(dx, dy, dz, dx, dy, dz));
+    acc.minf = mn;
+    acc.maxdu = (unsigned long long)__double_as_longlong(dot3d(dx, dy, dz, dx, dy, dz));
   }
   acc = mon_block(acc);
   if (threadIdx.x == 0) {
     ma.part_mass[blockIdx.x] = acc.mass;
-    ma.part_max[blockIdx.x] = acc.maxdu;
-    ma.part_min[blockIdx.x] = acc.minf;
+    ma.part_max[blockIdx.x] = __longlong_as_double((long long)acc.maxdu);
+    ma.part_min[blockIdx.x] = __longlong_as_double(acc.minf);
     ma.part_bad[blockIdx.x] = acc.bad;
   }
 }
 
 // Reduce the per-CTA partials of k_monitor in a fixed order into element 0 of
-// each partial array (one CTA of 256 threads; thread t folds partials t, t+256, ...).
-static __global__ void __launch_bounds__(256) k_monitor_final(MonitorArgs ma, int64_t nparts) {
+// each partial array (one CTA of 1024 threads; thread t folds partials t, t + 1024,
+// ...), the largest |du| and smallest f as values again.
+static __global__ void __launch_bounds__(1024) k_monitor_final(MonitorArgs ma, int64_t nparts) {
   MonAcc acc = mon_neutral();
-  for (int64_t i = threadIdx.x; i < nparts; i += blockDim.x)
-    mon_combine(acc, MonAcc{ma.part_mass[i], ma.part_max[i], ma.part_min[i], ma.part_bad[i], 1.0e300, -1.0e300,
-                            0.0});
-  __syncthreads();
+#pragma unroll 4
+  for (int64_t i = threadIdx.x; i < nparts; i += 1024) {
+    MonAcc p = mon_neutral();
+    p.mass = ma.part_mass[i];
+    p.maxdu = (unsigned long long)__double_as_longlong(ma.part_max[i]);
+    p.minf = __double_as_longlong(ma.part_min[i]);
+    p.bad = ma.part_bad[i];
+    mon_combine(acc, p);
+  }
   acc = mon_block(acc);
+  __syncthreads();
   if (threadIdx.x == 0) {
     ma.part_mass[0] = acc.mass;
-    ma.part_max[0] = acc.maxdu;
-    ma.part_min[0] = acc.minf;
+    ma.part_max[0] = sqrt(__longlong_as_double((long long)acc.maxdu));
+    ma.part_min[0] = ordered_value(acc.minf);
     ma.part_bad[0] = acc.bad;
   }
 }
@@ -1649,90 +1738,74 @@ __global__ void k_halo_unpack(void* f, const int64_t* off, int64_t n, int64_t li
 }
 }  // namespace hlbg
 
+namespace hlbg {
+// The stream-and-collide launch of an index (hlbg_set_launch_variant).
+template <int P>
+void launch_update(const StepArgs& a, const int32_t* bxyz, cudaStream_t st, int variant) {
+  if (a.list) {
+    const unsigned g = (unsigned)((a.list_count + 255) / 256);
+    if (g) k_stream_collide_list<P><<<g, 256, 0, st>>>(a, bxyz);
+    return;
+  }
+  if constexpr (P == 0) {  // two shapes: all slots (0..3) and the fluid list
+    if (variant < 4) {
+      if (a.mon_u) launch_sc<0, 128, 2, true>(a, bxyz, st);
+      else launch_sc<0, 128, 2>(a, bxyz, st);
+    } else {
+      if (a.mon_u) launch_listed<0, kListThreads64, kListMinb64, true>(a, bxyz, st);
+      else launch_listed<0, kListThreads64, kListMinb64, false>(a, bxyz, st);
+    }
+  } else if (a.mon_u) {
+    // monitored steps: one partial per CTA; the 10-CTA all-slots shape becomes 128 x 8,
+    // every other shape from index 4 up the 128 x 8 fluid list
+    switch (variant) {
+      case 0:
+      case 1: launch_sc<P, 128, 8, true>(a, bxyz, st); break;
+      case 2: launch_sc<P, 256, 4, true>(a, bxyz, st); break;
+      case 3: launch_sc<P, 512, 2, true>(a, bxyz, st); break;
+      default: launch_listed<P, 128, 8, true>(a, bxyz, st); break;
+    }
+  } else {
+    // the staged shapes need the block tables (the default layout)
+    if (variant == 4 && !a.blk_runs) variant = 6;
+    if (variant == 8 && !a.pipe_desc) variant = 6;
+    switch (variant) {
+      case 1: launch_sc<P, 128, 8>(a, bxyz, st); break;
+      case 2: launch_sc<P, 256, 4>(a, bxyz, st); break;
+      case 3: launch_sc<P, 512, 2>(a, bxyz, st); break;
+      case 4:
+        launch_block_staged<P, 256, 4>(a, bxyz, st);
+        launch_iolets<P>(a, bxyz, st);
+        break;
+      case 5: launch_listed<P, 128, 9, false>(a, bxyz, st); break;
+      case 6: launch_listed<P, 128, HLBG_LIST_MINB, false>(a, bxyz, st); break;
+      case 7: launch_listed<P, HLBG_LISTED7_THREADS, 1024 / HLBG_LISTED7_THREADS, false>(a, bxyz, st); break;
+      case 8:
+        launch_pipe<P, HLBG_PIPE_NCW, (P == 1 ? HLBG_PIPE_STAGES : 2 * HLBG_PIPE_STAGES)>(a, bxyz, st);
+        launch_iolets<P>(a, bxyz, st);
+        break;
+      default: launch_sc<P, HLBG_SC_THREADS, HLBG_SC_MINB>(a, bxyz, st); break;
+    }
+  }
+}
+
+// CTAs of a monitored step's update (one partial each).
+template <int P>
+int64_t monitored_ctas(int64_t nslot, int variant, int64_t n_warps) {
+  if (variant >= 4) return P == 0 ? (n_warps * 32 + kListThreads64 - 1) / kListThreads64 : (n_warps * 32 + 127) / 128;
+  if (P == 0 || variant < 2) return nslot / 128;
+  return variant == 2 ? nslot / 256 : nslot / 512;
+}
+}  // namespace hlbg
+
 #define HLBG_INSTANTIATE(P)                                                                     \
   namespace hlbg {                                                                              \
   void launch_stream_collide_##P(const StepArgs& a, const int32_t* bxyz, cudaStream_t st,      \
                                  int variant) {                                                 \
-    if (a.list) {                                                                               \
-      unsigned g = (unsigned)((a.list_count + 255) / 256);                                      \
-      if (g) k_stream_collide_list<P><<<g, 256, 0, st>>>(a, bxyz);                              \
-      return;                                                                                   \
-    }                                                                                           \
-    /* monitored steps: the 10-CTA all-slots shape becomes 128 x 8, every fluid-list    */      \
-    /* shape the 128 x 8 fluid list (one partial per 128-thread CTA)                     */      \
-    if (a.mon_u && variant == 0) variant = 1;                                                   \
-    if (a.mon_u && variant >= 4) variant = 6;                                                   \
-    if (variant == 4) {                                                                         \
-      if constexpr (P != 0) {                                                                   \
-        if (a.blk_runs) {                                                                       \
-          launch_block_staged<P, 256, 4>(a, bxyz, st);                                          \
-          launch_iolets<P>(a, bxyz, st);                                                        \
-          return;                                                                               \
-        }                                                                                       \
-      }                                                                                         \
-      variant = 6; /* FP64, or a layout without the block tables */                             \
-    }                                                                                           \
-    if (variant == 8) {                                                                         \
-      if constexpr (P != 0) {                                                                   \
-        if (a.pipe_desc && !a.mon_u) {                                                          \
-          launch_pipe<P, HLBG_PIPE_NCW, (P == 1 ? HLBG_PIPE_STAGES : 2 * HLBG_PIPE_STAGES)>(a, bxyz, st); \
-          launch_iolets<P>(a, bxyz, st);                                                        \
-          return;                                                                               \
-        }                                                                                       \
-      }                                                                                         \
-      variant = 6; /* FP64, monitored steps, or a layout without the block tables */            \
-    }                                                                                           \
-    if (variant == 5) {                                                                         \
-      launch_listed<P, 128, (P == 0 ? 2 : 9), false>(a, bxyz, st);                              \
-      return;                                                                                   \
-    }                                                                                           \
-    if (variant == 7) {                                                                         \
-      if (!a.mon_u) {                                                                           \
-        launch_listed<P, HLBG_LISTED7_THREADS, (P == 0 ? 2 : 1024 / HLBG_LISTED7_THREADS),      \
-                      false>(a, bxyz, st);                                                      \
-        return;                                                                                 \
-      }                                                                                         \
-      variant = 6; /* monitored steps keep 128-thread CTAs (one partial per CTA) */             \
-    }                                                                                           \
-    if (variant == 6) {                                                                         \
-      if (a.mon_u) launch_listed<P, 128, (P == 0 ? 2 : 8), true>(a, bxyz, st);                  \
-      else launch_listed<P, 128, (P == 0 ? 2 : HLBG_LIST_MINB), false>(a, bxyz, st);            \
-      return;                                                                                   \
-    }                                                                                           \
-    if (P == 0) variant = -1;                                                                   \
-    if (a.mon_u) { /* one partial per CTA */                                                    \
-      switch (variant) {                                                                        \
-        case 2: launch_sc<P, 256, (P == 0 ? 2 : 4), true>(a, bxyz, st); break;                  \
-        case 3: launch_sc<P, 512, (P == 0 ? 1 : 2), true>(a, bxyz, st); break;                  \
-        case -1: launch_sc<P, 128, 2, true>(a, bxyz, st); break;                                \
-        default: launch_sc<P, 128, (P == 0 ? 2 : 8), true>(a, bxyz, st); break;                 \
-      }                                                                                         \
-      return;                                                                                   \
-    }                                                                                           \
-    switch (variant) {                                                                          \
-      case 1: launch_sc<P, 128, (P == 0 ? 2 : 8)>(a, bxyz, st); break;                          \
-      case 2: launch_sc<P, 256, (P == 0 ? 2 : 4)>(a, bxyz, st); break;                          \
-      case 3: launch_sc<P, 512, (P == 0 ? 1 : 2)>(a, bxyz, st); break;                          \
-      case -1: launch_sc<P, 128, 2>(a, bxyz, st); break;                                        \
-      default: launch_sc<P, HLBG_SC_THREADS, HLBG_SC_MINB>(a, bxyz, st); break;                 \
-    }                                                                                           \
+    launch_update<P>(a, bxyz, st, variant);                                                     \
   }                                                                                             \
   int64_t monitored_grid_##P(int64_t nslot, int variant, int64_t n_warps) {                    \
-    if (variant >= 4) return (n_warps * 32 + 127) / 128; /* monitored 4..8 run as 6 */          \
-    if (P == 0) return nslot / 128;                                                             \
-    switch (variant) {                                                                          \
-      case 1: return nslot / 128;                                                               \
-      case 2: return nslot / 256;                                                               \
-      case 3: return nslot / 512;                                                               \
-      default: return nslot / 128; /* monitored steps: the 128 x 8 shape */                     \
-    }                                                                                           \
-  }                                                                                             \
-  void launch_mon_reduce_##P(const double* part, int64_t nparts, double* part2, int64_t n2,      \
-                             int32_t* mon_state, double* result, const SteadyArgs& sa,          \
-                             int steady, cudaStream_t st) {                                      \
-    const int64_t per = (nparts + n2 - 1) / n2;                                                 \
-    k_mon_stage2<<<(unsigned)n2, 256, 0, st>>>(part, nparts, per, part2, n2, P != 0);           \
-    k_mon_final<<<1, 256, 0, st>>>(part2, n2, mon_state, result, sa, steady);                   \
+    return monitored_ctas<P>(nslot, variant, n_warps);                                          \
   }                                                                                             \
   void launch_post_step_##P(const PostArgs& p, cudaStream_t st) {                               \
     unsigned g = (unsigned)((p.count + 255) / 256);                                             \
@@ -1767,7 +1840,7 @@ __global__ void k_halo_unpack(void* f, const int64_t* off, int64_t n, int64_t li
     (void)grid;                                                                                 \
     const int64_t nparts = (ma.nslot + 255) / 256;                                              \
     k_monitor<P><<<(unsigned)nparts, 256, 0, st>>>(ma);                                         \
-    k_monitor_final<<<1, 256, 0, st>>>(ma, nparts);                                             \
+    k_monitor_final<<<1, 1024, 0, st>>>(ma, nparts);                                            \
   }                                                                                             \
   void launch_halo_copy_##P(void* f, const int64_t* off, int64_t n, int64_t limit, void* buf,     \
                             int unpack, int32_t* err, cudaStream_t st) {                        \

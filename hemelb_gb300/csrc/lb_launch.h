@@ -9,7 +9,8 @@ namespace hlbg {
 
 struct StepArgs;
 
-// Launch variants of the stream-and-collide kernel (FP32 / FP16 forms; FP64 has one):
+// Launch variants of the stream-and-collide kernel (FP64: all slots for 0-3, the fluid
+// list with one warp per CTA from 4 up):
 // 0 default shape, 1: 128x8, 2: 256x4, 3: 512x2 threads x resident CTAs per SM,
 // 4: one CTA per block, staged by bulk copies; 5, 6, 7: the fluid-list launch;
 // 8: persistent, pipelined block staging (FP32 / FP16).
@@ -71,16 +72,6 @@ struct MonitorArgs {
   float fp16_scale, fp16_inv_scale;
 };
 
-// Steady-state detection after every step (StabilityTester with its convergence
-// check, Code/lb/StabilityTester.h:91-183): the last stage of the fused monitor's
-// reduction counts checks and records the first check whose max |u_new - u_old|
-// is within the threshold (tol * U_ref), and the first unstable one.
-struct SteadyArgs {
-  const double* threshold;  // tol * U_ref
-  double* last_du;          // max |du| of the latest check
-  long long* counters;      // [checks done, first converged check or -1, first unstable check or -1]
-};
-
 // f_cur <- (f_cur + f_prev) / 2 on every fluid slot
 struct AverageArgs {
   void* f_cur;
@@ -131,9 +122,6 @@ struct FluxArgs {
   /* load the monitor kernels now (with lazy module loading they load on first use) */ \
   cudaError_t preload_monitor_##P();                                                 \
   int64_t monitored_grid_##P(int64_t nslot, int variant, int64_t n_warps);                                   \
-  void launch_mon_reduce_##P(const double* part, int64_t nparts, double* part2, int64_t n2,    \
-                             int32_t* mon_state, double* result, const SteadyArgs& sa,        \
-                             int steady, cudaStream_t st);                                     \
   void launch_average_##P(const AverageArgs& aa, cudaStream_t st);                    \
   void launch_halo_copy_##P(void* f, const int64_t* off, int64_t n, int64_t limit, void* buf, \
                             int unpack, int32_t* err, cudaStream_t st);                  \

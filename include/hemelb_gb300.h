@@ -317,8 +317,9 @@ int hlbg_average_time_levels(hlbg_ctx *ctx);
  * FP64 runs index 6 instead); the fluid list, whose warps hold only fluid slots,
  * at 128x9, 128x8 and 64x16; one persistent CTA per SM whose producer warp stages
  * blocks into a ring of shared-memory buffers by bulk asynchronous copies ahead of
- * 31 consumer warps (FP32 / FP16; FP64 runs index 6 instead)); FP64 runs two
- * CTAs per SM.  Monitored steps run every index from 4 up as the 128x8 fluid
+ * 31 consumer warps (FP32 / FP16; FP64 runs index 6 instead)); FP64 runs
+ * all slots for 0..3 and the fluid list in one-warp CTAs for the others.  A new
+ * context starts with the fluid list (6; FP16: 5).  Monitored steps run every index from 4 up as the 128x8 fluid
  * list.  No reference counterpart. */
 int hlbg_set_launch_variant(hlbg_ctx *ctx, int32_t variant);
 /* Autotuner: time each launch shape / schedule of the stream-and-collide kernel
