@@ -1934,8 +1934,10 @@ int hlbg_set_time_step(hlbg_ctx* ctx, uint64_t t1) {
 
 static int gather_common(hlbg_ctx* ctx, double* out, int32_t which, bool to_host) {
   if (!ctx || !out || (which != 0 && which != 1)) return HLBG_ERR_INVAL;
-  int rc = ensure_stage(ctx);
-  if (rc) return rc;
+  if (to_host) {
+    int rc = ensure_stage(ctx);
+    if (rc) return rc;
+  }
   GatherArgs ga;
   fill_gather(ctx, ga);
   ga.f = ctx->f[ctx->cur ^ which];
