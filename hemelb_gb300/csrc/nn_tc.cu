@@ -2,28 +2,49 @@
 // cores: tcgen05.mma with the accumulators in tensor memory (TMEM), operands staged
 // in shared memory by TMA (cp.async.bulk.tensor), completion tracked on mbarriers.
 //
-// Implicit GEMM.  One CTA computes an output tile of 8 (x) x 16 (y) x BZ (z)
-// voxels for all C_out output channels: BZ MMAs of M = 128 rows (one z-plane each,
-// N = C_out, a multiple of 16 up to 256), each with its FP32 accumulator in its
-// own TMEM columns.  The reduction runs over C_in in slices of 16 channels and,
-// within a slice, over the 27 taps (K = 16 per MMA):
-//  * per slice, one TMA load brings the input tile with its halo -- 10 x 18 x 4
-//    voxels, 16 channels, in two planes of 8 channels (16-byte rows), positions
-//    outside the volume read as zeros, which is the convolution's zero padding --
-//    and every tap's A operand is a shared-memory descriptor into that one tile:
-//    the core-matrix layout without swizzle puts the 8 rows of a core matrix (8
-//    consecutive x) in 128 contiguous bytes and steps 160 bytes (one halo row of 10
-//    voxels) from one y to the next, so a tap is only a different start address;
-//  * per three taps (one x-row of the stencil; nine -- a z-plane of it -- when
-//    C_out > 128), a TMA load brings their weights for the slice (3 or 9 x C_out
-//    rows of 32 bytes, in the 32-byte swizzle) into a ring of stages: each tap
-//    feeds one MMA per z-plane (BZ = 2 z-planes, each accumulator C_out TMEM
-//    columns).
-// One thread issues the copies (waiting for a buffer to be free), one thread
-// issues the MMAs (waiting for it to be full) and returns each buffer with
-// tcgen05.commit.  The four warps then read the accumulators from TMEM (warp w
-// owns TMEM lanes 32w..32w+31: the rows y = 4w..4w+3 of the tile), add the bias,
-// apply the ReLU and store BF16 (and optionally FP32) channels-last.
+// Implicit GEMM, z-stacked.  One CTA computes a column of 8 (x) x 16 (y) x bz (z)
+// voxels for `ct` output channels: one FP32 accumulator of ct TMEM columns per plane.
+// The reduction runs over C_in in slices of 16 channels (K = 16 of an MMA) and, within
+// a slice, over the bz + 2 input planes and the nine (dy, dx) taps:
+//  * an input plane q feeds the output planes q + 1, q, q - 1 through the taps dz = 0,
+//    1, 2.  Their accumulators are neighbours in TMEM (planes in descending order) and
+//    the weights of the three dz are neighbours in shared memory, so one MMA of
+//    N = 3 ct does the three taps: the A operand, whose read from shared memory (4 KB,
+//    32 cycles) bounds an MMA of N < 128, is read once instead of three times;
+//  * a TMA load brings an input plane with its halo -- 10 x 18 voxels, up to 64
+//    channels, positions outside the volume (and channels past C_in) read as zeros,
+//    which is the convolution's zero padding -- as rows of 32, 64 or 128 bytes in the
+//    swizzle of that width.  The swizzle is a function of the shared-memory address, so
+//    a tap (dy, dx) is a start address in the tile and a 16-channel slice another, with
+//    8-row groups (8 consecutive x) one halo row of 10 voxels apart.  TMA moves about
+//    one row a cycle whatever its width: with two loads of 8 channels (16-byte rows) per
+//    slice it took 365 cycles a plane and slice, more than the nine MMAs;
+//  * per slice, three TMA loads (one per dy) bring the 27 taps' weights, rows of 32
+//    bytes in the 32-byte swizzle, ordered dx, dz, output channel; two buffers.
+// Per output value the products are added in the order slice, dz, dy, dx, whatever the
+// tile: the same order, and the same bits, as k_conv_brick (mma.sync); so the planes of
+// a load stay in shared memory until their last slice is done.  The accumulators start
+// as zeros.  Only MMAs of one accumulator range and shape are ordered by the hardware,
+// so the MMAs of a plane wait for those of the plane before to complete (about 250
+// cycles); a CTA therefore works on one or two such columns in turn (cols), and several
+// CTAs share an SM where TMEM and shared memory allow, to keep the pipe busy.
+// CTAs are persistent.  One thread loads planes, one weights; one warp, in uniform
+// control flow (its elected lane issues), the MMAs, and returns each buffer with
+// tcgen05.commit; four warps read the accumulators from TMEM (TMEM lanes 32w..32w+31:
+// the rows y = 4w..4w+3 of the tile), add the bias, apply the ReLU, store BF16 (and
+// optionally FP32) channels-last and clear the accumulators again.  Each of these runs
+// ahead of the next, into the next tile: with one tile a CTA the first loads (4,000
+// cycles), the MMAs (12,000) and the epilogue (7,000) of a 16-channel tile ran one after
+// the other, on all SMs at once.  The tile (ct, bz, cols) and the number of sets of
+// accumulators are chosen per call by conv_plan.  An MMA costs an SM max(N / 2,
+// 36 + N / 5) cycles (measured, M = 128, K = 16, any layout), so stacking dz also lifts
+// the pipe's use from 21 % (N = 16) to 55 %.  What bounds it now: the turns of the
+// columns (waits and issue), 1,000 to 2,000 cycles for 350 to 860 cycles of MMAs.
+// Measured at batch 4, C_in -> C_out at voxels (us; before: one MMA per tap and plane,
+// tiles of 8 x 16 x 2, one tile a CTA, 16-byte rows): 16 -> 16 at 96^3 208 -> 79,
+// 64 -> 16 568 -> 258, 16 -> 64 412 -> 226; 48 -> 48 at 48^3 89 -> 65, 144 -> 48
+// 214 -> 147, 48 -> 144 226 -> 172; 96 -> 96 at 24^3 44 -> 41, 288 -> 96 103 -> 84,
+// 96 -> 288 309 (mma.sync) -> 100; 192 -> 192 at 12^3 95 (mma.sync) -> 34.
 //
 // Every wait is bounded: a wait that gives up sets g_tc_err (read back by
 // hlbg_nn_tc_error), the CTA waits (bounded) for the copies it issued, frees its
@@ -36,22 +57,19 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <mutex>
 
 #include "../../include/hemelb_gb300_nn.h"
 
 namespace {
 
-constexpr int kM = 128;                      // rows of one MMA: an 8 x 16 plane of voxels
-constexpr int kHX = 10, kHY = 18;            // input tile with its halo in x and y
-// z-planes per CTA (MMAs per weight stage): BZ; the input tile is BZ + 2 deep
-template <int BZ>
-struct Tile {
-  static constexpr int kHZ = BZ + 2;
-  static constexpr int kAPlane = kHX * kHY * kHZ * 16;  // bytes of 8 channels of the tile
-  static constexpr int kATile = 2 * kAPlane;            // one 16-channel slice
-};
-constexpr int kMaxBStages = 16;
+constexpr int kM = 128;            // rows of one MMA: an 8 x 16 plane of voxels
+constexpr int kHX = 10, kHY = 18;  // input plane with its halo in x and y
+constexpr int kRows = kHX * kHY;
+constexpr int kMaxAStages = 40;
+// Bytes of a plane's stage for rows of `span` bytes: whole swizzle atoms of 8 rows.
+__host__ __device__ constexpr int stage_bytes(int span) { return (kRows * span + 8 * span - 1) / (8 * span) * (8 * span); }
 constexpr int64_t kWaitLimit = 1ll << 22;    // polls before a wait gives up
 
 __device__ int g_tc_err;
@@ -82,6 +100,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return false;
 }
 
+// The same by a whole warp, one answer for all its lanes.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+}
+
+// 32 bytes to a 32-byte aligned address: one whole sector.
+__device__ __forceinline__ void store32(void* p, const uint32_t* v) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+
 __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1,
                                             int c2, int c3, int c4) {
   asm volatile(
@@ -91,39 +121,26 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1,
-                                            int c2) {
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1,
+                                            int c2, int c3) {
   asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], "
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], "
       "[%2];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
 
-// Shared-memory matrix descriptor of a K-major operand in the core-matrix layout
-// without swizzle (core matrix: 8 rows x 16 bytes, contiguous): start address,
-// leading-dimension offset = bytes between the two core matrices along K (the two
-// 8-channel planes), stride-dimension offset = bytes between consecutive 8-row
-// groups, the descriptor version of tcgen05 (1) and layout code 0 (no swizzle).
-__device__ __forceinline__ uint64_t desc_noswizzle(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-  d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
-  d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
-  d |= (uint64_t)1u << 46;
-  return d;
-}
-
-// The same for a K-major tile of 32-byte rows (16 BF16) in the 32-byte swizzle
-// (the layout TMA writes with CU_TENSOR_MAP_SWIZZLE_32B): 8-row groups 256 bytes
-// apart, leading offset unused (1 by convention), layout code 6.
-__device__ __forceinline__ uint64_t desc_sw32(uint32_t saddr) {
+// Shared-memory matrix descriptor of a K-major tile of rows of `span` bytes (32, 64 or
+// 128) in the swizzle of that width (the layout TMA writes): start address, bytes
+// between 8-row groups, leading offset unused (1 by convention), the descriptor version
+// of tcgen05 (1), layout code 6, 4 or 2.
+__device__ __forceinline__ uint64_t desc_swizzled(uint32_t saddr, uint32_t span, uint32_t group) {
   uint64_t d = 0;
   d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
   d |= (uint64_t)1u << 16;
-  d |= (uint64_t)((256u >> 4) & 0x3FFFu) << 32;
+  d |= (uint64_t)((group >> 4) & 0x3FFFu) << 32;
   d |= (uint64_t)1u << 46;
-  d |= (uint64_t)6u << 61;
+  d |= (uint64_t)(span == 32u ? 6u : (span == 64u ? 4u : 2u)) << 61;
   return d;
 }
 
@@ -133,16 +150,24 @@ __device__ __forceinline__ uint32_t idesc_bf16(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
 }
 
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
+// D += A B, the descriptors given as their words.
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint32_t a_hi, uint32_t a_lo, uint32_t b_hi, uint32_t b_lo,
+                                          uint32_t idesc) {
   asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+      "{\n .reg .b64 a, b;\n mov.b64 a, {%2, %1};\n mov.b64 b, {%4, %3};\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, 1;\n}\n" ::"r"(tmem_d),
+      "r"(a_hi), "r"(a_lo), "r"(b_hi), "r"(b_lo), "r"(idesc));
 }
 
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+               : "memory");
+}
+
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(
+                   taddr),
+               "r"(0u)
                : "memory");
 }
 
@@ -153,190 +178,360 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
+}  // valid after tcgen05.wait::ld
 
+// SPAN: bytes of a row of an input plane, 32, 64 or 128 (16, 32 or 64 channels).  FULL:
+// 3x3x3, else 1x1x1.
 struct TcParams {
-  int Cin, Cout, N, D, H, W, taps, relu;
-  int nbx, nby, nbz;
-  int b_stages;          // weight stages in the ring (<= kMaxBStages)
-  int tps;               // taps per weight stage (3: one x-row of taps; 1 for a 1x1x1 convolution)
-  int b_stride;          // bytes of one weight stage (C_out x 32, rounded up to 128)
-  uint32_t ncols;        // TMEM columns allocated (a power of two >= 32 and >= 2 C_out)
+  int Cin, Cout, D, H, W, relu;
+  int ct, bz, cols;      // output channels, planes of a column, columns (consecutive in z) of a tile
+  int nbx, nby, nbz;     // tiles along x, y, z
+  int tiles;             // nbx nby nbz N
+  int a_stages;          // input planes in the ring (<= kMaxAStages; at least one load's of a tile)
+  int b_buffers;         // weight buffers: 2, or 1 for one slice (loaded once)
+  int t_buffers;         // sets of accumulators: 1 or 2
+  int wide;              // the outputs start on 32-byte boundaries: whole-sector stores
+  uint32_t b_bytes;      // bytes of one (slice) weight buffer: taps x ct x 32
+  uint32_t ncols;        // TMEM columns allocated (a power of two >= 32 and >= t_buffers cols bz ct)
   const float* bias;     // [C_out] or null
   __nv_bfloat16* out;    // [voxels][C_out]
   float* out_f32;        // [voxels][C_out] or null
 };
 
-template <int BZ>
-__global__ void __launch_bounds__(128, 1) k_conv3d_tc(const __grid_constant__ CUtensorMap tin,
+// One spatial tile: 8 x 16 voxels by cols columns of bz planes (fewer at the volume's
+// end: whole columns, then one of `rem` planes).
+struct TileAt {
+  int n, x0, y0, z0, depth, whole, rem;
+  __device__ __forceinline__ TileAt(const TcParams& p, int t) {
+    x0 = t % p.nbx * 8;
+    t /= p.nbx;
+    y0 = t % p.nby * 16;
+    t /= p.nby;
+    z0 = t % p.nbz * p.bz * p.cols;
+    n = t / p.nbz;
+    depth = min(p.bz * p.cols, p.D - z0);
+    whole = depth / p.bz;
+    rem = depth - whole * p.bz;
+  }
+  // output planes of column c; columns that read an input plane q of theirs; input planes
+  __device__ __forceinline__ int planes(const TcParams& p, int c) const { return c < whole ? p.bz : (c == whole ? rem : 0); }
+  __device__ __forceinline__ int readers(int q, int halo) const { return whole + (rem > 0 && q < rem + 2 * halo ? 1 : 0); }
+  __device__ __forceinline__ int inputs(const TcParams& p, int halo) const {
+    return whole * (p.bz + 2 * halo) + (rem > 0 ? rem + 2 * halo : 0);
+  }
+  __device__ __forceinline__ int most(const TcParams& p, int halo) const { return (whole > 0 ? p.bz : rem) + 2 * halo; }
+};
+
+// Warps 0 and 1: loads; 2, 3 and 8, 9: MMAs of columns 0, 1 and 2, 3; 4-7: epilogue.
+constexpr int kMaxCols = 4;
+constexpr int conv_threads(int cols) { return cols > 2 ? 320 : 256; }
+
+template <uint32_t SPAN, bool FULL>
+__global__ void __launch_bounds__(320, 2) k_conv3d_tc(const __grid_constant__ CUtensorMap tin,
                                                       const __grid_constant__ CUtensorMap tw, TcParams p) {
-  constexpr int kBZ = BZ, kAPlane = Tile<BZ>::kAPlane, kATile = Tile<BZ>::kATile;
-  constexpr int kARegion = (2 * kATile + 1023) / 1024 * 1024;  // the weight stages start 1024-aligned
   extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(16) float bias_sh[256];
+  __shared__ __align__(8) uint64_t bars[2 * kMaxAStages + 8 + kMaxCols];
+  __shared__ uint32_t tmem_slot;
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  // [input slice buffer 0 | buffer 1 | weight stages | barriers | TMEM address]
-  const uint32_t a_base = smem_u32(base);
-  const uint32_t b_base = a_base + kARegion;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(base + kARegion + p.b_stages * p.b_stride);
-  const uint32_t afull0 = smem_u32(bars), aempty0 = afull0 + 16, bfull0 = afull0 + 32,
-                 bempty0 = bfull0 + 8 * kMaxBStages, done = bempty0 + 8 * kMaxBStages;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4 + 2 * kMaxBStages + 1);
+  // [input plane stages | weight buffers]
+  constexpr uint32_t stage = (uint32_t)stage_bytes(SPAN);
+  const uint32_t a_base = smem_u32(base), b_base = a_base + ((p.a_stages * stage + 1023u) & ~1023u);
+  const uint32_t afull0 = smem_u32(bars), aempty0 = afull0 + 8 * kMaxAStages, bfull0 = aempty0 + 8 * kMaxAStages,
+                 bempty0 = bfull0 + 16, tfull0 = bempty0 + 16, tempty0 = tfull0 + 16, col0 = tempty0 + 16;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int co0 = blockIdx.y * p.ct;
+  constexpr int halo = FULL ? 1 : 0;  // input planes below and above a column
+  constexpr int per_load = SPAN / 32;
+  const int kslices = p.Cin / 16;
+  const int loads = (kslices + per_load - 1) / per_load;
+  const int AS = p.a_stages, BB = p.b_buffers, TB = p.t_buffers;
+  const int set = p.cols * p.bz * p.ct;  // columns of one set of accumulators
 
-  int bid = blockIdx.x;
-  const int bx = bid % p.nbx;
-  bid /= p.nbx;
-  const int by = bid % p.nby;
-  bid /= p.nby;
-  const int bz = bid % p.nbz;
-  const int n = bid / p.nbz;
-  const int x0 = bx * 8, y0 = by * 16, z0 = bz * kBZ;
-
+  if (threadIdx.x == 32) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tin)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tw)) : "memory");
+  }
   if (threadIdx.x == 0) {
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < AS; ++s) {
       mbar_init(afull0 + 8 * s, 1);
       mbar_init(aempty0 + 8 * s, 1);
     }
-    for (int s = 0; s < p.b_stages; ++s) {
+    for (int s = 0; s < 2; ++s) {
       mbar_init(bfull0 + 8 * s, 1);
-      mbar_init(bempty0 + 8 * s, 1);
+      mbar_init(bempty0 + 8 * s, p.cols);
+      mbar_init(tfull0 + 8 * s, p.cols);
+      mbar_init(tempty0 + 8 * s, 4);
     }
-    mbar_init(done, 1);
+    for (int c = 0; c < kMaxCols; ++c) mbar_init(col0 + 8 * c, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
                  "r"(p.ncols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  if (warp >= 4 && warp < 8)
+    for (int c = threadIdx.x - 128; c < p.ct; c += 128) bias_sh[c] = p.bias ? __ldg(p.bias + co0 + c) : 0.f;
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = tmem_slot;
 
-  const int kslices = p.Cin / 16;
-  const int SB = p.b_stages;
-  const int groups = p.taps / p.tps;  // weight stages per channel slice
-  const uint32_t b_bytes = (uint32_t)(p.tps * p.Cout * 32);
-  if (warp == 0 && lane == 0) {
-    // producer
-    int a_issued = 0, b_issued = 0;
-    bool ok = true;
-    for (int ks = 0; ks < kslices && ok; ++ks) {
-      const int a = ks & 1;
-      if (!mbar_wait(aempty0 + 8 * a, ((uint32_t)(ks >> 1) & 1u) ^ 1u)) {
-        ok = false;
-        break;
+  if (warp == 0) {
+    // ---- input planes, one thread: per load plane by plane, the columns in turn ----
+    if (lane == 0) {
+      int i = 0, s = 0;
+      uint32_t ph = 1u;
+      bool ok = true;
+      for (int t = blockIdx.x; t < p.tiles && ok; t += gridDim.x) {
+        const TileAt at(p, t);
+        const int most = at.most(p, halo);
+        for (int k = 0; k < loads && ok; ++k)
+          for (int q = 0; q < most && ok; ++q) {
+            const int n = at.readers(q, halo);
+            for (int c = 0; c < n; ++c) {
+              ok = mbar_wait(aempty0 + 8 * s, ph);
+              if (!ok) break;
+              mbar_expect_tx(afull0 + 8 * s, kRows * SPAN);
+              tma_load_5d(a_base + s * stage, &tin, afull0 + 8 * s, k * per_load * 16, at.x0 - 1, at.y0 - 1,
+                          at.z0 + c * p.bz - halo + q, at.n);
+              ++i;
+              if (++s == AS) {
+                s = 0;
+                ph ^= 1u;
+              }
+            }
+          }
       }
-      const uint32_t sa = a_base + a * kATile;
-      mbar_expect_tx(afull0 + 8 * a, (uint32_t)kATile);
-      tma_load_5d(sa, &tin, afull0 + 8 * a, ks * 16, x0 - 1, y0 - 1, z0 - 1, n);
-      tma_load_5d(sa + kAPlane, &tin, afull0 + 8 * a, ks * 16 + 8, x0 - 1, y0 - 1, z0 - 1, n);
-      ++a_issued;
-      for (int tg = 0; tg < groups; ++tg) {
-        const int i = ks * groups + tg, s = i % SB;
-        if (!mbar_wait(bempty0 + 8 * s, ((uint32_t)(i / SB) & 1u) ^ 1u)) {
-          ok = false;
-          break;
-        }
-        const uint32_t sb = b_base + s * p.b_stride;
-        mbar_expect_tx(bfull0 + 8 * s, b_bytes);
-        tma_load_3d(sb, &tw, bfull0 + 8 * s, ks * 16, 0, tg * p.tps);
-        ++b_issued;
+      if (!ok) {
+        atomicExch(&g_tc_err, 1);
+        // the copies in flight land before the CTA's shared memory goes away
+        for (int j = i > AS ? i - AS : 0; j < i; ++j) mbar_wait(afull0 + 8 * (j % AS), (uint32_t)(j / AS) & 1u);
       }
     }
-    if (!ok) {
-      atomicExch(&g_tc_err, 1);
-      // the copies in flight land before the CTA's shared memory goes away
-      for (int j = a_issued > 2 ? a_issued - 2 : 0; j < a_issued; ++j)
-        mbar_wait(afull0 + 8 * (j & 1), (uint32_t)(j >> 1) & 1u);
-      for (int j = b_issued > SB ? b_issued - SB : 0; j < b_issued; ++j)
-        mbar_wait(bfull0 + 8 * (j % SB), (uint32_t)(j / SB) & 1u);
-    }
-  } else if (warp == 1 && lane == 0) {
-    // MMA issuer
-    const uint32_t idesc = idesc_bf16(p.Cout);
-    bool ok = true;
-    for (int ks = 0; ks < kslices && ok; ++ks) {
-      const int a = ks & 1;
-      if (!mbar_wait(afull0 + 8 * a, (uint32_t)(ks >> 1) & 1u)) {
-        ok = false;
-        break;
-      }
-      const uint32_t sa = a_base + a * kATile;
-      for (int tg = 0; tg < groups; ++tg) {
-        const int i = ks * groups + tg, s = i % SB;
-        if (!mbar_wait(bfull0 + 8 * s, (uint32_t)(i / SB) & 1u)) {
-          ok = false;
-          break;
+    __syncwarp();
+  } else if (warp == 1) {
+    // ---- weights, one thread: every slice of every tile; a lone slice once ----
+    if (lane == 0) {
+      const int mine = (p.tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+      const int total = kslices == 1 ? 1 : mine * kslices;
+      const uint32_t row = (uint32_t)p.ct * 32u;  // one tap
+      int i = 0;
+      for (; i < total; ++i) {
+        const int s = i % BB, ks = i % kslices;
+        if (!mbar_wait(bempty0 + 8 * s, ((uint32_t)(i / BB) & 1u) ^ 1u)) break;
+        const uint32_t sb = b_base + s * p.b_bytes;
+        mbar_expect_tx(bfull0 + 8 * s, p.b_bytes);
+        if (FULL) {
+          for (int dy = 0; dy < 3; ++dy) tma_load_4d(sb + dy * 9 * row, &tw, bfull0 + 8 * s, ks * 16, co0, 0, dy * 3);
+        } else {
+          tma_load_4d(sb, &tw, bfull0 + 8 * s, ks * 16, co0, 0, 0);
         }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int j = 0; j < p.tps; ++j) {
-          const int t = tg * p.tps + j;
-          // the tap's offset in the halo tile (a 1x1x1 convolution uses the centre)
-          const int dz = p.taps == 27 ? t / 9 : 1, dy = p.taps == 27 ? (t / 3) % 3 : 1,
-                    dx = p.taps == 27 ? t % 3 : 1;
-          const uint64_t bdesc = desc_sw32(b_base + s * p.b_stride + (uint32_t)(j * p.Cout * 32));
+      }
+      if (i < total) {
+        atomicExch(&g_tc_err, 1);
+        for (int j = i > BB ? i - BB : 0; j < i; ++j) mbar_wait(bfull0 + 8 * (j % BB), (uint32_t)(j / BB) & 1u);
+      }
+    }
+    __syncwarp();
+  } else if (warp < 4 || warp >= 8) {
+    // ---- MMAs of one column, one thread.  Block h of the column's accumulators is its
+    // output plane planes - 1 - h.  The thread's own instructions are what takes the time
+    // (a plane's 9 MMAs take the tensor pipe 350 to 500 cycles, this thread over 1,000
+    // with its waits), hence a thread per column; stage numbers and phases run along
+    // instead of being divided out, and of a descriptor only the low word is added to (its
+    // bits 0-13 are the address in 16 bytes). ----
+    const int c = warp < 4 ? warp - 2 : warp - 6;
+    if (lane == 0 && c < p.cols) {
+      constexpr uint32_t kVox = SPAN >> 4, kRow = kHX * kVox;
+      const int per = 256 / p.ct;                       // planes one MMA covers at most
+      const uint32_t tap = (uint32_t)(p.ct * 2);        // one tap's rows of weights
+      const uint32_t cols1 = (uint32_t)(p.ct >> 3) << 17;  // instruction descriptor: one plane's columns
+      const uint32_t idesc0 = idesc_bf16(0);
+      const uint64_t a_desc = desc_swizzled(a_base, SPAN, kHX * SPAN), b_desc = desc_swizzled(b_base, 32u, 256u);
+      const uint32_t a_hi = (uint32_t)(a_desc >> 32), b_hi = (uint32_t)(b_desc >> 32);
+      const uint32_t a_lo0 = (uint32_t)a_desc, b_lo0 = (uint32_t)b_desc;
+      const uint32_t col = col0 + 8 * c;
+      uint32_t turn = 1u;  // phase of the column's barrier that was armed last
+      bool moved = false;
+      int first = 0, tc = 0, sbuf = 0, tb = 0;
+      uint32_t first_ph = 0u, b_ph = 0u, t_ph = 0u;
+      bool ok = true;
+      for (int t = blockIdx.x; t < p.tiles && ok; t += gridDim.x, ++tc) {
+        const TileAt at(p, t);
+        const int nz = at.planes(p, c), reads = nz > 0 ? nz + 2 * halo : 0, inputs = at.inputs(p, halo);
+        ok = mbar_wait(tempty0 + 8 * tb, t_ph);  // this set is zeroed
+        const uint32_t acc = tmem + (uint32_t)(tb * set + c * p.bz * p.ct);
+        for (int left = kslices; left > 0 && ok; left -= per_load) {
+          const int slices = min(left, per_load);
+          for (int sl = 0; sl < slices && ok; ++sl) {
+            if (kslices > 1 || tc == 0) ok = mbar_wait(bfull0 + 8 * sbuf, b_ph);
+            const uint32_t b_lo = b_lo0 + (uint32_t)sbuf * (p.b_bytes >> 4);
+            int s = first + c;
+            uint32_t ph = first_ph;
+            if (s >= AS) {
+              s -= AS;
+              ph ^= 1u;
+            }
+            for (int q = 0; q < reads && ok; ++q) {
+              if (sl == 0) ok = mbar_wait(afull0 + 8 * s, ph);
+              // the column's previous plane (one outstanding at most: a parity tells no more)
+              if (moved) ok = ok && mbar_wait(col, turn);
+              if (!ok) break;
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              // output planes hi, hi - 1, ..., lo through dz = q - hi, ... (1x1x1: plane q),
+              // at most `per` planes an MMA
+              const int hi = min(q, nz - 1), lo = FULL ? max(q - 2, 0) : q;
+              const uint32_t a_lo = a_lo0 + (uint32_t)s * (stage >> 4) + 2u * (uint32_t)sl;
+              uint32_t dst = acc + (uint32_t)((nz - 1 - hi) * p.ct);
+              uint32_t bd = b_lo + (FULL ? (uint32_t)(q - hi) * tap : 0u);
+              for (int n = hi - lo + 1; n > 0; n -= per) {
+                const int m = min(per, n);
+                const uint32_t idesc = idesc0 + (uint32_t)m * cols1;
+                if (FULL) {
+                  uint32_t bk = bd;
 #pragma unroll
-          for (int pz = 0; pz < kBZ; ++pz) {
-            const uint32_t start = sa + (uint32_t)((((pz + dz) * kHY + dy) * kHX + dx) * 16);
-            umma_bf16(tmem + (uint32_t)(pz * p.Cout), desc_noswizzle(start, (uint32_t)kAPlane, 160u), bdesc,
-                      idesc, (ks | t) != 0 ? 1u : 0u);
+                  for (int k = 0; k < 9; ++k, bk += 3 * tap)
+                    umma_bf16(dst, a_hi, a_lo + (k / 3) * kRow + (k % 3) * kVox, b_hi, bk, idesc);
+                } else {
+                  umma_bf16(dst, a_hi, a_lo + kRow + kVox, b_hi, bd, idesc);
+                }
+                dst += (uint32_t)(m * p.ct);
+                bd += (uint32_t)m * tap;
+              }
+              umma_commit(col);
+              if (sl == slices - 1) umma_commit(aempty0 + 8 * s);
+              moved = true;
+              turn ^= 1u;
+              s += at.readers(q, halo);
+              if (s >= AS) {
+                s -= AS;
+                ph ^= 1u;
+              }
+            }
+            if (kslices > 1) {
+              umma_commit(bempty0 + 8 * sbuf);
+              if (++sbuf == BB) {
+                sbuf = 0;
+                b_ph ^= 1u;
+              }
+            }
+          }
+          first += inputs;
+          if (first >= AS) {
+            first -= AS;
+            first_ph ^= 1u;
           }
         }
-        umma_commit(bempty0 + 8 * s);
+        umma_commit(tfull0 + 8 * tb);  // arrives once every MMA this thread issued has completed
+        if (++tb == TB) {
+          tb = 0;
+          t_ph ^= 1u;
+        }
       }
-      umma_commit(aempty0 + 8 * a);
+      if (!ok) atomicExch(&g_tc_err, 1);
     }
-    if (!ok) atomicExch(&g_tc_err, 1);
-    umma_commit(done);  // arrives once every MMA issued above has completed
-  }
-  __syncwarp();
-
-  // epilogue: TMEM lane = voxel row of a plane (x = row % 8, y = row / 8), columns
-  // [pz C_out, (pz + 1) C_out) = the output channels of z-plane pz
-  const bool finished = mbar_wait(done, 0);
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (!finished && lane == 0) atomicExch(&g_tc_err, 1);
-  const int row = warp * 32 + lane;
-  const int x = x0 + (row & 7), y = y0 + (row >> 3);
-  for (int pz = 0; pz < kBZ; ++pz) {
-    const int z = z0 + pz;
-    const bool inside = finished && x < p.W && y < p.H && z < p.D;
-    const int64_t vox = (((int64_t)n * p.D + z) * p.H + y) * p.W + x;
-    for (int c0 = 0; c0 < p.Cout; c0 += 16) {
-      uint32_t r[16];
-      __syncwarp();  // tcgen05.ld is warp-collective: every lane, converged
-      tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(pz * p.Cout + c0), r);
-      if (!inside) continue;
-      float v[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        v[j] = __uint_as_float(r[j]) + (p.bias ? __ldg(p.bias + c0 + j) : 0.f);
-        if (p.relu) v[j] = fmaxf(v[j], 0.f);
+    __syncwarp();
+  } else {
+    // ---- epilogue: TMEM lane = voxel row of a plane (x = row % 8, y = row / 8) ----
+    const uint32_t mine = tmem + ((uint32_t)((warp - 4) * 32) << 16);
+    auto release = [&](int tb) {  // the set is zeros again
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tempty0 + 8 * tb) : "memory");
+      __syncwarp();
+    };
+    for (int tb = 0; tb < TB; ++tb) {
+      for (int c = 0; c < set; c += 16) tmem_zero16(mine + (uint32_t)(tb * set + c));
+      release(tb);
+    }
+    const int r0 = (warp - 4) * 32 + lane, chunks = p.ct / 16;
+    int tc = 0;
+    for (int t = blockIdx.x; t < p.tiles; t += gridDim.x, ++tc) {
+      const TileAt at(p, t);
+      const int tb = tc % TB;
+      if (!warp_wait(tfull0 + 8 * tb, (uint32_t)(tc / TB) & 1u)) {
+        if (lane == 0) atomicExch(&g_tc_err, 1);
+        break;
       }
-      uint32_t packed[8];
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int x = at.x0 + (r0 & 7), y = at.y0 + (r0 >> 3);
+      const bool inside = x < p.W && y < p.H;
+      const int steps = at.depth * chunks;
+      // step k: output plane k / chunks, 16 channels; the next step's accumulators are read
+      // while this one's are stored
+      auto column_of = [&](int k) {
+        const int pz = k / chunks, c = pz / p.bz;
+        return (uint32_t)(tb * set + (c * p.bz + at.planes(p, c) - 1 - (pz - c * p.bz)) * p.ct + (k - pz * chunks) * 16);
+      };
+      uint32_t r[2][16];
+      tmem_ld16(mine + column_of(0), r[0]);
+#pragma unroll 2
+      for (int k = 0; k < steps; ++k) {
+        uint32_t* cur = r[k & 1];
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-        packed[j] = *reinterpret_cast<const uint32_t*>(&h);
+        for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(cur[j]));  // the values are there from here on
+        if (k + 1 < steps) tmem_ld16(mine + column_of(k + 1), r[(k + 1) & 1]);
+        if (inside) {
+          const int pz = k / chunks, c0 = (k - pz * chunks) * 16;
+          const int64_t voxel = (((int64_t)at.n * p.D + at.z0 + pz) * p.H + y) * p.W + x;
+          float v[16];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float4 bv = *reinterpret_cast<const float4*>(bias_sh + c0 + 4 * j);
+            v[4 * j] = __uint_as_float(cur[4 * j]) + bv.x;
+            v[4 * j + 1] = __uint_as_float(cur[4 * j + 1]) + bv.y;
+            v[4 * j + 2] = __uint_as_float(cur[4 * j + 2]) + bv.z;
+            v[4 * j + 3] = __uint_as_float(cur[4 * j + 3]) + bv.w;
+          }
+          if (p.relu) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j], 0.f);
+          }
+          uint32_t packed[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+            packed[j] = *reinterpret_cast<const uint32_t*>(&h);
+          }
+          __nv_bfloat16* dst = p.out + voxel * p.Cout + co0 + c0;
+          if (p.wide) {
+            store32(dst, packed);
+          } else {
+            reinterpret_cast<uint4*>(dst)[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            reinterpret_cast<uint4*>(dst)[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+          }
+          if (p.out_f32) {
+            float* df = p.out_f32 + voxel * p.Cout + co0 + c0;
+            if (p.wide) {
+              store32(df, reinterpret_cast<const uint32_t*>(v));
+              store32(df + 8, reinterpret_cast<const uint32_t*>(v + 8));
+            } else {
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                reinterpret_cast<float4*>(df)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            }
+          }
+        }
+        __syncwarp();  // tcgen05.ld is warp-collective: every lane, converged
       }
-      uint4* dst = reinterpret_cast<uint4*>(p.out + vox * p.Cout + c0);
-      dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-      dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-      if (p.out_f32) {
-        float4* df = reinterpret_cast<float4*>(p.out_f32 + vox * p.Cout + c0);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) df[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+      if (t + (int)gridDim.x * TB < p.tiles) {  // the set is used again
+        for (int c = 0; c < set; c += 16) tmem_zero16(mine + (uint32_t)(tb * set + c));
+        release(tb);
       }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0)
+  if (warp == 2) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(p.ncols) : "memory");
+  }
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -353,6 +548,116 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
+// Shared memory of an SM, what a CTA reserves and has as static arrays, and the most a
+// CTA may ask for on top of these.
+constexpr int kSmemSm = 233472, kSmemFixed = 1024 + 2048, kSmemDyn = 232448 - 2048;
+constexpr int kSms = 152;
+
+// Tile of a convolution (see TcParams) and the shared memory that goes with it.
+struct Plan {
+  int ct, bz, cols, span, tb, tmem, per_sm, a_stages, b_buffers, smem;
+};
+
+// Modelled cycles of an MMA of n columns on an SM's tensor pipe.
+double mma_cost(int n) { return std::max(n / 2.0, 36.0 + n / 5.0); }
+
+// Whether a tile fits, with per_sm CTAs on an SM: tb sets of accumulators within 512
+// TMEM columns, and within an equal share of shared memory (which is also requested, so
+// that no more CTAs come) the planes of one load and the weight buffers.
+bool conv_fit(int cin, int taps, int ct, int bz, int cols, int span, int tb, int per_sm, Plan& pl) {
+  int tmem = 32;
+  while (tmem < tb * cols * bz * ct) tmem *= 2;
+  if (per_sm * tmem > 512) return false;
+  const int smem = std::min(kSmemSm / per_sm - kSmemFixed, kSmemDyn);
+  const int slices = cin / 16, bufs = slices > 1 ? 2 : 1, weights = bufs * taps * ct * 32;
+  const int planes = cols * (bz + (taps == 27 ? 2 : 0)), loads = (slices * 32 + span - 1) / span;
+  const int room = (smem - 2 * 1024 - weights) / stage_bytes(span);  // both regions start 1024-aligned
+  const int stages = std::min({room, kMaxAStages, 2 * planes * loads});
+  if (stages < planes) return false;
+  pl = Plan{ct, bz, cols, span, tb, tmem, per_sm, stages, bufs, smem};
+  return true;
+}
+
+// Modelled cycles of the whole convolution.  The columns that share an SM take turns on
+// its tensor pipe, a plane and slice at a time; a turn also waits for its own last one
+// (kTurn, seen to fall with the number of columns).  A CTA's tile is its turns and, with
+// one set of accumulators, its epilogue (kStep per plane and 16 channels); the SM's TMA
+// rows (one a cycle) and bytes (loads and stores at 48 a cycle) bound it from below.
+double conv_time(int cin, int cout, int n, int d, int h, int wd, int taps, const Plan& pl) {
+  constexpr double kTurn = 1000.0, kLaunch = 6000.0, kStep = 500.0;
+  const int slices = cin / 16, planes = pl.bz + (taps == 27 ? 2 : 0), per = 256 / pl.ct;
+  const int loads = (slices * 32 + pl.span - 1) / pl.span;
+  const int columns = (d + pl.bz - 1) / pl.bz, ny = cout / pl.ct;
+  const int64_t tiles = (int64_t)n * ((wd + 7) / 8) * ((h + 15) / 16) * ((columns + pl.cols - 1) / pl.cols);
+  const int64_t ctas = std::min<int64_t>(tiles, std::max(1, kSms * pl.per_sm / ny)) * ny;
+  const double resident = std::max(1.0, std::min((double)pl.per_sm, (double)ctas / kSms));
+  const double tiles_per_cta = std::ceil((double)(tiles * ny) / (double)ctas);
+  double mma = 0;  // tensor cycles of a column's planes, one slice
+  for (int q = 0; q < planes; ++q) {
+    const int first = taps == 27 ? std::max(q - 2, 0) : q, end = taps == 27 ? std::min(q, pl.bz - 1) : q;
+    for (int m = end - first + 1; m > 0; m -= per) mma += (taps == 27 ? 9 : 1) * mma_cost(std::min(m, per) * pl.ct);
+  }
+  const double chains = resident * pl.cols;
+  const double turns = slices * (chains * mma + planes * kTurn / std::sqrt(chains));
+  const double rows = (double)pl.cols * planes * loads * kRows + (slices > 1 ? (double)slices * taps * pl.ct : 0.0);
+  const double bytes = (double)pl.cols * planes * kRows * cin * 2 +
+                       (slices > 1 ? (double)slices * taps * pl.ct * 32 : 0.0) + (double)pl.cols * pl.bz * pl.ct * 256;
+  const double epi = kStep * pl.cols * pl.bz * pl.ct / 16;
+  const double tile = std::max({pl.tb > 1 ? std::max(turns, epi) : turns + epi, resident * rows, resident * bytes / 48.0});
+  return tiles_per_cta * tile + kLaunch + epi;
+}
+
+// The tile with the smallest modelled time: output channels a multiple of 16 that
+// divides C_out (at most 256), every useful column height, one or two columns and sets
+// of accumulators, rows as wide as the channels allow or narrower (fewer bytes a plane).
+bool conv_plan(int cin, int cout, int n, int d, int h, int wd, int taps, Plan& best) {
+  double best_t = 0;
+  bool found = false;
+  for (int ct = 16; ct <= std::min(cout, 256); ct += 16) {
+    if (cout % ct) continue;
+    for (int bz = 1; bz <= std::min(d, 32) && bz * ct <= 512; ++bz) {
+      const int columns = (d + bz - 1) / bz;
+      if (bz > 1 && columns == (d + bz - 2) / (bz - 1)) continue;  // as many columns with fewer planes
+      for (int cols = 1; cols <= std::min(kMaxCols, columns); ++cols)
+        for (int span = 32; span <= 128 && (span == 32 || (taps == 27 && span < cin * 4)); span *= 2)
+          for (int tb = 1; tb <= 2; ++tb)
+            for (int per_sm = 3; per_sm >= 1; --per_sm) {
+              Plan pl;
+              if (!conv_fit(cin, taps, ct, bz, cols, span, tb, per_sm, pl)) continue;
+              const double t = conv_time(cin, cout, n, d, h, wd, taps, pl);
+              if (!found || t < best_t) {
+                found = true;
+                best_t = t;
+                best = pl;
+              }
+            }
+    }
+  }
+  return found;
+}
+
+// conv_plan takes 10 to 40 us of host time, so each thread keeps the plans of the last
+// shapes it asked for (a fixed table, by the shape alone).
+bool planned(int cin, int cout, int n, int d, int h, int wd, int taps, Plan& pl) {
+  struct Entry {
+    int shape[7];
+    Plan plan;
+  };
+  static thread_local Entry table[64] = {};
+  const int shape[7] = {cin, cout, n, d, h, wd, taps};
+  uint32_t hash = 0;
+  for (int v : shape) hash = hash * 2654435761u + (uint32_t)v;
+  Entry& e = table[hash >> 26];
+  if (!std::equal(shape, shape + 7, e.shape)) {  // a zeroed entry has no valid shape
+    Plan found;
+    if (!conv_plan(cin, cout, n, d, h, wd, taps, found)) return false;
+    std::copy(shape, shape + 7, e.shape);
+    e.plan = found;
+  }
+  pl = e.plan;
+  return true;
+}
+
 }  // namespace
 
 extern "C" {
@@ -360,7 +665,7 @@ extern "C" {
 int hlbg_nn_conv3d_tc(const void* in, int32_t cin, const void* w, const float* bias, void* out, float* out_f32,
                       int32_t cout, int32_t n, int32_t d, int32_t h, int32_t wd, int32_t taps, int32_t relu,
                       void* stream) {
-  if (!in || !w || !out || cin <= 0 || cin % 16 || cout < 16 || cout > 256 || cout % 16 || n <= 0 || d <= 0 ||
+  if (!in || !w || !out || cin <= 0 || cin % 16 || cout < 16 || cout % 16 || n <= 0 || d <= 0 ||
       h <= 0 || wd <= 0 || (taps != 27 && taps != 1))
     return 1;
   // TMA: 16-byte aligned base addresses; the output is stored in 16-byte vectors
@@ -369,27 +674,31 @@ int hlbg_nn_conv3d_tc(const void* in, int32_t cin, const void* w, const float* b
     return 1;
   auto enc = encode_fn();
   if (!enc) return 3;
-  // z-planes per CTA.  Four planes per weight stage (C_out <= 128) measured slower
-  // than two on the network's shapes (fewer CTAs per SM), so two throughout.
-  const int bz = 2;
+  Plan pl;
+  if (!planned(cin, cout, n, d, h, wd, taps, pl)) return 1;
   CUtensorMap tin, tw;
   {
     const cuuint64_t dims[5] = {(cuuint64_t)cin, (cuuint64_t)wd, (cuuint64_t)h, (cuuint64_t)d, (cuuint64_t)n};
     const cuuint64_t strides[4] = {(cuuint64_t)cin * 2, (cuuint64_t)cin * 2 * wd, (cuuint64_t)cin * 2 * wd * h,
                                    (cuuint64_t)cin * 2 * wd * h * d};
-    const cuuint32_t box[5] = {8, (cuuint32_t)kHX, (cuuint32_t)kHY, (cuuint32_t)(bz + 2), 1};
+    const cuuint32_t box[5] = {(cuuint32_t)(pl.span / 2), (cuuint32_t)kHX, (cuuint32_t)kHY, 1, 1};
+    const CUtensorMapSwizzle swizzle = pl.span == 32 ? CU_TENSOR_MAP_SWIZZLE_32B
+                                                     : (pl.span == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
     const cuuint32_t es[5] = {1, 1, 1, 1, 1};
     if (enc(&tin, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(in), dims, strides, box, es,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return 3;
   }
   {
-    const cuuint64_t dims[3] = {(cuuint64_t)cin, (cuuint64_t)cout, (cuuint64_t)taps};
-    const cuuint64_t strides[2] = {(cuuint64_t)cin * 2, (cuuint64_t)cin * 2 * cout};
-    const cuuint32_t box[3] = {16, (cuuint32_t)cout, (cuuint32_t)(taps == 27 ? (2 * cout > 256 ? 9 : 3) : 1)};
-    const cuuint32_t es[3] = {1, 1, 1};
-    if (enc(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(w), dims, strides, box, es,
+    // w[(dz * 9 + dy * 3 + dx)][co][ci] seen as [dy * 3 + dx][dz][co][ci]
+    const bool full = taps == 27;
+    const cuuint64_t tap = (cuuint64_t)cin * 2 * cout;
+    const cuuint64_t dims[4] = {(cuuint64_t)cin, (cuuint64_t)cout, full ? 3u : 1u, full ? 9u : 1u};
+    const cuuint64_t strides[3] = {(cuuint64_t)cin * 2, full ? 9 * tap : tap, tap};
+    const cuuint32_t box[4] = {16, (cuuint32_t)pl.ct, full ? 3u : 1u, full ? 3u : 1u};
+    const cuuint32_t es[4] = {1, 1, 1, 1};
+    if (enc(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(w), dims, strides, box, es,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return 3;
@@ -397,53 +706,44 @@ int hlbg_nn_conv3d_tc(const void* in, int32_t cin, const void* w, const float* b
   TcParams p{};
   p.Cin = cin;
   p.Cout = cout;
-  p.N = n;
   p.D = d;
   p.H = h;
   p.W = wd;
-  p.taps = taps;
   p.relu = relu;
+  p.ct = pl.ct;
+  p.bz = pl.bz;
+  p.cols = pl.cols;
   p.nbx = (wd + 7) / 8;
   p.nby = (h + 15) / 16;
-  p.nbz = (d + bz - 1) / bz;
-  uint32_t cols = 32;
-  while (cols < (uint32_t)(bz * cout)) cols *= 2;
-  p.ncols = cols;
-  // taps per weight stage: one x-row of the stencil (3), or a whole z-plane of it (9)
-  // when 2 C_out > 256 TMEM columns leave the SM to one CTA anyway (measured: 9
-  // is faster there, 3 where two or more CTAs share an SM)
-  p.tps = taps == 27 ? (2 * cout > 256 ? 9 : 3) : 1;
-  p.b_stride = (p.tps * cout * 32 + 1023) / 1024 * 1024;  // swizzled TMA destinations: 1024-byte aligned
+  p.nbz = (d + pl.bz * pl.cols - 1) / (pl.bz * pl.cols);
+  const int64_t tiles = (int64_t)n * p.nbz * p.nby * p.nbx;
+  if (tiles > 0x3fffffff) return 1;
+  p.tiles = (int)tiles;
+  p.a_stages = pl.a_stages;
+  p.b_buffers = pl.b_buffers;
+  p.t_buffers = pl.tb;
+  p.b_bytes = (uint32_t)(taps * pl.ct * 32);
+  p.ncols = (uint32_t)pl.tmem;
   p.bias = bias;
   p.out = static_cast<__nv_bfloat16*>(out);
   p.out_f32 = out_f32;
-  // CTAs per SM: at most what its 512 TMEM columns hold (an allocation beyond them
-  // would wait), at most 4; each gets an equal share of the
-  // SM's shared memory, which is also its floor (so no more CTAs fit), and fills
-  // it with weight stages
-  const int a_tile = Tile<2>::kATile;
-  const int fixed = 1024 + (2 * a_tile + 1023) / 1024 * 1024 + (4 + 2 * kMaxBStages + 1) * 8 + 16;
-  // fewer CTAs per SM when four weight stages would not fit in an equal share
-  int per_sm = std::min(512 / (int)cols, 4), share = 0;
-  for (;; --per_sm) {
-    share = 233472 / per_sm - 1024;  // per-SM capacity less the per-CTA reserve
-    p.b_stages = std::min(kMaxBStages, (std::min(share, 232448) - fixed) / p.b_stride);
-    if (p.b_stages >= 4 || per_sm == 1) break;
-  }
-  if (p.b_stages < 2) return 1;
-  const int smem = std::min(share, 232448);
-  // the opt-in shared-memory limit is a per-device attribute of the kernel
+  p.wide = ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_f32)) & 31u) == 0;
+  const auto kernel = taps == 1 ? k_conv3d_tc<32, false>
+                      : pl.span == 32 ? k_conv3d_tc<32, true>
+                                      : (pl.span == 64 ? k_conv3d_tc<64, true> : k_conv3d_tc<128, true>);
+  // the opt-in shared-memory limit is a per-device attribute of each kernel
   static std::atomic<bool> configured[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 3;
   if (!configured[dev].load()) {
-    if (cudaFuncSetAttribute(k_conv3d_tc<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448) != cudaSuccess)
-      return 3;
+    for (auto k : {k_conv3d_tc<32, false>, k_conv3d_tc<32, true>, k_conv3d_tc<64, true>, k_conv3d_tc<128, true>})
+      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemDyn) != cudaSuccess) return 3;
     configured[dev].store(true);
   }
-  const int64_t grid = (int64_t)n * p.nbz * p.nby * p.nbx;
-  if (grid > 0x7fffffff) return 1;
-  k_conv3d_tc<2><<<(unsigned)grid, 128, smem, static_cast<cudaStream_t>(stream)>>>(tin, tw, p);
+  // persistent CTAs, as many as the SMs hold, over the tiles of each block of output channels
+  const int ny = cout / pl.ct;
+  const unsigned gx = (unsigned)std::min<int64_t>(tiles, std::max(1, kSms * pl.per_sm / ny));
+  kernel<<<dim3(gx, (unsigned)ny), conv_threads(pl.cols), pl.smem, static_cast<cudaStream_t>(stream)>>>(tin, tw, p);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 

@@ -41,19 +41,19 @@ def _ok(rc, what):
 
 
 def tc_eligible(cin: int, cout: int, *tensors) -> bool:
-    """Shapes the tcgen05 convolution takes: C_in a multiple of 16, C_out a multiple
-    of 16 up to 256, 16-byte aligned buffers."""
-    return (cin % 16 == 0 and cout % 16 == 0 and 16 <= cout <= 256
+    """Shapes the tcgen05 convolution takes: C_in and C_out multiples of 16, 16-byte
+    aligned buffers."""
+    return (cin % 16 == 0 and cout % 16 == 0 and cout >= 16
             and all(t is None or t.data_ptr() % 16 == 0 for t in tensors))
 
 
-def tc_tiles(n: int, d: int, h: int, w: int) -> int:
-    """CTAs of the tcgen05 convolution: one per 8 x 16 x 2 output tile."""
-    return n * -(-d // 2) * -(-h // 16) * -(-w // 8)
-
-
-# Below one tile per SM the mma.sync kernel is faster (measured on the 12^3 layers).
-_TC_MIN_TILES = 152
+def tc_faster(cin: int, cout: int, voxels: int, taps: int) -> bool:
+    """Where the tcgen05 convolution is the faster one (the two give the same bits): all
+    but small volumes at 16 -> 16 channels and of the 1x1x1 convolution, whose one slice
+    the mma.sync kernel finishes in less than a tcgen05 CTA's set-up.  Measured, us,
+    mma.sync / tcgen05: 16 -> 16 at 12^3 4.3 / 5.2, 24^3 6.0 / 6.5, 48^3 20.5 / 13.7;
+    48 -> 48 at 8^3 9.4 / 9.1; 192 -> 192 at 6^3 61 / 27."""
+    return voxels >= 1 << 15 or (taps == 27 and cin * cout > 256)
 
 
 def conv3d(x, w, bias, out, out_f32=None, taps=27, relu=False, engine="auto"):
@@ -74,7 +74,7 @@ def conv3d(x, w, bias, out, out_f32=None, taps=27, relu=False, engine="auto"):
     if out_f32 is not None:
         _need(out_f32, _F32, "conv3d FP32 output")
     if engine == "auto":
-        engine = ("tc" if tc_eligible(cin, cout, x, w, out, out_f32) and tc_tiles(n, d, h, wd) >= _TC_MIN_TILES
+        engine = ("tc" if tc_eligible(cin, cout, x, w, out, out_f32) and tc_faster(cin, cout, n * d * h * wd, taps)
                   else "mma")
     fn = _lib().hlbg_nn_conv3d_tc if engine == "tc" else _lib().hlbg_nn_conv3d
     _ok(fn(_p(x), cin, _p(w), _p(bias), _p(out), _p(out_f32), cout, n, d, h, wd, taps, int(relu), _stream()),
@@ -82,7 +82,7 @@ def conv3d(x, w, bias, out, out_f32=None, taps=27, relu=False, engine="auto"):
 
 
 def conv3d_tc(x, w, bias, out, out_f32=None, taps=27, relu=False):
-    """conv3d on the tcgen05 tensor cores (cin and cout multiples of 16, cout <= 256)."""
+    """conv3d on the tcgen05 tensor cores (cin and cout multiples of 16)."""
     conv3d(x, w, bias, out, out_f32, taps, relu, engine="tc")
 
 
