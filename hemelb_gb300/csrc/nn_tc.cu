@@ -658,6 +658,8 @@ bool planned(int cin, int cout, int n, int d, int h, int wd, int taps, Plan& pl)
   return true;
 }
 
+#include "nn_wgrad_tc.cuh"
+
 }  // namespace
 
 extern "C" {
@@ -745,6 +747,11 @@ int hlbg_nn_conv3d_tc(const void* in, int32_t cin, const void* w, const float* b
   const unsigned gx = (unsigned)std::min<int64_t>(tiles, std::max(1, kSms * pl.per_sm / ny));
   kernel<<<dim3(gx, (unsigned)ny), conv_threads(pl.cols), pl.smem, static_cast<cudaStream_t>(stream)>>>(tin, tw, p);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
+}
+
+int hlbg_nn_conv3d_wgrad_tc(const void* x, int32_t cin, const void* dy, int32_t cout, float* dw, int32_t n, int32_t d,
+                            int32_t h, int32_t wd, int32_t taps, void* stream) {
+  return wgrad_tc(x, cin, dy, cout, dw, n, d, h, wd, taps, static_cast<cudaStream_t>(stream));
 }
 
 int hlbg_nn_tc_error(int32_t reset) {

@@ -36,6 +36,11 @@ int hlbg_nn_tc_error(int32_t reset);
 /* dw[tap][co][ci] += sum over voxels of dy[m, co] * x[m + off(tap), ci] (FP32) */
 int hlbg_nn_conv3d_wgrad(const void *x, int32_t cin, const void *dy, int32_t cout, float *dw,
                          int32_t n, int32_t d, int32_t h, int32_t wd, int32_t taps, void *stream);
+/* The same on the fifth-generation tensor cores: cin and cout multiples of 16, x, dy and
+ * dw 16-byte aligned.  Returns 1 for what it does not take (hlbg_nn_conv3d_wgrad, which
+ * uses it where it is the faster one, takes every shape). */
+int hlbg_nn_conv3d_wgrad_tc(const void *x, int32_t cin, const void *dy, int32_t cout, float *dw,
+                            int32_t n, int32_t d, int32_t h, int32_t wd, int32_t taps, void *stream);
 /* wt[taps-1-tap][ci][co] = w[tap][co][ci]: weights of the data-gradient convolution */
 int hlbg_nn_flip_transpose(const void *w, void *wt, int32_t cout, int32_t cin, int32_t taps,
                            void *stream);
