@@ -203,6 +203,12 @@ struct StepArgs {
   const int32_t* io_meta;
   int64_t n_io_links;
   uint32_t io_ctas;
+  // When the next launch may start beside this one: 1 once all CTAs of this one have
+  // started, 0 once they have done their sites (monitored steps: once they have ended).  A launch of several waves takes 1 (the
+  // successor's lists are read while the last wave ends).  One of few waves takes 0: its
+  // successor's CTAs would be dealt out to the SMs while its own still hold places, as
+  // unevenly as these (1,000 one-warp CTAs of a 34k-site FP64 step: 42 us instead of 28).
+  int32_t let_in;
   const IoletDev* iolets;     // [n_in + n_out]
   const double* iolet_rho;    // [n_in + n_out] ghost density for this step (Nash)
   const double* iolet_umax;   // [n_in + n_out] peak speed for this step (Ladd)
@@ -216,6 +222,16 @@ struct StepArgs {
   float fp16_scale, fp16_inv_scale;
 };
 
+// ---- overlapped launches -----------------------------------------------------
+// The update's launches may start while the kernel before them on the stream still
+// runs its last CTAs (programmatic stream serialization): a kernel lets its successor
+// in (StepArgs::let_in says when), reads what no kernel changes (lists,
+// neighbour tables, records), and waits for its predecessor's completion before it
+// touches anything else.  What it reads after the wait is read by ordinary loads: the
+// read-only path (__ldg) may be moved above it.
+__device__ __forceinline__ void let_next_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- storage forms ---------------------------------------------------------
 // FP64: f itself.  FP32DEV / FP16: g = f - w_d (FP16 scaled by fp16_scale).
 template <int P>
@@ -224,7 +240,7 @@ template <>
 struct Store<0> {
   using S = double;
   static __device__ __forceinline__ double load(const S* p, int64_t i, const StepArgs&) {
-    return __ldg(p + i);
+    return p[i];
   }
   static __device__ __forceinline__ void store(S* p, int64_t i, double v, const StepArgs&) {
     p[i] = v;
@@ -233,8 +249,7 @@ struct Store<0> {
 // Distributions of the old array are read exactly once per step.  The streaming
 // hint (ld.global.cs, HLBG_STREAM_LOADS=1) was meant to keep them from displacing
 // the partially written sectors of the new array in L2, but on the 187M-site
-// forest it measured 6% slower than the read-only path (25.3 vs 26.9 GLUPS), so
-// plain __ldg is the default.
+// forest it measured 6% slower than plain loads (25.3 vs 26.9 GLUPS).
 #ifndef HLBG_STREAM_LOADS
 #define HLBG_STREAM_LOADS 0
 #endif
@@ -249,7 +264,7 @@ struct Store<1> {
 #if HLBG_STREAM_LOADS
     return __ldcs(p + i);
 #else
-    return __ldg(p + i);
+    return p[i];
 #endif
   }
   static __device__ __forceinline__ void store(S* p, int64_t i, float v, const StepArgs&) {
@@ -267,7 +282,7 @@ struct Store<2> {
 #if HLBG_STREAM_LOADS
     return __half2float(__ldcs(p + i)) * a.fp16_inv_scale;
 #else
-    return __half2float(__ldg(p + i)) * a.fp16_inv_scale;
+    return __half2float(p[i]) * a.fp16_inv_scale;
 #endif
   }
   static __device__ __forceinline__ void store(S* p, int64_t i, float v, const StepArgs& a) {

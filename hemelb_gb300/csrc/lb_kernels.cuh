@@ -582,6 +582,7 @@ __device__ __forceinline__ void mon_finish(const StepArgs& a, const MonAccT<P>& 
   const unsigned groups = (unsigned)((n + kMonGroup - 1) / kMonGroup), g = cta / kMonGroup;
   const int lane = threadIdx.x & 31;
   int last = 0;
+  wait_for_previous();  // its last CTAs may still read the partials
   if constexpr (P == 0) {
     const MonAcc r = mon_block(acc);
     if (threadIdx.x == 0) mon_store(a.mon_part, n, cta, r);
@@ -706,6 +707,7 @@ __device__ __forceinline__ void iolet_link(const StepArgs& a, int64_t i, const i
   const int ls = site_of_slot(a, s, (__ldg(a.block_nbr + b * 27 + 13) & kPackedBit) != 0);
   const int gx = block_xyz[3 * b] * 8 + (ls >> 6), gy = block_xyz[3 * b + 1] * 8 + ((ls >> 3) & 7),
             gz = block_xyz[3 * b + 2] * 8 + (ls & 7);
+  wait_for_previous();
   T f[Q], fpost[Q];
 #pragma unroll
   for (int k = 0; k < Q; ++k) f[k] = St::load(fo, k * kSites, a);
@@ -739,8 +741,7 @@ __global__ void __launch_bounds__(128) k_iolet_links(StepArgs a, const int32_t* 
 // every lane of a warp with any fluid site stays converged through the pushes.
 template <int P, bool MON>
 __device__ __forceinline__ void collide_slot(const StepArgs& a, int64_t s,
-                                             const int32_t* __restrict__ block_xyz, MonAccT<P>& acc,
-                                             bool check) {
+                                             const int32_t* __restrict__ block_xyz, MonAccT<P>& acc) {
   using St = Store<P>;
   using S = typename St::S;
   using T = typename Calc<P>::T;
@@ -758,7 +759,9 @@ __device__ __forceinline__ void collide_slot(const StepArgs& a, int64_t s,
   const int l = site_of_slot(a, s, packed);
   const S* fo = static_cast<const S*>(a.f_old) + b * (Q * kSites) + j;
   S* fn = static_cast<S*>(a.f_new);
+  wait_for_previous();
   MonOld<P> uo;
+  const bool check = MON && *a.mon_state != 0;
   if constexpr (MON) uo.load(a, s, check && code != 0);
   T f[Q], fpost[Q];
   if (code != 0) {
@@ -824,8 +827,7 @@ __device__ __forceinline__ void collide_and_push(const StepArgs& a, int64_t b, i
 // The unit's list entries (block e, this lane's slot js) are loaded by the caller.
 template <int P, bool MON>
 __device__ __forceinline__ void collide_listed_unit(const StepArgs& a, int32_t e, unsigned js,
-                                                    const int32_t* __restrict__ block_xyz, MonAccT<P>& acc,
-                                                    bool check) {
+                                                    const int32_t* __restrict__ block_xyz, MonAccT<P>& acc) {
   using St = Store<P>;
   using S = typename St::S;
   using T = typename Calc<P>::T;
@@ -836,6 +838,7 @@ __device__ __forceinline__ void collide_listed_unit(const StepArgs& a, int32_t e
   const int64_t s = b * kSites + j;
   S* fn = static_cast<S*>(a.f_new);
   if (e < 0) {  // zero-fill warp: complete the sectors its slots share with fluid
+    wait_for_previous();
     if (on) {
 #pragma unroll
       for (int d = 0; d < Q; ++d) St::store(fn, fidx(s, d), (T)0, a);
@@ -850,7 +853,9 @@ __device__ __forceinline__ void collide_listed_unit(const StepArgs& a, int32_t e
   const bool packed = (__shfl_sync(0xffffffffu, tabreg, 13) & kPackedBit) != 0;
   const int l = on ? site_of_slot(a, s, packed) : 0;
   const S* fo = static_cast<const S*>(a.f_old) + b * (Q * kSites) + j;
+  wait_for_previous();
   MonOld<P> uo;
+  const bool check = MON && *a.mon_state != 0;
   if constexpr (MON) uo.load(a, s, check && on);
   T f[Q];
   if (on) {
@@ -865,24 +870,23 @@ __device__ __forceinline__ void collide_listed_unit(const StepArgs& a, int32_t e
 
 template <int P, bool MON>
 __device__ __forceinline__ void collide_listed_warp(const StepArgs& a, int64_t w,
-                                                    const int32_t* __restrict__ block_xyz, MonAccT<P>& acc,
-                                                    bool check) {
+                                                    const int32_t* __restrict__ block_xyz, MonAccT<P>& acc) {
   if (w >= a.n_warps) return;  // whole warp
   collide_listed_unit<P, MON>(a, __ldg(a.warp_block + w), __ldg(a.lane_slot + w * 32 + (threadIdx.x & 31)),
-                              block_xyz, acc, check);
+                              block_xyz, acc);
 }
 
 template <int P, int THREADS, int MINB, bool MON>
 __global__ void __launch_bounds__(THREADS, MINB) k_stream_collide_listed(StepArgs a, const int32_t* block_xyz) {
+  if (a.let_in) let_next_in();
   if (blockIdx.x < a.io_ctas) {  // whole CTA
     iolet_link<P>(a, (int64_t)blockIdx.x * THREADS + threadIdx.x, block_xyz);
     return;
   }
   const unsigned cta = blockIdx.x - a.io_ctas;
   MonAccT<P> acc = mon_neutral_t<P>();
-  bool check = false;
-  if constexpr (MON) check = *a.mon_state != 0;
-  collide_listed_warp<P, MON>(a, ((int64_t)cta * THREADS + threadIdx.x) >> 5, block_xyz, acc, check);
+  collide_listed_warp<P, MON>(a, ((int64_t)cta * THREADS + threadIdx.x) >> 5, block_xyz, acc);
+  if (!MON && !a.let_in) let_next_in();
   if constexpr (MON) {
     if (a.mon_fold) mon_finish<P>(a, acc, cta);
   }
@@ -1025,6 +1029,23 @@ __global__ void __launch_bounds__(THREADS, MINB) k_stream_collide_block(StepArgs
       for (int d = 0; d < Q; ++d) Store<P>::store(fn, fidx(b * kSites + j, d), (T)0, a);
     }
   }
+}
+
+// Launch that may start beside the last CTAs of the kernel before it on the stream (see
+// wait_for_previous, which the kernel calls).  Behind anything but a kernel it is an
+// ordinary launch.
+template <class K, class... A>
+void launch_overlapped(K kernel, unsigned grid, unsigned threads, cudaStream_t st, const A&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 template <int P, int THREADS, int MINB>
@@ -1257,7 +1278,8 @@ void launch_listed(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
   const int64_t g = (a.n_warps * 32 + THREADS - 1) / THREADS;
   StepArgs b = a;
   b.io_ctas = (uint32_t)((a.n_io_links + THREADS - 1) / THREADS);
-  if (g) k_stream_collide_listed<P, THREADS, MINB, MON><<<(unsigned)g + b.io_ctas, THREADS, 0, st>>>(b, bxyz);
+  b.let_in = g >= 4 * 152 * MINB;
+  if (g) launch_overlapped(k_stream_collide_listed<P, THREADS, MINB, MON>, (unsigned)g + b.io_ctas, THREADS, st, b, bxyz);
 }
 
 template <int P>
@@ -1278,15 +1300,15 @@ void launch_iolets(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
 template <int P, int THREADS, int MINB, bool MON>
 __global__ void __launch_bounds__(THREADS, MINB)
     k_stream_collide(StepArgs a, const int32_t* block_xyz) {
+  if (a.let_in) let_next_in();
   if (blockIdx.x < a.io_ctas) {  // whole CTA
     iolet_link<P>(a, (int64_t)blockIdx.x * THREADS + threadIdx.x, block_xyz);
     return;
   }
   const unsigned cta = blockIdx.x - a.io_ctas;
   MonAccT<P> acc = mon_neutral_t<P>();
-  bool check = false;
-  if constexpr (MON) check = *a.mon_state != 0;
-  collide_slot<P, MON>(a, (int64_t)cta * THREADS + threadIdx.x, block_xyz, acc, check);
+  collide_slot<P, MON>(a, (int64_t)cta * THREADS + threadIdx.x, block_xyz, acc);
+  if (!MON && !a.let_in) let_next_in();
   if constexpr (MON) {
     if (a.mon_fold) mon_finish<P>(a, acc, cta);
   }
@@ -1310,6 +1332,7 @@ template <int P>
 __global__ void k_post_step(PostArgs p) {
   using St = Store<P>;
   using S = typename St::S;
+  if (p.count >= 1 << 16) let_next_in();  // the update that follows has several waves of CTAs
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.count) return;
   StepArgs a{};
@@ -1319,13 +1342,15 @@ __global__ void k_post_step(PostArgs p) {
   const int64_t s = p.slot[i];
   const int d = p.dir[i];
   const int inv = c_inv[d];
+  const float qf = p.q[i];
+  wait_for_previous();
   if constexpr (P == 0) {
-    const double q = (double)p.q[i];
+    const double q = (double)qf;
     const double vi = St::load(fn, fidx(s, inv), a);
     const double vd = St::load(fn, fidx(s, d), a);
     St::store(fn, fidx(s, inv), 2.0 * q * vi + (1.0 - 2.0 * q) * vd, a);
   } else {
-    const float q = p.q[i];
+    const float q = qf;
     const float vi = St::load(fn, fidx(s, inv), a);
     const float vd = St::load(fn, fidx(s, d), a);
     St::store(fn, fidx(s, inv), 2.f * q * vi + (1.f - 2.f * q) * vd, a);
@@ -1729,7 +1754,8 @@ void launch_sc(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
   const unsigned g = (unsigned)(a.nslot / THREADS);
   StepArgs b = a;
   b.io_ctas = (uint32_t)((a.n_io_links + THREADS - 1) / THREADS);
-  if (g) k_stream_collide<P, THREADS, MINB, MON><<<g + b.io_ctas, THREADS, 0, st>>>(b, bxyz);
+  b.let_in = g >= 4 * 152 * MINB;
+  if (g) launch_overlapped(k_stream_collide<P, THREADS, MINB, MON>, g + b.io_ctas, THREADS, st, b, bxyz);
 }
 }  // namespace hlbg
 
@@ -1838,7 +1864,7 @@ int64_t monitored_ctas(int64_t nslot, int variant, int64_t n_warps) {
   }                                                                                             \
   void launch_post_step_##P(const PostArgs& p, cudaStream_t st) {                               \
     unsigned g = (unsigned)((p.count + 255) / 256);                                             \
-    if (g) k_post_step<P><<<g, 256, 0, st>>>(p);                                                \
+    if (g) launch_overlapped(k_post_step<P>, g, 256, st, p);                                    \
   }                                                                                             \
   void launch_init_uniform_##P(const InitArgs& ia, cudaStream_t st) {                           \
     unsigned g = (unsigned)((ia.nslot + 255) / 256);                                            \
