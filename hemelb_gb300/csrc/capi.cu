@@ -19,6 +19,7 @@
 #include <new>
 #include <string>
 #include <thread>
+#include <tuple>
 #include <vector>
 
 #include "../../include/hemelb_gb300.h"
@@ -46,12 +47,6 @@ const int HINV[19] = {0, 2, 1, 4, 3, 6, 5, 8, 7, 10, 9, 12, 11, 14, 13, 16, 15, 
 // for FP16 and 0 otherwise.
 #ifndef HLBG_LIST_SPLIT
 #define HLBG_LIST_SPLIT -1
-#endif
-
-// Device block order (HLBG_BLOCK_SORT): 0 z-columns in 2-D Morton order of (x, y);
-// 1 3-D Morton order; 2 z-columns along a 2-D Hilbert curve of (x, y).
-#ifndef HLBG_BLOCK_SORT
-#define HLBG_BLOCK_SORT 0
 #endif
 
 // Index of (x, y) along a 2-D Hilbert curve over an n x n grid (n a power of two):
@@ -411,23 +406,32 @@ int build_layout(hlbg_ctx* ctx, const hlbg_geometry* g) {
   if (nb * 512 >= (1ll << 31)) return fail(ctx, HLBG_ERR_INVAL, "more than 2^31 slots");
   // Device block order: z-columns (2-D Morton order of (x, y), then z).  The two
   // writers of every z-shifted row of a push are z-adjacent blocks; running them
-  // back to back lets their partial 32-byte sectors merge in L2.  The reference's
-  // own numbering (3-D Morton order) is kept separately in ref_rank below.
+  // back to back lets their partial 32-byte sectors merge in L2, and the kernels take
+  // a z-neighbour to be the next block (HLBG_Z_COLUMNS).  The reference's own numbering
+  // (3-D Morton order) is kept separately in ref_order below.
   uint32_t hn = 1;  // Hilbert grid side: a power of two covering the block grid
   while (hn < (uint32_t)std::max(NX, NY)) hn *= 2;
   (void)hn;
-  std::vector<std::pair<uint64_t, int64_t>> order((size_t)nb);
+  struct Place {  // curve key (16 bits of x and y), then the exact x, y (one column), then z
+    uint64_t key;
+    int32_t x, y, z;
+    int64_t second;
+    bool operator<(const Place& o) const {
+      return std::tie(key, x, y, z, second) < std::tie(o.key, o.x, o.y, o.z, o.second);
+    }
+  };
+  std::vector<Place> order((size_t)nb);
   std::vector<std::pair<uint64_t, int64_t>> ref_order((size_t)nb);
   for (int64_t b = 0; b < nb; ++b) {
     int32_t x = g->block_coords[3 * b], y = g->block_coords[3 * b + 1], z = g->block_coords[3 * b + 2];
     if (x < 0 || y < 0 || z < 0 || x >= NX || y >= NY || z >= NZ)
       return fail(ctx, HLBG_ERR_INVAL, "block coordinate outside the block grid");
 #if HLBG_BLOCK_SORT == 1
-    order[b] = {morton3(x, y, z), b};
+    order[b] = {morton3(x, y, z), x, y, z, b};
 #elif HLBG_BLOCK_SORT == 2
-    order[b] = {(hilbert2(hn, x, y) << 16) | (uint64_t)z, b};
+    order[b] = {hilbert2(hn, x, y), x, y, z, b};
 #else
-    order[b] = {(morton3(x, y, 0) << 16) | (uint64_t)z, b};
+    order[b] = {morton3(x, y, 0), x, y, z, b};
 #endif
     ref_order[b] = {morton3(x, y, z), b};
   }

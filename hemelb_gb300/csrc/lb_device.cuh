@@ -112,6 +112,15 @@ constexpr unsigned kListBoundary = 1u << 14;
 #if HLBG_PACK && HLBG_BLOCK_ORDER
 #error "the packed layout is built on z-row blocks (HLBG_BLOCK_ORDER=0)"
 #endif
+// Device block order (HLBG_BLOCK_SORT): 0 z-columns in 2-D Morton order of (x, y);
+// 1 3-D Morton order; 2 z-columns along a 2-D Hilbert curve of (x, y).
+#ifndef HLBG_BLOCK_SORT
+#define HLBG_BLOCK_SORT 0
+#endif
+// In z-column order the non-empty blocks next to each other in z are consecutive, so a
+// push that crosses a z face moves by one whole block (PushTargets); the other build
+// options look every neighbour up.
+#define HLBG_Z_COLUMNS (!HLBG_PACK && !HLBG_BLOCK_ORDER && HLBG_BLOCK_SORT != 1)
 // bits 0, 1, 2 of v to bits 0, 3, 6 and back
 __host__ __device__ __forceinline__ int dilate3(int v) { return (v & 1) | ((v & 2) << 2) | ((v & 4) << 4); }
 __host__ __device__ __forceinline__ int undilate3(int m) { return (m & 1) | ((m >> 2) & 2) | ((m >> 4) & 4); }

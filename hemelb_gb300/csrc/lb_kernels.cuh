@@ -240,10 +240,7 @@ struct PushMixed {
   template <class S, class T, class B>
   static __device__ __forceinline__ void run(S* fn, const StepArgs& a, const B& base, int x, int y,
                                              int z, int j, int64_t own, bool active, bool row_fluid,
-                                             uint64_t links,
-                                             int64_t r, int type, int ioid, const T* fpost, T m0,
-                                             T mx, T my, T mz, int64_t b,
-                                             const int32_t* __restrict__ block_xyz) {
+                                             uint64_t links, int64_t r, const T* fpost) {
     constexpr int cx = Lat::cx(D), cy = Lat::cy(D), cz = Lat::cz(D);
     constexpr int inv = Lat::inv(D);
     const int xx = x + cx, yy = y + cy, zz = z + cz;
@@ -277,17 +274,179 @@ struct PushMixed {
     }
     if (st) Store<P>::store(fn, off, v, a);
     push_fence();
-    PushMixed<P, D + 1>::run(fn, a, base, x, y, z, j, own, active, row_fluid, links, r, type, ioid,
-                             fpost, m0, mx, my, mz, b, block_xyz);
+    PushMixed<P, D + 1>::run(fn, a, base, x, y, z, j, own, active, row_fluid, links, r, fpost);
   }
 };
 template <int P>
 struct PushMixed<P, Q> {
   template <class S, class T, class B>
   static __device__ __forceinline__ void run(S*, const StepArgs&, const B&, int, int, int, int,
-                                             int64_t, bool, bool, uint64_t, int64_t, int, int,
-                                             const T*, T, T, T, T, int64_t, const int32_t*) {}
+                                             int64_t, bool, bool, uint64_t, int64_t, const T*) {}
 };
+
+#if HLBG_Z_COLUMNS
+// Where a lane's site pushes to.  A site crosses at most one face per axis, so four
+// blocks are all it needs: its own, the one across its x face, across its y face, and
+// across both (three shuffles of the neighbour table); z-neighbours follow or precede
+// each of these.  Every push is then one of nine (x, y) pointers, moved along z by an
+// element offset and to its direction's plane by an immediate.  Looking the block of
+// each of the 19 pushes up by shuffle and wrapping its coordinates took about 200
+// instructions a warp; this takes 30 when no site of the warp lies on an x face (most
+// warps: 32 slots have one x), 80 otherwise.  Lookups -> pointers, us a step: FP32 tree of
+// 16.9M sites 584 -> 573, FP16 tree of 7.8M sites 252 -> 248, FP32 bifurcation of 1.5M
+// sites 54 -> 51, FP64 pipe 19.4 -> 19.0.  The rest of the update's distance from memory
+// speed is its stores: a z shift sends every 32-byte row to two blocks (30.7M sectors
+// written in the FP16 tree for 9.2M full ones, the L1's port to L2 busy 64 % of the time).
+// MIXED: the warp has boundary sites, whose neighbour across a face may be missing where
+// the one also across the z face is not; that one's column is then taken from it.
+template <int P, bool MIXED>
+struct PushTargets {
+  using S = typename Store<P>::S;
+  static constexpr int kBlock = Q * kSites;
+  S *own, *yp, *ym;  // direction 0 of the site's slot, and one step in y
+  S *xp, *xm, *pp, *pm, *mp, *mm;  // x faces only: one step in x, in x and y
+  int zp, zm;        // elements of a step in z
+  bool xface;        // some lane of the warp lies on an x face
+
+  __device__ __forceinline__ int32_t block(int32_t tabreg, int sx, int sy, int sz) const {
+    int32_t e = __shfl_sync(0xffffffffu, tabreg, 13 + 9 * sx + 3 * sy);
+    if (MIXED) {
+      const int32_t far = __shfl_sync(0xffffffffu, tabreg, 13 + 9 * sx + 3 * sy + sz);
+      if (e < 0) e = far - sz;
+    }
+    return e;
+  }
+  // every lane of the warp takes part; j: the site's slot in block b
+  __device__ __forceinline__ PushTargets(S* fn, int64_t b, int32_t tabreg, int x, int y, int z, int j) {
+    const int sx = x == 7 ? 1 : (x == 0 ? -1 : 0), sy = y == 7 ? 1 : (y == 0 ? -1 : 0),
+              sz = z == 7 ? 1 : (z == 0 ? -1 : 0);
+    own = fn + b * kBlock + j;
+    zp = z == 7 ? kBlock - 7 : 1;
+    zm = z == 0 ? 7 - kBlock : -1;
+    S* const yb = fn + (int64_t)block(tabreg, 0, sy, sz) * kBlock + j;
+    yp = (y == 7 ? yb : own) + (y == 7 ? -56 : 8);
+    ym = (y == 0 ? yb : own) + (y == 0 ? 56 : -8);
+    xface = __any_sync(0xffffffffu, sx != 0);
+    if (xface) {
+      S* const xb = fn + (int64_t)block(tabreg, sx, 0, sz) * kBlock + j;
+      S* const xyb = fn + (int64_t)block(tabreg, sx, sy, sz) * kBlock + j;
+      xp = (x == 7 ? xb : own) + (x == 7 ? -448 : 64);
+      xm = (x == 0 ? xb : own) + (x == 0 ? 448 : -64);
+      pp = (x == 7 ? (y == 7 ? xyb : xb) : (y == 7 ? yb : own)) + ((x == 7 ? -448 : 64) + (y == 7 ? -56 : 8));
+      pm = (x == 7 ? (y == 0 ? xyb : xb) : (y == 0 ? yb : own)) + ((x == 7 ? -448 : 64) + (y == 0 ? 56 : -8));
+      mp = (x == 0 ? (y == 7 ? xyb : xb) : (y == 7 ? yb : own)) + ((x == 0 ? 448 : -64) + (y == 7 ? -56 : 8));
+      mm = (x == 0 ? (y == 0 ? xyb : xb) : (y == 0 ? yb : own)) + ((x == 0 ? 448 : -64) + (y == 0 ? 56 : -8));
+    }
+  }
+  // Direction 0 of the slot direction D streams to (add D kSites).
+  template <int D, bool XFACE>
+  __device__ __forceinline__ S* at() const {
+    constexpr int cx = Lat::cx(D), cy = Lat::cy(D), cz = Lat::cz(D);
+    S* p;
+    if (!XFACE || cx == 0) {
+      p = (cy == 0 ? own : (cy > 0 ? yp : ym)) + 64 * cx;
+    } else if (cx > 0) {
+      p = cy == 0 ? xp : (cy > 0 ? pp : pm);
+    } else {
+      p = cy == 0 ? xm : (cy > 0 ? mp : mm);
+    }
+    return cz == 0 ? p : p + (cz > 0 ? zp : zm);
+  }
+};
+
+// Pushes of a bulk site along directions D, D + 1, ...
+template <int P, int D, bool XFACE>
+struct PushEach {
+  template <class T>
+  static __device__ __forceinline__ void run(const PushTargets<P, false>& t, const StepArgs& a, const T* fpost) {
+    Store<P>::store(t.template at<D, XFACE>(), D * kSites, fpost[D], a);
+    PushEach<P, D + 1, XFACE>::run(t, a, fpost);
+  }
+};
+template <int P, bool XFACE>
+struct PushEach<P, Q, XFACE> {
+  template <class T>
+  static __device__ __forceinline__ void run(const PushTargets<P, false>&, const StepArgs&, const T*) {}
+};
+
+// Pushes of a warp that holds at least one boundary site: a boundary lane redirects the
+// link by its precomputed code as in PushMixed.
+template <int P, int D, bool XFACE>
+struct PushEachMixed {
+  template <class T>
+  static __device__ __forceinline__ void run(const PushTargets<P, true>& t, const StepArgs& a, bool active,
+                                             bool row_fluid, uint64_t links, int64_t r, const T* fpost) {
+    constexpr int inv = Lat::inv(D);
+    const unsigned lc = (unsigned)(links >> (3 * D)) & 7u;
+    typename Store<P>::S* p = t.template at<D, XFACE>() + D * kSites;
+    T v = fpost[D];
+    bool st = true;
+    if (!active) {
+      // A solid slot is never written by a push nor ever read; a zero there completes
+      // the 32-byte sector of slots it shares with fluid slots (sectors without any
+      // receive no write at all and stay untouched).
+      p = t.own + D * kSites;
+      v = (T)0;
+      st = row_fluid;
+    } else if (lc != HLBG_LC_PUSH) {
+      p = t.own + inv * kSites;
+      st = lc != HLBG_LC_SKIP && lc != HLBG_LC_IOLET;  // iolet links: written by iolet_link
+      if (lc == HLBG_LC_BFL) {
+        const T q = (T)a.b_cut[r * (Q - 1) + D - 1];
+        v = (fpost[D] + ((T)2.0 * q - (T)1) * fpost[inv]) / ((T)2.0 * q);
+      }
+    }
+    if (st) Store<P>::store(p, 0, v, a);
+    PushEachMixed<P, D + 1, XFACE>::run(t, a, active, row_fluid, links, r, fpost);
+  }
+};
+template <int P, bool XFACE>
+struct PushEachMixed<P, Q, XFACE> {
+  template <class T>
+  static __device__ __forceinline__ void run(const PushTargets<P, true>&, const StepArgs&, bool, bool, uint64_t,
+                                             int64_t, const T*) {}
+};
+#endif
+
+// The pushes of one warp of one block b: this lane's site in slot j, local coordinates
+// x, y, z, post-collision values fpost, code as site_code (0: no site here; a zero goes
+// to its slot where row_fluid).  tabreg: the block's neighbour table in lanes 0..26.
+// Every lane of the warp takes part.  A monitored FP32 or FP16 update keeps the lookup of
+// each push: beside its accumulators the nine pointers cost more in registers than they
+// save (12 steps of a monitored 7.8M-site FP32 tree: 4764 us with the lookups, 4811 with
+// the pointers).
+template <int P, bool MON, class T>
+__device__ __forceinline__ void push_warp(const StepArgs& a, int64_t b, int32_t tabreg, int x, int y, int z, int j,
+                                          uint32_t code, bool row_fluid, const T* fpost) {
+  using S = typename Store<P>::S;
+  S* fn = static_cast<S*>(a.f_new);
+  const bool bnd = code >= 2;
+  const bool mixed = __ballot_sync(0xffffffffu, bnd) != 0;
+  const int64_t r = bnd ? (int64_t)code - 2 : 0;
+#if HLBG_Z_COLUMNS
+  if constexpr (!MON || P == 0) {
+    if (!mixed) {
+      const PushTargets<P, false> t(fn, b, tabreg, x, y, z, j);
+      if (code == 1) {
+        if (t.xface) PushEach<P, 0, true>::run(t, a, fpost);
+        else PushEach<P, 0, false>::run(t, a, fpost);
+      }
+    } else {
+      const uint64_t links = bnd ? a.b_links[r] : 0ull;
+      const PushTargets<P, true> t(fn, b, tabreg, x, y, z, j);
+      if (t.xface) PushEachMixed<P, 0, true>::run(t, a, code != 0, row_fluid, links, r, fpost);
+      else PushEachMixed<P, 0, false>::run(t, a, code != 0, row_fluid, links, r, fpost);
+    }
+    return;
+  }
+#endif
+  if (!mixed) {
+    PushBulk<P, 0>::run(fn, a, ShflBase{tabreg}, x, y, z, code == 1, fpost);
+  } else {
+    const uint64_t links = bnd ? a.b_links[r] : 0ull;
+    PushMixed<P, 0>::run(fn, a, ShflBase{tabreg}, x, y, z, j, b * (Q * kSites), code != 0, row_fluid, links, r, fpost);
+  }
+}
 
 // StabilityTester::PostSendToParent (Code/lb/StabilityTester.h:91-149) and
 // ComputeRelativeDifference (:160-183) plus total mass: one slot per thread, one
@@ -740,8 +899,7 @@ __global__ void __launch_bounds__(128) k_iolet_links(StepArgs a, const int32_t* 
 // hold the block's neighbour table and serve it to the bulk pushes by shuffle, so
 // every lane of a warp with any fluid site stays converged through the pushes.
 template <int P, bool MON>
-__device__ __forceinline__ void collide_slot(const StepArgs& a, int64_t s,
-                                             const int32_t* __restrict__ block_xyz, MonAccT<P>& acc) {
+__device__ __forceinline__ void collide_slot(const StepArgs& a, int64_t s, MonAccT<P>& acc) {
   using St = Store<P>;
   using S = typename St::S;
   using T = typename Calc<P>::T;
@@ -758,7 +916,6 @@ __device__ __forceinline__ void collide_slot(const StepArgs& a, int64_t s,
   const bool packed = (__shfl_sync(0xffffffffu, tabreg, 13) & kPackedBit) != 0;
   const int l = site_of_slot(a, s, packed);
   const S* fo = static_cast<const S*>(a.f_old) + b * (Q * kSites) + j;
-  S* fn = static_cast<S*>(a.f_new);
   wait_for_previous();
   MonOld<P> uo;
   const bool check = MON && *a.mon_state != 0;
@@ -776,18 +933,7 @@ __device__ __forceinline__ void collide_slot(const StepArgs& a, int64_t s,
   if constexpr (MON) {
     if (code != 0) mon_site<P>(a, s, f, m0, mx, my, mz, acc, check, uo);
   }
-  const int x = l >> 6, y = (l >> 3) & 7, z = l & 7;
-  const bool bnd = code >= 2;
-  if (__ballot_sync(0xffffffffu, bnd) == 0) {
-    PushBulk<P, 0>::run(fn, a, ShflBase{tabreg}, x, y, z, code == 1, fpost);
-  } else {
-    const int64_t r = bnd ? (int64_t)code - 2 : 0;
-    const uint64_t links = bnd ? a.b_links[r] : 0ull;
-    const int type = bnd ? (int)a.b_type[r] : 0;
-    const int ioid = bnd ? a.b_ioid[r] : 0;
-    PushMixed<P, 0>::run(fn, a, ShflBase{tabreg}, x, y, z, j, b * (Q * kSites), code != 0, row_fluid,
-                         links, r, type, ioid, fpost, m0, mx, my, mz, b, block_xyz);
-  }
+  push_warp<P, MON>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, row_fluid, fpost);
 }
 
 // One warp of the fluid list: 32 fluid sites of one block (or the zero-fill of its
@@ -799,35 +945,21 @@ __device__ __forceinline__ void collide_slot(const StepArgs& a, int64_t s,
 template <int P, bool MON>
 __device__ __forceinline__ void collide_and_push(const StepArgs& a, int64_t b, int j, int64_t s, int l,
                                                  uint32_t code, int32_t tabreg, typename Calc<P>::T* f,
-                                                 const int32_t* __restrict__ block_xyz, MonAccT<P>& acc,
-                                                 bool check, const MonOld<P>& uo) {
-  using S = typename Store<P>::S;
+                                                 MonAccT<P>& acc, bool check, const MonOld<P>& uo) {
   using T = typename Calc<P>::T;
-  S* fn = static_cast<S*>(a.f_new);
   T fpost[Q];
   T m0, mx, my, mz;
   collide_any<P>(a, b, f, m0, mx, my, mz, fpost);
   if constexpr (MON) {
     if (code != 0) mon_site<P>(a, s, f, m0, mx, my, mz, acc, check, uo);
   }
-  const int x = l >> 6, y = (l >> 3) & 7, z = l & 7;
-  const bool bnd = code >= 2;
-  if (__ballot_sync(0xffffffffu, bnd) == 0) {
-    PushBulk<P, 0>::run(fn, a, ShflBase{tabreg}, x, y, z, code == 1, fpost);
-  } else {
-    const int64_t r = bnd ? (int64_t)code - 2 : 0;
-    const uint64_t links = bnd ? a.b_links[r] : 0ull;
-    const int type = bnd ? (int)a.b_type[r] : 0;
-    const int ioid = bnd ? a.b_ioid[r] : 0;
-    PushMixed<P, 0>::run(fn, a, ShflBase{tabreg}, x, y, z, j, b * (Q * kSites), code != 0, false, links,
-                         r, type, ioid, fpost, m0, mx, my, mz, b, block_xyz);
-  }
+  push_warp<P, MON>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, false, fpost);
 }
 
 // The unit's list entries (block e, this lane's slot js) are loaded by the caller.
 template <int P, bool MON>
 __device__ __forceinline__ void collide_listed_unit(const StepArgs& a, int32_t e, unsigned js,
-                                                    const int32_t* __restrict__ block_xyz, MonAccT<P>& acc) {
+                                                    MonAccT<P>& acc) {
   using St = Store<P>;
   using S = typename St::S;
   using T = typename Calc<P>::T;
@@ -865,15 +997,14 @@ __device__ __forceinline__ void collide_listed_unit(const StepArgs& a, int32_t e
 #pragma unroll
     for (int i = 0; i < Q; ++i) f[i] = (T)(P == 0 ? weight_d(i) : 0.0);
   }
-  collide_and_push<P, MON>(a, b, j, s, l, code, tabreg, f, block_xyz, acc, check, uo);
+  collide_and_push<P, MON>(a, b, j, s, l, code, tabreg, f, acc, check, uo);
 }
 
 template <int P, bool MON>
-__device__ __forceinline__ void collide_listed_warp(const StepArgs& a, int64_t w,
-                                                    const int32_t* __restrict__ block_xyz, MonAccT<P>& acc) {
+__device__ __forceinline__ void collide_listed_warp(const StepArgs& a, int64_t w, MonAccT<P>& acc) {
   if (w >= a.n_warps) return;  // whole warp
   collide_listed_unit<P, MON>(a, __ldg(a.warp_block + w), __ldg(a.lane_slot + w * 32 + (threadIdx.x & 31)),
-                              block_xyz, acc);
+                              acc);
 }
 
 template <int P, int THREADS, int MINB, bool MON>
@@ -885,7 +1016,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_stream_collide_listed(StepArg
   }
   const unsigned cta = blockIdx.x - a.io_ctas;
   MonAccT<P> acc = mon_neutral_t<P>();
-  collide_listed_warp<P, MON>(a, ((int64_t)cta * THREADS + threadIdx.x) >> 5, block_xyz, acc);
+  collide_listed_warp<P, MON>(a, ((int64_t)cta * THREADS + threadIdx.x) >> 5, acc);
   if (!MON && !a.let_in) let_next_in();
   if constexpr (MON) {
     if (a.mon_fold) mon_finish<P>(a, acc, cta);
@@ -1018,7 +1149,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_stream_collide_block(StepArgs
       else
         f[d] = on ? __half2float(stage[d * kSites + j]) * a.fp16_inv_scale : 0.f;
     }
-    collide_and_push<P, false>(a, b, j, s, j, code, tabreg, f, block_xyz, acc, false, uo);
+    collide_and_push<P, false>(a, b, j, s, j, code, tabreg, f, acc, false, uo);
   }
   // solid slots of the rows that hold fluid: zeros complete their sectors
   S* fn = static_cast<S*>(a.f_new);
@@ -1228,7 +1359,7 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) k_stream_collide_pipe(StepA
         else
           f[d] = on ? __half2float(stage[d * kSites + j]) * a.fp16_inv_scale : 0.f;
       }
-      collide_and_push<P, false>(a, b, j, s, j, code, tabreg, f, block_xyz, acc, false, uo);
+      collide_and_push<P, false>(a, b, j, s, j, code, tabreg, f, acc, false, uo);
     }
     rot = (rot + ntask) % NCW;
     __syncwarp();
@@ -1307,7 +1438,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   }
   const unsigned cta = blockIdx.x - a.io_ctas;
   MonAccT<P> acc = mon_neutral_t<P>();
-  collide_slot<P, MON>(a, (int64_t)cta * THREADS + threadIdx.x, block_xyz, acc);
+  collide_slot<P, MON>(a, (int64_t)cta * THREADS + threadIdx.x, acc);
   if (!MON && !a.let_in) let_next_in();
   if constexpr (MON) {
     if (a.mon_fold) mon_finish<P>(a, acc, cta);
