@@ -1730,9 +1730,10 @@ __global__ void __launch_bounds__(256) k_monitor(MonitorArgs ma) {
   }
 }
 
-// Reduce the per-CTA partials of k_monitor in a fixed order into element 0 of
-// each partial array (one CTA of 1024 threads; thread t folds partials t, t + 1024,
-// ...), the largest |du| and smallest f as values again.
+// Reduce the per-CTA partials of k_monitor in a fixed order (one CTA of 1024 threads;
+// thread t folds partials t, t + 1024, ...) into part_mass[0..3], so that the host
+// fetches all with one copy: mass, the largest |du| and smallest f as values again, the
+// count's bits.
 static __global__ void __launch_bounds__(1024) k_monitor_final(MonitorArgs ma, int64_t nparts) {
   MonAcc acc = mon_neutral();
 #pragma unroll 4
@@ -1748,9 +1749,9 @@ static __global__ void __launch_bounds__(1024) k_monitor_final(MonitorArgs ma, i
   __syncthreads();
   if (threadIdx.x == 0) {
     ma.part_mass[0] = acc.mass;
-    ma.part_max[0] = sqrt(__longlong_as_double((long long)acc.maxdu));
-    ma.part_min[0] = ordered_value(acc.minf);
-    ma.part_bad[0] = acc.bad;
+    ma.part_mass[1] = sqrt(__longlong_as_double((long long)acc.maxdu));
+    ma.part_mass[2] = ordered_value(acc.minf);
+    ma.part_mass[3] = __longlong_as_double((long long)acc.bad);
   }
 }
 
