@@ -24,14 +24,14 @@
 // of B's and one dz group, into one set of accumulators, added to dw at its end (red of
 // 16 bytes).  `steps` is the run the mma.sync kernel sums on its tensor cores before its
 // FP32 additions to dw, so the rounding of the sums does not grow.  CTAs are persistent:
-// one thread loads, one issues MMAs (all of one accumulator and shape are ordered), four
+// one thread loads, one warp issues MMAs (all of one accumulator and shape are ordered), four
 // warps add the finished set to dw while the other set fills.  Waits are bounded as in
 // the convolution.
-// Measured at batch 4 (us, mma.sync -> this; the tensor pipe's share in cycles is half to
-// two thirds of it, the rest the issuing thread, about 50 cycles an MMA): 16 -> 16 at
-// 96^3 272 -> 162, 64 -> 16 887 -> 285, 48 -> 48 at 48^3 299 -> 88, 144 -> 48 865 -> 222,
-// 288 -> 96 at 24^3 376 -> 141, 192 -> 192 at 12^3 101 -> 48; 1x1x1, 16 -> 16 at 96^3
-// 556 -> 69.
+// Measured at batch 4 (us; mma.sync, issued from a branch of one lane, now; the tensor
+// pipe's share in cycles is half to two thirds of it, the rest the issue): 16 -> 16 at
+// 96^3 272, 162, 139; 64 -> 16 887, 285, 246; 48 -> 48 at 48^3 299, 88, 84; 144 -> 48 865,
+// 222, 215; 288 -> 96 at 24^3 376, 141, 122; 192 -> 192 at 12^3 101, 48, 44; 1x1x1,
+// 16 -> 16 at 96^3 556, 69, 54.
 #pragma once
 
 struct WgParams {
@@ -68,12 +68,12 @@ __device__ __forceinline__ uint64_t desc_mn(uint32_t saddr, uint32_t span, uint3
   return d;
 }
 
-__device__ __forceinline__ void umma_first(uint32_t tmem_d, uint32_t a_hi, uint32_t a_lo, uint32_t b_hi, uint32_t b_lo,
-                                           uint32_t idesc) {  // D = A B
+__device__ __forceinline__ void umma_first(uint32_t on, uint32_t tmem_d, uint32_t a_hi, uint32_t a_lo, uint32_t b_hi,
+                                           uint32_t b_lo, uint32_t idesc) {
   asm volatile(
-      "{\n .reg .b64 a, b;\n mov.b64 a, {%2, %1};\n mov.b64 b, {%4, %3};\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, 0;\n}\n" ::"r"(tmem_d),
-      "r"(a_hi), "r"(a_lo), "r"(b_hi), "r"(b_lo), "r"(idesc));
+      "{\n .reg .b64 a, b;\n .reg .pred p;\n setp.ne.b32 p, %6, 0;\n mov.b64 a, {%2, %1};\n mov.b64 b, {%4, %3};\n"
+      " @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, 0;\n}\n" ::"r"(tmem_d),
+      "r"(a_hi), "r"(a_lo), "r"(b_hi), "r"(b_lo), "r"(idesc), "r"(on));
 }
 
 __device__ __forceinline__ void red4(float* p, float a, float b, float c, float d) {
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(kWgThreads, 2) k_wgrad_tc(const __grid_constan
   const uint32_t b_base = smem_u32(base), a_base = b_base + (((uint32_t)p.stages_b * kBBytes + 1023u) & ~1023u);
   const uint32_t afull0 = smem_u32(bars), aempty0 = afull0 + 8 * kWgMaxStages, bfull0 = aempty0 + 8 * kWgMaxStages,
                  bempty0 = bfull0 + 8 * kWgMaxStages, tfull0 = bempty0 + 8 * kWgMaxStages, tempty0 = tfull0 + 16;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // uniform, also to the compiler
   const int units = p.runs * p.na * p.nb * p.nzg;
   const int set = ZG * p.groups * N;  // columns of a set of accumulators
 
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(kWgThreads, 2) k_wgrad_tc(const __grid_constan
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
   if (warp == 0) {
     // ---- loads, one thread: per tile A's plane and the planes of B that are not there ----
@@ -208,8 +208,9 @@ __global__ void __launch_bounds__(kWgThreads, 2) k_wgrad_tc(const __grid_constan
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ---- MMAs, one thread ----
-    if (lane == 0) {
+    // ---- MMAs, one warp in uniform control flow, issued by its lane 0 ----
+    {
+      const uint32_t leader = lane == 0 ? 1u : 0u;
       constexpr uint32_t kPitchA = 10 * kSpanA, kPitchB = 8 * kSpanB;
       const uint64_t a_desc = desc_mn(a_base, kSpanA, WA == 128 ? kABytes / 2 : kSpanA, kPitchA);
       const uint64_t b_desc = desc_mn(b_base, kSpanB, kPitchB, kPitchB);
@@ -222,12 +223,12 @@ __global__ void __launch_bounds__(kWgThreads, 2) k_wgrad_tc(const __grid_constan
       bool ok = true;
       for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
         const WgUnit w(p, u);
-        ok = mbar_wait(tempty0 + 8 * ts, pt);
+        ok = warp_wait(tempty0 + 8 * ts, pt);
         int z = w.first % p.D;
         bool fresh = true;
         const uint32_t acc = tmem + (uint32_t)(ts * set);
         for (int k = 0; k < w.count && ok; ++k) {
-          ok = mbar_wait(afull0 + 8 * sa, pa);
+          ok = warp_wait(afull0 + 8 * sa, pa);
           const bool end = k + 1 == w.count || z + 1 == p.D;  // B's planes go on with the next tile otherwise
 #pragma unroll 1
           for (int e = 0; e < ZG && ok; ++e) {
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(kWgThreads, 2) k_wgrad_tc(const __grid_constan
               s -= p.stages_b;
               ph ^= 1u;
             }
-            if (ZG == 1 || fresh || e == ZG - 1) ok = mbar_wait(bfull0 + 8 * s, ph);
+            if (ZG == 1 || fresh || e == ZG - 1) ok = warp_wait(bfull0 + 8 * s, ph);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // 1x1x1: the unshifted voxels (column 1 of A's halo, row 1 of B's)
@@ -247,23 +248,23 @@ __global__ void __launch_bounds__(kWgThreads, 2) k_wgrad_tc(const __grid_constan
               const uint32_t dst = acc + (uint32_t)((e * p.groups + j) * N);
               const uint32_t aj = a_lo + (uint32_t)(WA == 64 ? 2 * j : j) * (kSpanA >> 4);
               if (k == 0)
-                umma_first(dst, a_hi, aj, b_hi, b_lo, idesc);
+                umma_first(leader, dst, a_hi, aj, b_hi, b_lo, idesc);
               else
-                umma_bf16(dst, a_hi, aj, b_hi, b_lo, idesc);
+                umma_bf16(leader, dst, a_hi, aj, b_hi, b_lo, idesc);
 #pragma unroll
               for (int t = 1; t < 8; ++t)
-                umma_bf16(dst, a_hi, aj + (uint32_t)t * (2 * kPitchA >> 4), b_hi, b_lo + (uint32_t)t * (2 * kPitchB >> 4), idesc);
+                umma_bf16(leader, dst, a_hi, aj + (uint32_t)t * (2 * kPitchA >> 4), b_hi, b_lo + (uint32_t)t * (2 * kPitchB >> 4), idesc);
             }
           }
           if (!ok) break;
-          umma_commit(aempty0 + 8 * sa);
+          umma_commit(leader, aempty0 + 8 * sa);
           if (++sa == p.stages_a) {
             sa = 0;
             pa ^= 1u;
           }
           const int free_b = ZG == 1 ? 1 : (end ? ZG : 1);
           for (int f = 0; f < free_b; ++f) {
-            umma_commit(bempty0 + 8 * sb);
+            umma_commit(leader, bempty0 + 8 * sb);
             if (++sb == p.stages_b) {
               sb = 0;
               pb ^= 1u;
@@ -272,13 +273,13 @@ __global__ void __launch_bounds__(kWgThreads, 2) k_wgrad_tc(const __grid_constan
           fresh = end;
           if (++z == p.D) z = 0;
         }
-        umma_commit(tfull0 + 8 * ts);
+        umma_commit(leader, tfull0 + 8 * ts);
         if (++ts == p.sets) {
           ts = 0;
           pt ^= 1u;
         }
       }
-      if (!ok) atomicExch(&g_tc_err, 1);
+      if (!ok && lane == 0) atomicExch(&g_tc_err, 1);
     }
     __syncwarp();
   } else if (warp >= 4) {

@@ -71,3 +71,18 @@ def test_outputs_off_a_32_byte_boundary(taps, off):
     assert torch.equal(got, want) and torch.equal(got32, want32)
     assert bool((buf[:off] == 7).all()) and bool((buf[off + n:] == 7).all())
     assert bool((buf32[:off // 2] == 7).all()) and bool((buf32[off // 2 + n:] == 7).all())
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (2, 5, 17, 9), (1, 13, 33, 24), (3, 2, 1, 40)])
+@pytest.mark.parametrize("cin,cout", [(16, 16), (48, 80), (144, 48), (16, 272)])
+def test_1x1x1_same_bits_as_mma_sync(shape, cin, cout):
+    """Planes without a halo; one slice (planes in any order) and several."""
+    x, w, b = _operands(shape, cin, cout, 1)
+    got = torch.empty(shape + (cout,), dtype=torch.bfloat16, device="cuda")
+    got32 = torch.empty(shape + (cout,), device="cuda")
+    want, want32 = torch.empty_like(got), torch.empty_like(got32)
+    nn.tc_error(reset=True)
+    nn.conv3d(x, w, b, want, want32, taps=1, relu=True, engine="mma")
+    nn.conv3d(x, w, b, got, got32, taps=1, relu=True, engine="tc")
+    assert torch.equal(got32, want32) and torch.equal(got, want)
+    assert nn.tc_error() == 0
