@@ -32,6 +32,8 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include "overlap.cuh"
+
 namespace hlbg {
 
 constexpr int Q = 19;
@@ -230,16 +232,6 @@ struct StepArgs {
   const double* blk_omega;  // optional [n_blocks * 2]: (omega+, omega-) per block (ensembles)
   float fp16_scale, fp16_inv_scale;
 };
-
-// ---- overlapped launches -----------------------------------------------------
-// The update's launches may start while the kernel before them on the stream still
-// runs its last CTAs (programmatic stream serialization): a kernel lets its successor
-// in (StepArgs::let_in says when), reads what no kernel changes (lists,
-// neighbour tables, records), and waits for its predecessor's completion before it
-// touches anything else.  What it reads after the wait is read by ordinary loads: the
-// read-only path (__ldg) may be moved above it.
-__device__ __forceinline__ void let_next_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- storage forms ---------------------------------------------------------
 // FP64: f itself.  FP32DEV / FP16: g = f - w_d (FP16 scaled by fp16_scale).

@@ -1162,23 +1162,6 @@ __global__ void __launch_bounds__(THREADS, MINB) k_stream_collide_block(StepArgs
   }
 }
 
-// Launch that may start beside the last CTAs of the kernel before it on the stream (see
-// wait_for_previous, which the kernel calls).  Behind anything but a kernel it is an
-// ordinary launch.
-template <class K, class... A>
-void launch_overlapped(K kernel, unsigned grid, unsigned threads, cudaStream_t st, const A&... args) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.stream = st;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 template <int P, int THREADS, int MINB>
 void launch_block_staged(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
   constexpr size_t smem = (size_t)Q * kSites * sizeof(typename Store<P>::S);
@@ -1410,7 +1393,7 @@ void launch_listed(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
   StepArgs b = a;
   b.io_ctas = (uint32_t)((a.n_io_links + THREADS - 1) / THREADS);
   b.let_in = g >= 4 * 152 * MINB;
-  if (g) launch_overlapped(k_stream_collide_listed<P, THREADS, MINB, MON>, (unsigned)g + b.io_ctas, THREADS, st, b, bxyz);
+  if (g) launch_overlapped(k_stream_collide_listed<P, THREADS, MINB, MON>, (unsigned)g + b.io_ctas, THREADS, 0, st, b, bxyz);
 }
 
 template <int P>
@@ -1887,7 +1870,7 @@ void launch_sc(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
   StepArgs b = a;
   b.io_ctas = (uint32_t)((a.n_io_links + THREADS - 1) / THREADS);
   b.let_in = g >= 4 * 152 * MINB;
-  if (g) launch_overlapped(k_stream_collide<P, THREADS, MINB, MON>, g + b.io_ctas, THREADS, st, b, bxyz);
+  if (g) launch_overlapped(k_stream_collide<P, THREADS, MINB, MON>, g + b.io_ctas, THREADS, 0, st, b, bxyz);
 }
 }  // namespace hlbg
 
@@ -1996,7 +1979,7 @@ int64_t monitored_ctas(int64_t nslot, int variant, int64_t n_warps) {
   }                                                                                             \
   void launch_post_step_##P(const PostArgs& p, cudaStream_t st) {                               \
     unsigned g = (unsigned)((p.count + 255) / 256);                                             \
-    if (g) launch_overlapped(k_post_step<P>, g, 256, st, p);                                    \
+    if (g) launch_overlapped(k_post_step<P>, g, 256, 0, st, p);                                 \
   }                                                                                             \
   void launch_init_uniform_##P(const InitArgs& ia, cudaStream_t st) {                           \
     unsigned g = (unsigned)((ia.nslot + 255) / 256);                                            \

@@ -15,6 +15,7 @@
 #include <cmath>
 
 #include "../../include/hemelb_gb300_nn.h"
+#include "overlap.cuh"
 
 namespace {
 
@@ -413,8 +414,9 @@ __global__ void __launch_bounds__(256) k_conv_brick(const __nv_bfloat16* __restr
 
 // Flipped, transposed weights for the data-gradient convolution:
 // wt[26 - tap][ci][co] = w[tap][co][ci]
-__global__ void k_flip_transpose(const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wt,
+__global__ void k_flip_transpose(const __nv_bfloat16* w, __nv_bfloat16* wt,
                                  int Cout, int Cin, int taps) {
+  wait_for_previous();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t n = (int64_t)taps * Cout * Cin;
   if (i >= n) return;
@@ -534,9 +536,10 @@ __global__ void k_mse(const float* __restrict__ pred, const float* __restrict__ 
   if ((threadIdx.x & 31) == 0) atomicAdd(loss, l);
 }
 // Adam on FP32 master weights, refreshing the BF16 copy
-__global__ void k_adam(float* __restrict__ w, __nv_bfloat16* __restrict__ wb, const float* __restrict__ g,
-                       float* __restrict__ m, float* __restrict__ v, int64_t n, float lr, float b1,
+__global__ void k_adam(float* w, __nv_bfloat16* wb, const float* g,
+                       float* m, float* v, int64_t n, float lr, float b1,
                        float b2, float eps, float c1, float c2) {
+  wait_for_previous();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float gi = g[i];
@@ -567,6 +570,12 @@ __global__ void k_f32_to_bf16(const float* __restrict__ x, __nv_bfloat16* __rest
 // (us): ReLU mask and bias sums 1457 + 2842 -> 318; upsampling and concatenation
 // 1272 + 1116 -> 123; their gradients 214 + 1027 -> 111; loss 2872 (one atomic per
 // warp on one word) -> 83 (6.9 TB/s); pooling gradient and sum 486 + 218 -> 50.
+// These kernels, the Adam update, the flipped weights and the tcgen05 kernels are
+// overlapped launches: each starts, up to its wait, while the last CTAs before it run,
+// which takes 1.9 us off each of a training step's 148 launches.  They let their
+// successor in at their exit: CTAs let in earlier sit beside the running ones and end up
+// unevenly on the SMs (training step 4580 us with ordinary launches, 4500 let in at the
+// start, 4305 at the exit; prediction 448, 409, 399).
 // ---------------------------------------------------------------------------
 struct V8 {
   float v[8];
@@ -599,8 +608,9 @@ __device__ __forceinline__ uint32_t mask_positive(uint32_t d, uint32_t y) {
 // dy *= (y > 0) in place (y not null) and db[c] += sum_m dy[m, c] (db not null).  A
 // thread keeps one group of 8 channels (G groups) and walks the voxels; four rows in
 // flight per thread.
-__global__ void __launch_bounds__(256) k_relu_bias_v8(uint4* __restrict__ dy, const uint4* __restrict__ y,
-                                                      float* __restrict__ db, uint32_t M, uint32_t G) {
+__global__ void __launch_bounds__(256) k_relu_bias_v8(uint4* dy, const uint4* y,
+                                                      float* db, uint32_t M, uint32_t G) {
+  wait_for_previous();
   __shared__ float sh[256 * 8];
   const uint32_t rows = 256u / G, r = threadIdx.x / G, g = threadIdx.x - r * G;
   float acc[8];
@@ -614,7 +624,7 @@ __global__ void __launch_bounds__(256) k_relu_bias_v8(uint4* __restrict__ dy, co
       for (int u = 0; u < 4; ++u) {
         const uint32_t mu = m + u * step;
         d[u] = mu < M ? dy[(size_t)mu * G + g] : make_uint4(0u, 0u, 0u, 0u);
-        if (y) yy[u] = mu < M ? __ldg(y + (size_t)mu * G + g) : make_uint4(0u, 0u, 0u, 0u);
+        if (y) yy[u] = mu < M ? *(y + (size_t)mu * G + g) : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -657,15 +667,16 @@ __device__ __forceinline__ uint32_t fine_at(const Fine& f, int k) {  // k = 4 z 
   return f.first + (k >> 2) * f.zs + ((k >> 1) & 1) * f.ys + (k & 1);
 }
 
-__global__ void __launch_bounds__(256) k_pool2_v8(const uint4* __restrict__ x, uint4* __restrict__ y, uint32_t nv,
+__global__ void __launch_bounds__(256) k_pool2_v8(const uint4* x, uint4* y, uint32_t nv,
                                                   uint32_t G, uint32_t D, uint32_t H, uint32_t W) {
+  wait_for_previous();
   const uint32_t i = blockIdx.x * 256 + threadIdx.x;
   if (i >= nv) return;
   const uint32_t cv = i / G, g = i - cv * G;
   const Fine f = fine_of(cv, D, H, W);
   uint4 u[8];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) u[k] = __ldg(x + (size_t)fine_at(f, k) * G + g);
+  for (int k = 0; k < 8; ++k) u[k] = *(x + (size_t)fine_at(f, k) * G + g);
   V8 s = {};
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
@@ -679,14 +690,15 @@ __global__ void __launch_bounds__(256) k_pool2_v8(const uint4* __restrict__ x, u
 }
 // dx = dy / 8 spread over the 8 fine voxels (acc null), or acc += that (rounded to
 // BF16 first, as the two passes round)
-__global__ void __launch_bounds__(256) k_pool2_bwd_v8(const uint4* __restrict__ dy, uint4* __restrict__ dx,
+__global__ void __launch_bounds__(256) k_pool2_bwd_v8(const uint4* dy, uint4* dx,
                                                       uint32_t nv, uint32_t G, uint32_t D, uint32_t H, uint32_t W,
                                                       int add) {
+  wait_for_previous();
   const uint32_t i = blockIdx.x * 256 + threadIdx.x;
   if (i >= nv) return;
   const uint32_t cv = i / G, g = i - cv * G;
   const Fine f = fine_of(cv, D, H, W);
-  V8 v = unpack8(__ldg(dy + i));
+  V8 v = unpack8(*(dy + i));
 #pragma unroll
   for (int c = 0; c < 8; ++c) v.v[c] *= 0.125f;
   const uint4 q = pack8(v);
@@ -708,37 +720,39 @@ __global__ void __launch_bounds__(256) k_pool2_bwd_v8(const uint4* __restrict__ 
   }
 }
 // y (fine, Ga + Gb groups a voxel) = [x of the coarse voxel | skip]
-__global__ void __launch_bounds__(256) k_up2_concat_v8(const uint4* __restrict__ x, uint32_t Ga,
-                                                       const uint4* __restrict__ skip, uint32_t Gb,
-                                                       uint4* __restrict__ y, uint32_t nv, uint32_t D, uint32_t H,
+__global__ void __launch_bounds__(256) k_up2_concat_v8(const uint4* x, uint32_t Ga,
+                                                       const uint4* skip, uint32_t Gb,
+                                                       uint4* y, uint32_t nv, uint32_t D, uint32_t H,
                                                        uint32_t W) {
+  wait_for_previous();
   const uint32_t i = blockIdx.x * 256 + threadIdx.x, G = Ga + Gb;
   if (i >= nv) return;
   const uint32_t cv = i / G, g = i - cv * G;
   const Fine f = fine_of(cv, D, H, W);
   if (g < Ga) {
-    const uint4 v = __ldg(x + (size_t)cv * Ga + g);
+    const uint4 v = *(x + (size_t)cv * Ga + g);
 #pragma unroll
     for (int k = 0; k < 8; ++k) y[(size_t)fine_at(f, k) * G + g] = v;
   } else {
     uint4 v[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = __ldg(skip + (size_t)fine_at(f, k) * Gb + (g - Ga));
+    for (int k = 0; k < 8; ++k) v[k] = *(skip + (size_t)fine_at(f, k) * Gb + (g - Ga));
 #pragma unroll
     for (int k = 0; k < 8; ++k) y[(size_t)fine_at(f, k) * G + g] = v[k];
   }
 }
 // its gradient: dx (coarse) = sum of the 8 fine values, dskip = the other channels
-__global__ void __launch_bounds__(256) k_up2_split_v8(const uint4* __restrict__ dy, uint4* __restrict__ dx,
-                                                      uint32_t Ga, uint4* __restrict__ dskip, uint32_t Gb,
+__global__ void __launch_bounds__(256) k_up2_split_v8(const uint4* dy, uint4* dx,
+                                                      uint32_t Ga, uint4* dskip, uint32_t Gb,
                                                       uint32_t nv, uint32_t D, uint32_t H, uint32_t W) {
+  wait_for_previous();
   const uint32_t i = blockIdx.x * 256 + threadIdx.x, G = Ga + Gb;
   if (i >= nv) return;
   const uint32_t cv = i / G, g = i - cv * G;
   const Fine f = fine_of(cv, D, H, W);
   uint4 u[8];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) u[k] = __ldg(dy + (size_t)fine_at(f, k) * G + g);
+  for (int k = 0; k < 8; ++k) u[k] = *(dy + (size_t)fine_at(f, k) * G + g);
   if (g < Ga) {
     V8 s = {};
 #pragma unroll
@@ -755,9 +769,10 @@ __global__ void __launch_bounds__(256) k_up2_split_v8(const uint4* __restrict__ 
 }
 
 // Masked squared error, 4 values of one voxel per vector (C a multiple of 4)
-__global__ void __launch_bounds__(256) k_mse_v4(const float4* __restrict__ pred, const float4* __restrict__ target,
-                                                const float* __restrict__ mask, uint2* __restrict__ dpred,
-                                                float* __restrict__ loss, uint32_t nv, uint32_t G, float inv_count) {
+__global__ void __launch_bounds__(256) k_mse_v4(const float4* pred, const float4* target,
+                                                const float* mask, uint2* dpred,
+                                                float* loss, uint32_t nv, uint32_t G, float inv_count) {
+  wait_for_previous();
   __shared__ float sh[8];
   float l = 0.f;
   const uint32_t step = gridDim.x * 256;
@@ -768,9 +783,9 @@ __global__ void __launch_bounds__(256) k_mse_v4(const float4* __restrict__ pred,
     for (int u = 0; u < 4; ++u) {
       const uint32_t i = i0 + u * step;
       const bool ok = i < nv;
-      p[u] = ok ? __ldg(pred + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-      t[u] = ok ? __ldg(target + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-      mk[u] = ok ? __ldg(mask + i / G) : 0.f;
+      p[u] = ok ? *(pred + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      t[u] = ok ? *(target + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      mk[u] = ok ? *(mask + i / G) : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -808,8 +823,8 @@ inline bool relu_bias(void* dy, const void* y, float* db, int64_t m, int32_t c, 
   if (!vec8(m * c, c) || c > 2048 || m >= 0x7fff0000ll || !aligned16(dy, y)) return false;
   const uint32_t G = (uint32_t)c / 8, rows = 256 / G;
   const int64_t want = (m + 4 * rows - 1) / (4 * rows);
-  k_relu_bias_v8<<<(unsigned)std::min<int64_t>(want, 1216), 256, 0, st>>>((uint4*)dy, (const uint4*)y, db, (uint32_t)m,
-                                                                          G);
+  launch_overlapped(k_relu_bias_v8, (unsigned)std::min<int64_t>(want, 1216), 256, 0, st, (uint4*)dy, (const uint4*)y, db,
+                    (uint32_t)m, G);
   return true;
 }
 
@@ -900,8 +915,8 @@ int hlbg_nn_conv3d_wgrad(const void* x, int32_t cin, const void* dy, int32_t cou
 
 int hlbg_nn_flip_transpose(const void* w, void* wt, int32_t cout, int32_t cin, int32_t taps, void* stream) {
   const int64_t n = (int64_t)taps * cout * cin;
-  k_flip_transpose<<<blocks(n), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)w, (__nv_bfloat16*)wt,
-                                                                  cout, cin, taps);
+  launch_overlapped(k_flip_transpose, blocks(n), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)w,
+                    (__nv_bfloat16*)wt, cout, cin, taps);
   return check_launch();
 }
 
@@ -931,9 +946,9 @@ int hlbg_nn_pool2(const void* x, void* y, int32_t n, int32_t d, int32_t h, int32
   if (vec8(fine, c) && even3(d, h, w) && aligned16(x, y)) {
     const uint32_t nv = (uint32_t)(fine / 64);
     if (!backward)
-      k_pool2_v8<<<blocks(nv), 256, 0, st>>>((const uint4*)x, (uint4*)y, nv, c / 8, d, h, w);
+      launch_overlapped(k_pool2_v8, blocks(nv), 256, 0, st, (const uint4*)x, (uint4*)y, nv, c / 8, d, h, w);
     else
-      k_pool2_bwd_v8<<<blocks(nv), 256, 0, st>>>((const uint4*)x, (uint4*)y, nv, c / 8, d, h, w, 0);
+      launch_overlapped(k_pool2_bwd_v8, blocks(nv), 256, 0, st, (const uint4*)x, (uint4*)y, nv, c / 8, d, h, w, 0);
     return check_launch();
   }
   if (!backward) {
@@ -952,12 +967,14 @@ int hlbg_nn_up2(const void* x, void* y, int32_t n, int32_t d, int32_t h, int32_t
   const int64_t cnt = (int64_t)n * d * h * w * c;
   if (!backward && vec8(cnt, c) && even3(d, h, w) && aligned16(x, y)) {
     const uint32_t nv = (uint32_t)(cnt / 64);
-    k_up2_concat_v8<<<blocks(nv), 256, 0, st>>>((const uint4*)x, c / 8, nullptr, 0, (uint4*)y, nv, d, h, w);
+    launch_overlapped(k_up2_concat_v8, blocks(nv), 256, 0, st, (const uint4*)x, c / 8, (const uint4*)nullptr, 0,
+                      (uint4*)y, nv, d, h, w);
     return check_launch();
   }
   if (backward && vec8(8 * cnt, c) && aligned16(x, y)) {
     const uint32_t nv = (uint32_t)(cnt / 8);
-    k_up2_split_v8<<<blocks(nv), 256, 0, st>>>((const uint4*)x, (uint4*)y, c / 8, nullptr, 0, nv, 2 * d, 2 * h, 2 * w);
+    launch_overlapped(k_up2_split_v8, blocks(nv), 256, 0, st, (const uint4*)x, (uint4*)y, c / 8, (uint4*)nullptr, 0, nv,
+                      2 * d, 2 * h, 2 * w);
     return check_launch();
   }
   if (!backward)  // d, h, w fine sizes
@@ -986,8 +1003,8 @@ int hlbg_nn_up2_concat(const void* x, int32_t ca, const void* skip, int32_t cb, 
   const int64_t cnt = (int64_t)n * d * h * w * (ca + cb);
   if (ca <= 0 || cb <= 0 || ca % 8 || cb % 8 || !vec8(cnt, ca + cb) || !even3(d, h, w) || !aligned16(x, skip, y)) return 1;
   const uint32_t nv = (uint32_t)(cnt / 64);
-  k_up2_concat_v8<<<blocks(nv), 256, 0, (cudaStream_t)stream>>>((const uint4*)x, ca / 8, (const uint4*)skip, cb / 8,
-                                                                (uint4*)y, nv, d, h, w);
+  launch_overlapped(k_up2_concat_v8, blocks(nv), 256, 0, (cudaStream_t)stream, (const uint4*)x, ca / 8,
+                    (const uint4*)skip, cb / 8, (uint4*)y, nv, d, h, w);
   return check_launch();
 }
 
@@ -996,8 +1013,8 @@ int hlbg_nn_up2_split(const void* dy, void* dx, int32_t ca, void* dskip, int32_t
   const int64_t cnt = (int64_t)n * d * h * w * (ca + cb);
   if (ca <= 0 || cb <= 0 || ca % 8 || cb % 8 || !vec8(cnt, ca + cb) || !even3(d, h, w) || !aligned16(dy, dx, dskip)) return 1;
   const uint32_t nv = (uint32_t)(cnt / 64);
-  k_up2_split_v8<<<blocks(nv), 256, 0, (cudaStream_t)stream>>>((const uint4*)dy, (uint4*)dx, ca / 8, (uint4*)dskip,
-                                                               cb / 8, nv, d, h, w);
+  launch_overlapped(k_up2_split_v8, blocks(nv), 256, 0, (cudaStream_t)stream, (const uint4*)dy, (uint4*)dx, ca / 8,
+                    (uint4*)dskip, cb / 8, nv, d, h, w);
   return check_launch();
 }
 
@@ -1006,7 +1023,8 @@ int hlbg_nn_pool2_bwd_add(const void* dy, void* acc, int32_t n, int32_t d, int32
   const int64_t cnt = (int64_t)n * d * h * w * c;
   if (!vec8(cnt, c) || !even3(d, h, w) || !aligned16(dy, acc)) return 1;
   const uint32_t nv = (uint32_t)(cnt / 64);
-  k_pool2_bwd_v8<<<blocks(nv), 256, 0, (cudaStream_t)stream>>>((const uint4*)dy, (uint4*)acc, nv, c / 8, d, h, w, 1);
+  launch_overlapped(k_pool2_bwd_v8, blocks(nv), 256, 0, (cudaStream_t)stream, (const uint4*)dy, (uint4*)acc, nv, c / 8, d,
+                    h, w, 1);
   return check_launch();
 }
 
@@ -1020,8 +1038,8 @@ int hlbg_nn_mse(const float* pred, const float* target, const float* mask, void*
   if (c > 0 && c % 4 == 0 && m > 0 && m * c / 4 < 0x7fff0000ll && aligned16(pred, target, dpred)) {
     const uint32_t nv = (uint32_t)(m * c / 4);
     const unsigned g = std::min(blocks((nv + 3) / 4), 1216u);  // 8 CTAs a SM; one atomic per CTA
-    k_mse_v4<<<g, 256, 0, (cudaStream_t)stream>>>((const float4*)pred, (const float4*)target, mask, (uint2*)dpred, loss,
-                                                  nv, c / 4, inv_count);
+    launch_overlapped(k_mse_v4, g, 256, 0, (cudaStream_t)stream, (const float4*)pred, (const float4*)target, mask,
+                      (uint2*)dpred, loss, nv, c / 4, inv_count);
     return check_launch();
   }
   k_mse<<<blocks(m * c), 256, 0, (cudaStream_t)stream>>>(pred, target, mask, (__nv_bfloat16*)dpred, loss, m, c,
@@ -1032,7 +1050,8 @@ int hlbg_nn_mse(const float* pred, const float* target, const float* mask, void*
 int hlbg_nn_adam(float* w, void* wb, const float* g, float* m, float* v, int64_t n, float lr, float b1, float b2,
                  float eps, int32_t step, void* stream) {
   const float c1 = 1.f / (1.f - powf(b1, (float)step)), c2 = 1.f / (1.f - powf(b2, (float)step));
-  k_adam<<<blocks(n), 256, 0, (cudaStream_t)stream>>>(w, (__nv_bfloat16*)wb, g, m, v, n, lr, b1, b2, eps, c1, c2);
+  launch_overlapped(k_adam, blocks(n), 256, 0, (cudaStream_t)stream, w, (__nv_bfloat16*)wb, g, m, v, n, lr, b1, b2, eps,
+                    c1, c2);
   return check_launch();
 }
 

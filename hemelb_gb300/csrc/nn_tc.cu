@@ -64,6 +64,7 @@
 #include <mutex>
 
 #include "../../include/hemelb_gb300_nn.h"
+#include "overlap.cuh"
 
 namespace {
 
@@ -288,8 +289,10 @@ __global__ void __launch_bounds__(320, 2) k_conv3d_tc(const __grid_constant__ CU
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  // the loads wait for the kernel before this one, and with them all that depends on them
+  if (warp < 2 || (warp >= 4 && warp < 8)) wait_for_previous();
   if (warp >= 4 && warp < 8)
-    for (int c = threadIdx.x - 128; c < p.ct; c += 128) bias_sh[c] = p.bias ? __ldg(p.bias + co0 + c) : 0.f;
+    for (int c = threadIdx.x - 128; c < p.ct; c += 128) bias_sh[c] = p.bias ? p.bias[co0 + c] : 0.f;
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -804,7 +807,8 @@ int hlbg_nn_conv3d_tc(const void* in, int32_t cin, const void* w, const float* b
   // persistent CTAs, as many as the SMs hold, over the tiles of each block of output channels
   const int ny = cout / pl.ct;
   const unsigned gx = (unsigned)std::min<int64_t>(tiles, std::max(1, kSms * pl.per_sm / ny));
-  kernel<<<dim3(gx, (unsigned)ny), conv_threads(pl.cols), pl.smem, static_cast<cudaStream_t>(stream)>>>(tin, tw, p);
+  launch_overlapped(kernel, dim3(gx, (unsigned)ny), conv_threads(pl.cols), pl.smem, static_cast<cudaStream_t>(stream),
+                    tin, tw, p);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 

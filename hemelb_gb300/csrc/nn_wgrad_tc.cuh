@@ -151,6 +151,7 @@ __global__ void __launch_bounds__(kWgThreads, 2) k_wgrad_tc(const __grid_constan
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
+  if (warp == 0) wait_for_previous();  // the loads, and with them all that depends on them
   if (warp == 0) {
     // ---- loads, one thread: per tile A's plane and the planes of B that are not there ----
     if (lane == 0) {
@@ -475,6 +476,6 @@ int wgrad_tc(const void* x, int cin, const void* dy, int cout, float* dw, int n,
                                     : wg_kernel<128>(pl.wb, pl.zg, taps);
   // a per-device attribute of the kernel, always the same value (several threads may be here)
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemDyn) != cudaSuccess) return 3;
-  kernel<<<(unsigned)std::min<int64_t>(units, ctas), kWgThreads, pl.smem, st>>>(ta, tb, p);
+  launch_overlapped(kernel, (unsigned)std::min<int64_t>(units, ctas), kWgThreads, pl.smem, st, ta, tb, p);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
