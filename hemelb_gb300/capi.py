@@ -191,6 +191,8 @@ SIGNATURES = {
                               C.c_int32, C.c_float, C.c_void_p]),
     "hlbg_nn_adam": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64,
                                C.c_float, C.c_float, C.c_float, C.c_float, C.c_int32, C.c_void_p]),
+    "hlbg_nn_adam_list": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32,
+                                    C.c_float, C.c_float, C.c_float, C.c_float, C.c_int32, C.c_void_p]),
     "hlbg_nn_to_bf16": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]),
 }
 

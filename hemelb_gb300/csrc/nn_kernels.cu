@@ -413,15 +413,25 @@ __global__ void __launch_bounds__(256) k_conv_brick(const __nv_bfloat16* __restr
 }
 
 // Flipped, transposed weights for the data-gradient convolution:
-// wt[26 - tap][ci][co] = w[tap][co][ci]
-__global__ void k_flip_transpose(const __nv_bfloat16* w, __nv_bfloat16* wt,
-                                 int Cout, int Cin, int taps) {
+// wt[taps - 1 - tap][ci][co] = w[tap][co][ci], 32 x 32 channels of a tap by a CTA through
+// shared memory, so that both sides are 64-byte runs (192 -> 192 channels, 27 taps, 2 MB:
+// 12.4 us with a thread per value, whose stores lay C_out values apart, 4.5 now).
+__global__ void __launch_bounds__(256) k_flip_transpose(const __nv_bfloat16* w, __nv_bfloat16* wt, int Cout, int Cin,
+                                                        int taps) {
+  __shared__ __nv_bfloat16 tile[32][34];
   wait_for_previous();
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t n = (int64_t)taps * Cout * Cin;
-  if (i >= n) return;
-  const int ci = (int)(i % Cin), co = (int)((i / Cin) % Cout), tap = (int)(i / ((int64_t)Cin * Cout));
-  wt[((int64_t)(taps - 1 - tap) * Cin + ci) * Cout + co] = w[i];
+  const unsigned nci = (unsigned)(Cin + 31) / 32, nco = (unsigned)(Cout + 31) / 32, q = blockIdx.x / nci;
+  const int ci0 = (int)(blockIdx.x - q * nci) * 32, co0 = (int)(q % nco) * 32, tap = (int)(q / nco);
+  const int a = threadIdx.x & 31, b = threadIdx.x >> 5;
+  const __nv_bfloat16* src = w + (int64_t)tap * Cout * Cin;
+  __nv_bfloat16* dst = wt + (int64_t)(taps - 1 - tap) * Cout * Cin;
+#pragma unroll
+  for (int k = b; k < 32; k += 8)
+    if (co0 + k < Cout && ci0 + a < Cin) tile[k][a] = src[(int64_t)(co0 + k) * Cin + ci0 + a];
+  __syncthreads();
+#pragma unroll
+  for (int k = b; k < 32; k += 8)
+    if (ci0 + k < Cin && co0 + a < Cout) dst[(int64_t)(ci0 + k) * Cout + co0 + a] = tile[a][k];
 }
 
 // ReLU gradient in place: dy *= (y > 0)
@@ -535,21 +545,54 @@ __global__ void k_mse(const float* __restrict__ pred, const float* __restrict__ 
   for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
   if ((threadIdx.x & 31) == 0) atomicAdd(loss, l);
 }
-// Adam on FP32 master weights, refreshing the BF16 copy
-__global__ void k_adam(float* w, __nv_bfloat16* wb, const float* g,
-                       float* m, float* v, int64_t n, float lr, float b1,
-                       float b2, float eps, float c1, float c2) {
+// Adam on FP32 master weights, refreshing the BF16 copies: up to kAdamTensors tensors in
+// a launch, 1,024 values of one tensor by a CTA.  A network has two tensors a layer, most
+// of them small: one launch a tensor took 110 us for a step of the U-Net (30 tensors, 3.2M
+// values) beside the gaps between them, this takes 15.
+constexpr int kAdamTensors = 32, kAdamBlock = 1024;
+struct AdamList {
+  float* w[kAdamTensors];
+  __nv_bfloat16* wb[kAdamTensors];
+  const float* g[kAdamTensors];
+  float* m[kAdamTensors];
+  float* v[kAdamTensors];
+  int64_t n[kAdamTensors];
+  uint32_t first[kAdamTensors + 1];  // CTA each tensor starts at; the end
+  int count;
+};
+__global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamList a, float lr, float b1, float b2, float eps,
+                                              float c1, float c2) {
+  int t = 0;
+  while (t + 1 < a.count && blockIdx.x >= a.first[t + 1]) ++t;
+  const int64_t i0 = (int64_t)(blockIdx.x - a.first[t]) * kAdamBlock + threadIdx.x;
+  float *w = a.w[t], *m = a.m[t], *v = a.v[t];
+  const float* g = a.g[t];
+  __nv_bfloat16* wb = a.wb[t];
+  const int64_t n = a.n[t];
   wait_for_previous();
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.f - b1) * gi;
-  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float wi = w[i] - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-  w[i] = wi;
-  if (wb) wb[i] = __float2bfloat16_rn(wi);
+  float gi[4], mi[4], vi[4], wi[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int64_t i = i0 + k * 256;
+    if (i < n) {
+      gi[k] = g[i];
+      mi[k] = m[i];
+      vi[k] = v[i];
+      wi[k] = w[i];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int64_t i = i0 + k * 256;
+    if (i >= n) break;
+    const float mn = b1 * mi[k] + (1.f - b1) * gi[k];
+    const float vn = b2 * vi[k] + (1.f - b2) * gi[k] * gi[k];
+    m[i] = mn;
+    v[i] = vn;
+    const float wn = wi[k] - lr * (mn * c1) / (sqrtf(vn * c2) + eps);
+    w[i] = wn;
+    if (wb) wb[i] = __float2bfloat16_rn(wn);
+  }
 }
 __global__ void k_f32_to_bf16(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, int64_t n) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -572,7 +615,7 @@ __global__ void k_f32_to_bf16(const float* __restrict__ x, __nv_bfloat16* __rest
 // warp on one word) -> 83 (6.9 TB/s); pooling gradient and sum 486 + 218 -> 50.
 // These kernels, the Adam update, the flipped weights and the tcgen05 kernels are
 // overlapped launches: each starts, up to its wait, while the last CTAs before it run,
-// which takes 1.9 us off each of a training step's 148 launches.  They let their
+// which took 1.9 us off each of a training step's 148 launches (90 since).  They let their
 // successor in at their exit: CTAs let in earlier sit beside the running ones and end up
 // unevenly on the SMs (training step 4580 us with ordinary launches, 4500 let in at the
 // start, 4305 at the exit; prediction 448, 409, 399).
@@ -914,9 +957,9 @@ int hlbg_nn_conv3d_wgrad(const void* x, int32_t cin, const void* dy, int32_t cou
 }
 
 int hlbg_nn_flip_transpose(const void* w, void* wt, int32_t cout, int32_t cin, int32_t taps, void* stream) {
-  const int64_t n = (int64_t)taps * cout * cin;
-  launch_overlapped(k_flip_transpose, blocks(n), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)w,
-                    (__nv_bfloat16*)wt, cout, cin, taps);
+  const int64_t tiles = (int64_t)((cin + 31) / 32) * ((cout + 31) / 32) * taps;
+  launch_overlapped(k_flip_transpose, (unsigned)tiles, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)w, (__nv_bfloat16*)wt,
+                    cout, cin, taps);
   return check_launch();
 }
 
@@ -1047,12 +1090,38 @@ int hlbg_nn_mse(const float* pred, const float* target, const float* mask, void*
   return check_launch();
 }
 
+int hlbg_nn_adam_list(float* const* w, void* const* wb, const float* const* g, float* const* m, float* const* v,
+                      const int64_t* n, int32_t count, float lr, float b1, float b2, float eps, int32_t step,
+                      void* stream) {
+  if (count < 0 || (count > 0 && (!w || !wb || !g || !m || !v || !n))) return 1;
+  const float c1 = 1.f / (1.f - powf(b1, (float)step)), c2 = 1.f / (1.f - powf(b2, (float)step));
+  AdamList a;
+  a.count = 0;
+  a.first[0] = 0;
+  for (int32_t i = 0; i < count; ++i) {
+    const int64_t ctas = (n[i] + kAdamBlock - 1) / kAdamBlock;
+    if (n[i] < 0 || ctas > 0x3fffffff) return 1;
+    if (ctas > 0) {
+      const int k = a.count++;
+      a.w[k] = w[i];
+      a.wb[k] = static_cast<__nv_bfloat16*>(wb[i]);
+      a.g[k] = g[i];
+      a.m[k] = m[i];
+      a.v[k] = v[i];
+      a.n[k] = n[i];
+      a.first[k + 1] = a.first[k] + (uint32_t)ctas;
+    }
+    if (a.count == 0 || (a.count < kAdamTensors && i + 1 < count && a.first[a.count] < 0x3fffffffu)) continue;
+    launch_overlapped(k_adam, a.first[a.count], 256, 0, (cudaStream_t)stream, a, lr, b1, b2, eps, c1, c2);
+    a.count = 0;
+  }
+  return check_launch();
+}
+
 int hlbg_nn_adam(float* w, void* wb, const float* g, float* m, float* v, int64_t n, float lr, float b1, float b2,
                  float eps, int32_t step, void* stream) {
-  const float c1 = 1.f / (1.f - powf(b1, (float)step)), c2 = 1.f / (1.f - powf(b2, (float)step));
-  launch_overlapped(k_adam, blocks(n), 256, 0, (cudaStream_t)stream, w, (__nv_bfloat16*)wb, g, m, v, n, lr, b1, b2, eps,
-                    c1, c2);
-  return check_launch();
+  if (n <= 0) return 3;  // as a launch of no threads
+  return hlbg_nn_adam_list(&w, &wb, &g, &m, &v, &n, 1, lr, b1, b2, eps, step, stream);
 }
 
 int hlbg_nn_to_bf16(const float* x, void* y, int64_t n, void* stream) {

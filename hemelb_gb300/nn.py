@@ -7,6 +7,8 @@ current stream.  There is no fallback: the kernels are the implementation.
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import torch
 
 from . import capi
@@ -271,6 +273,21 @@ def adam(w, wb, g, m, v, lr, step, b1=0.9, b2=0.999, eps=1e-8):
         _need(wb, _BF16, "adam bf16 copy")
     _ok(_lib().hlbg_nn_adam(_p(w), _p(wb), _p(g), _p(m), _p(v), w.numel(), lr, b1, b2, eps, step,
                             _stream()), "hlbg_nn_adam")
+
+
+def adam_list(tensors, lr, step, b1=0.9, b2=0.999, eps=1e-8):
+    """adam for a list of (w, wb or None, g, m, v) in one launch per 32 tensors."""
+    for w, wb, g, m, v in tensors:
+        for t, n in ((w, "adam w"), (g, "adam g"), (m, "adam m"), (v, "adam v")):
+            _need(t, _F32, n)
+        if wb is not None:
+            _need(wb, _BF16, "adam bf16 copy")
+        if not w.numel() == g.numel() == m.numel() == v.numel() == (w if wb is None else wb).numel():
+            raise ValueError("adam_list sizes")
+    k = len(tensors)
+    ptrs = [(C.c_void_p * k)(*map(_p, column)) for column in zip(*tensors)] if k else [None] * 5
+    sizes = (C.c_int64 * k)(*(t[0].numel() for t in tensors))
+    _ok(_lib().hlbg_nn_adam_list(*ptrs, sizes, k, lr, b1, b2, eps, step, _stream()), "hlbg_nn_adam_list")
 
 
 def to_bf16(x, y):

@@ -257,8 +257,11 @@ class Conv:
         self.gb.zero_()
 
     def step(self, lr, t):
-        nn.adam(self.w, self.wb, self.gw, self.mw, self.vw, lr, t)
-        nn.adam(self.b, None, self.gb, self.mb, self.vb, lr, t)
+        nn.adam_list(self.tensors(), lr, t)
+
+    def tensors(self):
+        """What an Adam update takes: (w, BF16 copy, gradient, moments) of weights and bias."""
+        return ((self.w, self.wb, self.gw, self.mw, self.vw), (self.b, None, self.gb, self.mb, self.vb))
 
     def state(self):
         return {"w": self.w.cpu().numpy(), "b": self.b.cpu().numpy()}
@@ -354,13 +357,11 @@ class UNet:
         self._saved = None
 
     def zero_grad(self):
-        for c in self.L.values():
-            c.zero_grad()
+        torch._foreach_zero_([g for c in self.L.values() for g in (c.gw, c.gb)])
 
     def step(self, lr):
         self.t += 1
-        for c in self.L.values():
-            c.step(lr, self.t)
+        nn.adam_list([t for c in self.L.values() for t in c.tensors()], lr, self.t)
 
     def state(self):
         return {k: c.state() for k, c in self.L.items()}

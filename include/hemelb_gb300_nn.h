@@ -75,6 +75,11 @@ int hlbg_nn_mse(const float *pred, const float *target, const float *mask, void 
 /* Adam step `step` (1-based) on FP32 weights, refreshing the BF16 copy wb (may be NULL) */
 int hlbg_nn_adam(float *w, void *wb, const float *g, float *m, float *v, int64_t n, float lr,
                  float b1, float b2, float eps, int32_t step, void *stream);
+/* The same for `count` tensors, 32 in a launch: tensor i has n[i] values (none: passed over)
+ * at w[i], wb[i] (may be NULL), g[i], m[i], v[i]; the arrays are the host's. */
+int hlbg_nn_adam_list(float *const *w, void *const *wb, const float *const *g, float *const *m, float *const *v,
+                      const int64_t *n, int32_t count, float lr, float b1, float b2, float eps, int32_t step,
+                      void *stream);
 int hlbg_nn_to_bf16(const float *x, void *y, int64_t n, void *stream);
 
 #ifdef __cplusplus

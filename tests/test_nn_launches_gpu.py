@@ -10,7 +10,7 @@ torch = pytest.importorskip("torch")
 
 from hemelb_gb300 import nn, surrogate  # noqa: E402
 
-CALLS = ("conv3d", "up2_concat", "up2_split", "pool2", "pool2_backward_add", "flip_transpose", "adam",
+CALLS = ("conv3d", "up2_concat", "up2_split", "pool2", "pool2_backward_add", "flip_transpose", "adam_list",
          "relu_bias_backward", "bias_grad", "conv3d_weight_grad", "mse")
 
 
