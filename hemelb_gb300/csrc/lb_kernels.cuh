@@ -369,8 +369,61 @@ struct PushEach<P, Q, XFACE> {
   static __device__ __forceinline__ void run(const PushTargets<P, false>&, const StepArgs&, const T*) {}
 };
 
+// The interpolated links (BFL, q >= 1/2) of one warp, gathered: of a warp's 32 sites a few
+// have such links, in most of the 18 directions, and an FP64 instruction takes the warp
+// its 16 cycles however few lanes take part.  So the links' operands go to shared memory
+// and 32 links are evaluated at a time (14 FP64 instructions, a division among them)
+// instead of each direction's by themselves: FP64 bifurcation of 1.5M sites 678 -> 615 us
+// a step.
+struct BflQueue {
+  double out[64], back[64];  // post-collision values along the link and against it
+  float q[64];
+  int32_t to[64];            // element of the block
+};
+struct BflGather {
+  BflQueue& s;
+  double* block;
+  const StepArgs& a;
+  int count;
+  // entries first .. first + n - 1 (n <= 32), one by lane
+  __device__ __forceinline__ void eval(int first, int n) {
+    __syncwarp();
+    const int lane = threadIdx.x & 31, k = first + lane;
+    if (lane < n) {
+      const double q = (double)s.q[k];
+      Store<0>::store(block, s.to[k], (s.out[k] + (2.0 * q - 1.0) * s.back[k]) / (2.0 * q), a);
+    }
+    __syncwarp();
+  }
+  template <int D>
+  __device__ __forceinline__ void add(bool is, int j, int64_t r, const double* fpost) {
+    const unsigned m = __ballot_sync(0xffffffffu, is);
+    if (m == 0) return;
+    if (is) {
+      const int k = count + __popc(m & ((1u << (threadIdx.x & 31)) - 1u));
+      s.out[k] = fpost[D];
+      s.back[k] = fpost[Lat::inv(D)];
+      s.q[k] = a.b_cut[r * (Q - 1) + D - 1];
+      s.to[k] = Lat::inv(D) * kSites + j;
+    }
+    count += __popc(m);
+    if (count >= 32) eval(count -= 32, 32);
+  }
+};
+template <int D>
+struct BflEach {
+  static __device__ __forceinline__ void run(BflGather& g, uint64_t links, int j, int64_t r, const double* fpost) {
+    g.add<D>(((unsigned)(links >> (3 * D)) & 7u) == HLBG_LC_BFL, j, r, fpost);
+    BflEach<D + 1>::run(g, links, j, r, fpost);
+  }
+};
+template <>
+struct BflEach<Q> {
+  static __device__ __forceinline__ void run(BflGather&, uint64_t, int, int64_t, const double*) {}
+};
+
 // Pushes of a warp that holds at least one boundary site: a boundary lane redirects the
-// link by its precomputed code as in PushMixed.
+// link by its precomputed code as in PushMixed (FP64: BFL links by BflGather).
 template <int P, int D, bool XFACE>
 struct PushEachMixed {
   template <class T>
@@ -391,7 +444,9 @@ struct PushEachMixed {
     } else if (lc != HLBG_LC_PUSH) {
       p = t.own + inv * kSites;
       st = lc != HLBG_LC_SKIP && lc != HLBG_LC_IOLET;  // iolet links: written by iolet_link
-      if (lc == HLBG_LC_BFL) {
+      if constexpr (P == 0) {
+        if (lc == HLBG_LC_BFL) st = false;
+      } else if (lc == HLBG_LC_BFL) {
         const T q = (T)a.b_cut[r * (Q - 1) + D - 1];
         v = (fpost[D] + ((T)2.0 * q - (T)1) * fpost[inv]) / ((T)2.0 * q);
       }
@@ -415,7 +470,8 @@ struct PushEachMixed<P, Q, XFACE> {
 // each push: beside its accumulators the nine pointers cost more in registers than they
 // save (12 steps of a monitored 7.8M-site FP32 tree: 4764 us with the lookups, 4811 with
 // the pointers).
-template <int P, bool MON, class T>
+// W: warps of the CTA.
+template <int P, bool MON, int W, class T>
 __device__ __forceinline__ void push_warp(const StepArgs& a, int64_t b, int32_t tabreg, int x, int y, int z, int j,
                                           uint32_t code, bool row_fluid, const T* fpost) {
   using S = typename Store<P>::S;
@@ -436,6 +492,14 @@ __device__ __forceinline__ void push_warp(const StepArgs& a, int64_t b, int32_t 
       const PushTargets<P, true> t(fn, b, tabreg, x, y, z, j);
       if (t.xface) PushEachMixed<P, 0, true>::run(t, a, code != 0, row_fluid, links, r, fpost);
       else PushEachMixed<P, 0, false>::run(t, a, code != 0, row_fluid, links, r, fpost);
+      if constexpr (P == 0) {
+        if (a.wall == 1) {
+          __shared__ BflQueue queue[W];
+          BflGather g{queue[threadIdx.x >> 5], static_cast<double*>(a.f_new) + b * (Q * kSites), a, 0};
+          BflEach<1>::run(g, links, j, r, fpost);
+          if (g.count) g.eval(0, g.count);
+        }
+      }
     }
     return;
   }
@@ -898,7 +962,7 @@ __global__ void __launch_bounds__(128) k_iolet_links(StepArgs a, const int32_t* 
 // One warp's 32 slots of one block (a warp never spans two blocks).  Lanes 0..26
 // hold the block's neighbour table and serve it to the bulk pushes by shuffle, so
 // every lane of a warp with any fluid site stays converged through the pushes.
-template <int P, bool MON>
+template <int P, bool MON, int W>
 __device__ __forceinline__ void collide_slot(const StepArgs& a, int64_t s, MonAccT<P>& acc) {
   using St = Store<P>;
   using S = typename St::S;
@@ -933,7 +997,7 @@ __device__ __forceinline__ void collide_slot(const StepArgs& a, int64_t s, MonAc
   if constexpr (MON) {
     if (code != 0) mon_site<P>(a, s, f, m0, mx, my, mz, acc, check, uo);
   }
-  push_warp<P, MON>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, row_fluid, fpost);
+  push_warp<P, MON, W>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, row_fluid, fpost);
 }
 
 // One warp of the fluid list: 32 fluid sites of one block (or the zero-fill of its
@@ -942,7 +1006,7 @@ __device__ __forceinline__ void collide_slot(const StepArgs& a, int64_t s, MonAc
 // stored nowhere) and push its post-collision values, on the warp's bulk path when
 // no lane has a boundary record.  tabreg: the block's neighbour table in lanes
 // 0..26.  Every lane of the warp must take part (shuffles, ballot).
-template <int P, bool MON>
+template <int P, bool MON, int W>
 __device__ __forceinline__ void collide_and_push(const StepArgs& a, int64_t b, int j, int64_t s, int l,
                                                  uint32_t code, int32_t tabreg, typename Calc<P>::T* f,
                                                  MonAccT<P>& acc, bool check, const MonOld<P>& uo) {
@@ -953,11 +1017,11 @@ __device__ __forceinline__ void collide_and_push(const StepArgs& a, int64_t b, i
   if constexpr (MON) {
     if (code != 0) mon_site<P>(a, s, f, m0, mx, my, mz, acc, check, uo);
   }
-  push_warp<P, MON>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, false, fpost);
+  push_warp<P, MON, W>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, false, fpost);
 }
 
 // The unit's list entries (block e, this lane's slot js) are loaded by the caller.
-template <int P, bool MON>
+template <int P, bool MON, int W>
 __device__ __forceinline__ void collide_listed_unit(const StepArgs& a, int32_t e, unsigned js,
                                                     MonAccT<P>& acc) {
   using St = Store<P>;
@@ -997,13 +1061,13 @@ __device__ __forceinline__ void collide_listed_unit(const StepArgs& a, int32_t e
 #pragma unroll
     for (int i = 0; i < Q; ++i) f[i] = (T)(P == 0 ? weight_d(i) : 0.0);
   }
-  collide_and_push<P, MON>(a, b, j, s, l, code, tabreg, f, acc, check, uo);
+  collide_and_push<P, MON, W>(a, b, j, s, l, code, tabreg, f, acc, check, uo);
 }
 
-template <int P, bool MON>
+template <int P, bool MON, int W>
 __device__ __forceinline__ void collide_listed_warp(const StepArgs& a, int64_t w, MonAccT<P>& acc) {
   if (w >= a.n_warps) return;  // whole warp
-  collide_listed_unit<P, MON>(a, __ldg(a.warp_block + w), __ldg(a.lane_slot + w * 32 + (threadIdx.x & 31)),
+  collide_listed_unit<P, MON, W>(a, __ldg(a.warp_block + w), __ldg(a.lane_slot + w * 32 + (threadIdx.x & 31)),
                               acc);
 }
 
@@ -1016,7 +1080,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_stream_collide_listed(StepArg
   }
   const unsigned cta = blockIdx.x - a.io_ctas;
   MonAccT<P> acc = mon_neutral_t<P>();
-  collide_listed_warp<P, MON>(a, ((int64_t)cta * THREADS + threadIdx.x) >> 5, acc);
+  collide_listed_warp<P, MON, THREADS / 32>(a, ((int64_t)cta * THREADS + threadIdx.x) >> 5, acc);
   if (!MON && !a.let_in) let_next_in();
   if constexpr (MON) {
     if (a.mon_fold) mon_finish<P>(a, acc, cta);
@@ -1149,7 +1213,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_stream_collide_block(StepArgs
       else
         f[d] = on ? __half2float(stage[d * kSites + j]) * a.fp16_inv_scale : 0.f;
     }
-    collide_and_push<P, false>(a, b, j, s, j, code, tabreg, f, acc, false, uo);
+    collide_and_push<P, false, 1>(a, b, j, s, j, code, tabreg, f, acc, false, uo);
   }
   // solid slots of the rows that hold fluid: zeros complete their sectors
   S* fn = static_cast<S*>(a.f_new);
@@ -1342,7 +1406,7 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) k_stream_collide_pipe(StepA
         else
           f[d] = on ? __half2float(stage[d * kSites + j]) * a.fp16_inv_scale : 0.f;
       }
-      collide_and_push<P, false>(a, b, j, s, j, code, tabreg, f, acc, false, uo);
+      collide_and_push<P, false, 1>(a, b, j, s, j, code, tabreg, f, acc, false, uo);
     }
     rot = (rot + ntask) % NCW;
     __syncwarp();
@@ -1421,7 +1485,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   }
   const unsigned cta = blockIdx.x - a.io_ctas;
   MonAccT<P> acc = mon_neutral_t<P>();
-  collide_slot<P, MON>(a, (int64_t)cta * THREADS + threadIdx.x, acc);
+  collide_slot<P, MON, THREADS / 32>(a, (int64_t)cta * THREADS + threadIdx.x, acc);
   if (!MON && !a.let_in) let_next_in();
   if constexpr (MON) {
     if (a.mon_fold) mon_finish<P>(a, acc, cta);

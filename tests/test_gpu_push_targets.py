@@ -40,7 +40,7 @@ def sparse_geometry(seed, shape, fill):
                 fluid_mask=np.packbits(fluid.reshape(-1, 64), axis=1, bitorder="little").view(np.uint64).copy(),
                 link_site=sites[edge].astype(np.int64), wall_mask=wall[edge].copy(),
                 iolet_mask=np.zeros(n, np.uint32), iolet_id=np.full(n, -1, np.int32),
-                site_type=np.ones(n, np.int8), cut_distance=np.full((n, 18), 0.5, np.float32))
+                site_type=np.ones(n, np.int8), cut_distance=rng.uniform(0.01, 0.99, (n, 18)).astype(np.float32))
     g = capi.Geometry()
     g.q, g.block_size, g.n_blocks, g.n_link_sites = 19, 8, len(coords), n
     g.blocks[:] = shape
@@ -73,6 +73,31 @@ def test_pushes_across_missing_blocks_fp64_bit_exact(fill, variant):
     s.DoTimeStep(3)
     o.step(3)
     assert np.array_equal(s.GetFOld(), o.fold())
+
+
+@pytest.mark.parametrize("fill", [0.3, 0.55, 0.97])
+@pytest.mark.parametrize("variant", [1, 6])
+def test_gathered_interpolated_links_fp64_bit_exact(fill, variant):
+    """BFL walls: from no interpolated link in a warp to several hundred."""
+    g = sparse_geometry(13, (2, 3, 3), fill)
+    p = LbmParameters(tau=0.8, precision=capi.FP64, wall=capi.WALL_BFL)
+    for monitored in (False, True):
+        s = LBM(g, p)
+        rho, u = start(s.n_sites, 7)
+        s.SetInitialField(rho, u)
+        s.SetLaunchVariant(variant)
+        f = s.GetFOld()
+        o = OracleLBM(g, p, [], [])
+        o.set_equilibrium()
+        o.f_old[: f.size] = f.reshape(-1)
+        o.f_new[: f.size] = s.GetFNew().reshape(-1)
+        if monitored:
+            for _ in range(3):
+                s.StepMonitored(1)
+        else:
+            s.DoTimeStep(3)
+        o.step(3)
+        assert np.array_equal(s.GetFOld(), o.fold())
 
 
 @pytest.mark.parametrize("precision", [capi.FP32DEV, capi.FP16])
