@@ -231,6 +231,22 @@ struct PushBulk<P, Q> {
                                              const T*) {}
 };
 
+// The code of direction D in a boundary record's links, tested bit by bit in place (one
+// logic operation each): 0 push, 1 skip, 2 bounce, 3 BFL, 4 iolet (HLBG_LC_*).
+template <int D>
+struct LinkAt {
+  uint64_t links;
+  __device__ __forceinline__ explicit LinkAt(uint64_t l) : links(l) {}
+  __device__ __forceinline__ bool push() const { return (links & (7ull << (3 * D))) == 0; }
+  __device__ __forceinline__ bool back() const { return (links & (2ull << (3 * D))) != 0; }  // bounce or BFL
+  __device__ __forceinline__ bool bounce() const { return (links & (3ull << (3 * D))) == 2ull << (3 * D); }
+};
+// BFL eq. 5b
+template <class T>
+__device__ __forceinline__ T bfl_value(T out, T back, T q) {
+  return (out + ((T)2.0 * q - (T)1) * back) / ((T)2.0 * q);
+}
+
 // Pushes of a warp that holds at least one boundary site.  Every lane computes
 // the bulk target (shuffles stay converged); a boundary lane then redirects the
 // link by its precomputed code: skip (the reference's rubbish site), bounce-back
@@ -239,7 +255,7 @@ template <int P, int D>
 struct PushMixed {
   template <class S, class T, class B>
   static __device__ __forceinline__ void run(S* fn, const StepArgs& a, const B& base, int x, int y,
-                                             int z, int j, int64_t own, bool active, bool row_fluid,
+                                             int z, int j, int64_t own, bool active, bool zero,
                                              uint64_t links, int64_t r, const T* fpost) {
     constexpr int cx = Lat::cx(D), cy = Lat::cy(D), cz = Lat::cz(D);
     constexpr int inv = Lat::inv(D);
@@ -247,34 +263,16 @@ struct PushMixed {
     const int k = 13 + 9 * (xx >> 3) + 3 * (yy >> 3) + (zz >> 3);
     const int tl = slot_in_block(xx & 7, yy & 7, zz & 7);
     const int32_t e = base(k);  // every lane shuffles
-    const unsigned lc = (unsigned)((links >> (3 * D)) & 7u);
-    int64_t off = 0;
-    T v = fpost[D];
-    bool st = true;
-    if (!active) {
-      // A solid slot is never written by a push nor ever read; a zero there completes
-      // the 32-byte sector of slots it shares with fluid slots (sectors without any
-      // receive no write at all and stay untouched).
-      off = own + D * kSites + j;
-      v = (T)0;
-      st = row_fluid;
-    } else if (lc == HLBG_LC_PUSH) {
-      off = target_off(a, e, D, tl);
-    } else {
-      if (lc == HLBG_LC_SKIP) {
-        st = false;
-      } else {
-        off = own + inv * kSites + j;
-        if (lc == HLBG_LC_BFL) {
-          const T q = (T)a.b_cut[r * (Q - 1) + D - 1];
-          v = (fpost[D] + ((T)2.0 * q - (T)1) * fpost[inv]) / ((T)2.0 * q);
-        }
-        if (lc == HLBG_LC_IOLET) st = false;  // written by iolet_link
-      }
+    const LinkAt<D> link(links);
+    if (active && link.push()) Store<P>::store(fn, target_off(a, e, D, tl), fpost[D], a);
+    if (link.back()) {
+      T v = fpost[D];
+      if (!link.bounce()) v = bfl_value(fpost[D], fpost[inv], (T)a.b_cut[r * (Q - 1) + D - 1]);
+      Store<P>::store(fn, own + inv * kSites + j, v, a);
     }
-    if (st) Store<P>::store(fn, off, v, a);
+    if (zero) Store<P>::store(fn, own + D * kSites + j, (T)0, a);
     push_fence();
-    PushMixed<P, D + 1>::run(fn, a, base, x, y, z, j, own, active, row_fluid, links, r, fpost);
+    PushMixed<P, D + 1>::run(fn, a, base, x, y, z, j, own, active, zero, links, r, fpost);
   }
 };
 template <int P>
@@ -391,7 +389,7 @@ struct BflGather {
     const int lane = threadIdx.x & 31, k = first + lane;
     if (lane < n) {
       const double q = (double)s.q[k];
-      Store<0>::store(block, s.to[k], (s.out[k] + (2.0 * q - 1.0) * s.back[k]) / (2.0 * q), a);
+      Store<0>::store(block, s.to[k], bfl_value(s.out[k], s.back[k], q), a);
     }
     __syncwarp();
   }
@@ -413,7 +411,8 @@ struct BflGather {
 template <int D>
 struct BflEach {
   static __device__ __forceinline__ void run(BflGather& g, uint64_t links, int j, int64_t r, const double* fpost) {
-    g.add<D>(((unsigned)(links >> (3 * D)) & 7u) == HLBG_LC_BFL, j, r, fpost);
+    const LinkAt<D> link(links);
+    g.add<D>(link.back() && !link.bounce(), j, r, fpost);
     BflEach<D + 1>::run(g, links, j, r, fpost);
   }
 };
@@ -423,40 +422,34 @@ struct BflEach<Q> {
 };
 
 // Pushes of a warp that holds at least one boundary site: a boundary lane redirects the
-// link by its precomputed code as in PushMixed (FP64: BFL links by BflGather).
-template <int P, int D, bool XFACE>
+// link by its precomputed code as in PushMixed (FP64: BFL links by BflGather).  A push and
+// a value sent back are two stores under two conditions, where one store of a selected
+// value to a selected address took twice the instructions; warps with boundary sites are
+// a third of all and the slowest.  BFL: the walls have interpolated links; without their
+// code in each of the 18 directions the other walls' warps are faster.  FP16 tree of 7.8M
+// sites 251 -> 233 us a step without that code, 231 with two stores; FP32 ensemble of 4.9M
+// 189 -> 182 -> 181; FP32 bifurcation (BFL) 69.3 -> 67.6; FP32 tree of 16.9M 573 -> 540.
+template <int P, int D, bool XFACE, bool BFL>
 struct PushEachMixed {
   template <class T>
   static __device__ __forceinline__ void run(const PushTargets<P, true>& t, const StepArgs& a, bool active,
-                                             bool row_fluid, uint64_t links, int64_t r, const T* fpost) {
+                                             bool zero, uint64_t links, int64_t r, const T* fpost) {
     constexpr int inv = Lat::inv(D);
-    const unsigned lc = (unsigned)(links >> (3 * D)) & 7u;
-    typename Store<P>::S* p = t.template at<D, XFACE>() + D * kSites;
-    T v = fpost[D];
-    bool st = true;
-    if (!active) {
-      // A solid slot is never written by a push nor ever read; a zero there completes
-      // the 32-byte sector of slots it shares with fluid slots (sectors without any
-      // receive no write at all and stay untouched).
-      p = t.own + D * kSites;
-      v = (T)0;
-      st = row_fluid;
-    } else if (lc != HLBG_LC_PUSH) {
-      p = t.own + inv * kSites;
-      st = lc != HLBG_LC_SKIP && lc != HLBG_LC_IOLET;  // iolet links: written by iolet_link
-      if constexpr (P == 0) {
-        if (lc == HLBG_LC_BFL) st = false;
-      } else if (lc == HLBG_LC_BFL) {
-        const T q = (T)a.b_cut[r * (Q - 1) + D - 1];
-        v = (fpost[D] + ((T)2.0 * q - (T)1) * fpost[inv]) / ((T)2.0 * q);
+    const LinkAt<D> link(links);
+    if (active && link.push()) Store<P>::store(t.template at<D, XFACE>(), D * kSites, fpost[D], a);
+    if (P == 0 ? link.bounce() : link.back()) {
+      T v = fpost[D];
+      if constexpr (P != 0 && BFL) {
+        if (!link.bounce()) v = bfl_value(fpost[D], fpost[inv], (T)a.b_cut[r * (Q - 1) + D - 1]);
       }
+      Store<P>::store(t.own, inv * kSites, v, a);
     }
-    if (st) Store<P>::store(p, 0, v, a);
-    PushEachMixed<P, D + 1, XFACE>::run(t, a, active, row_fluid, links, r, fpost);
+    if (zero) Store<P>::store(t.own, D * kSites, (T)0, a);
+    PushEachMixed<P, D + 1, XFACE, BFL>::run(t, a, active, zero, links, r, fpost);
   }
 };
-template <int P, bool XFACE>
-struct PushEachMixed<P, Q, XFACE> {
+template <int P, bool XFACE, bool BFL>
+struct PushEachMixed<P, Q, XFACE, BFL> {
   template <class T>
   static __device__ __forceinline__ void run(const PushTargets<P, true>&, const StepArgs&, bool, bool, uint64_t,
                                              int64_t, const T*) {}
@@ -479,6 +472,10 @@ __device__ __forceinline__ void push_warp(const StepArgs& a, int64_t b, int32_t 
   const bool bnd = code >= 2;
   const bool mixed = __ballot_sync(0xffffffffu, bnd) != 0;
   const int64_t r = bnd ? (int64_t)code - 2 : 0;
+  // A solid slot is never written by a push nor ever read; a zero there completes the
+  // 32-byte sector of slots it shares with fluid slots (sectors without any receive no
+  // write at all and stay untouched).
+  const bool zero = code == 0 && row_fluid;
 #if HLBG_Z_COLUMNS
   if constexpr (!MON || P == 0) {
     if (!mixed) {
@@ -490,8 +487,13 @@ __device__ __forceinline__ void push_warp(const StepArgs& a, int64_t b, int32_t 
     } else {
       const uint64_t links = bnd ? a.b_links[r] : 0ull;
       const PushTargets<P, true> t(fn, b, tabreg, x, y, z, j);
-      if (t.xface) PushEachMixed<P, 0, true>::run(t, a, code != 0, row_fluid, links, r, fpost);
-      else PushEachMixed<P, 0, false>::run(t, a, code != 0, row_fluid, links, r, fpost);
+      if (P != 0 && a.wall == 1) {  // the only walls with interpolated links
+        if (t.xface) PushEachMixed<P, 0, true, true>::run(t, a, code != 0, zero, links, r, fpost);
+        else PushEachMixed<P, 0, false, true>::run(t, a, code != 0, zero, links, r, fpost);
+      } else {
+        if (t.xface) PushEachMixed<P, 0, true, false>::run(t, a, code != 0, zero, links, r, fpost);
+        else PushEachMixed<P, 0, false, false>::run(t, a, code != 0, zero, links, r, fpost);
+      }
       if constexpr (P == 0) {
         if (a.wall == 1) {
           __shared__ BflQueue queue[W];
@@ -508,7 +510,7 @@ __device__ __forceinline__ void push_warp(const StepArgs& a, int64_t b, int32_t 
     PushBulk<P, 0>::run(fn, a, ShflBase{tabreg}, x, y, z, code == 1, fpost);
   } else {
     const uint64_t links = bnd ? a.b_links[r] : 0ull;
-    PushMixed<P, 0>::run(fn, a, ShflBase{tabreg}, x, y, z, j, b * (Q * kSites), code != 0, row_fluid, links, r, fpost);
+    PushMixed<P, 0>::run(fn, a, ShflBase{tabreg}, x, y, z, j, b * (Q * kSites), code != 0, zero, links, r, fpost);
   }
 }
 
