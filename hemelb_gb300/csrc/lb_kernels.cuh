@@ -207,6 +207,23 @@ struct PushAll<P, Q> {
   static __device__ __forceinline__ void run(S*, const StepArgs&, const B&, int, int, int, const T*) {}
 };
 
+// The code of direction D in a boundary record's links, tested bit by bit in place (one
+// logic operation each): 0 push, 1 skip, 2 bounce, 3 BFL, 4 iolet (HLBG_LC_*).
+template <int D>
+struct LinkAt {
+  uint64_t links;
+  __device__ __forceinline__ explicit LinkAt(uint64_t l) : links(l) {}
+  __device__ __forceinline__ bool push() const { return (links & (7ull << (3 * D))) == 0; }
+  __device__ __forceinline__ bool back() const { return (links & (2ull << (3 * D))) != 0; }  // bounce or BFL
+  __device__ __forceinline__ bool bounce() const { return (links & (3ull << (3 * D))) == 2ull << (3 * D); }
+};
+// BFL eq. 5b
+template <class T>
+__device__ __forceinline__ T bfl_value(T out, T back, T q) {
+  return (out + ((T)2.0 * q - (T)1) * back) / ((T)2.0 * q);
+}
+
+#if !HLBG_Z_COLUMNS
 // Pushes of the all-slots kernel: every lane takes part in the shuffles, only
 // bulk sites store.
 template <int P, int D>
@@ -230,22 +247,6 @@ struct PushBulk<P, Q> {
   static __device__ __forceinline__ void run(S*, const StepArgs&, const B&, int, int, int, bool,
                                              const T*) {}
 };
-
-// The code of direction D in a boundary record's links, tested bit by bit in place (one
-// logic operation each): 0 push, 1 skip, 2 bounce, 3 BFL, 4 iolet (HLBG_LC_*).
-template <int D>
-struct LinkAt {
-  uint64_t links;
-  __device__ __forceinline__ explicit LinkAt(uint64_t l) : links(l) {}
-  __device__ __forceinline__ bool push() const { return (links & (7ull << (3 * D))) == 0; }
-  __device__ __forceinline__ bool back() const { return (links & (2ull << (3 * D))) != 0; }  // bounce or BFL
-  __device__ __forceinline__ bool bounce() const { return (links & (3ull << (3 * D))) == 2ull << (3 * D); }
-};
-// BFL eq. 5b
-template <class T>
-__device__ __forceinline__ T bfl_value(T out, T back, T q) {
-  return (out + ((T)2.0 * q - (T)1) * back) / ((T)2.0 * q);
-}
 
 // Pushes of a warp that holds at least one boundary site.  Every lane computes
 // the bulk target (shuffles stay converged); a boundary lane then redirects the
@@ -281,6 +282,7 @@ struct PushMixed<P, Q> {
   static __device__ __forceinline__ void run(S*, const StepArgs&, const B&, int, int, int, int,
                                              int64_t, bool, bool, uint64_t, int64_t, const T*) {}
 };
+#endif
 
 #if HLBG_Z_COLUMNS
 // Where a lane's site pushes to.  A site crosses at most one face per axis, so four
@@ -421,8 +423,9 @@ struct BflEach<Q> {
   static __device__ __forceinline__ void run(BflGather&, uint64_t, int, int64_t, const double*) {}
 };
 
-// Pushes of a warp that holds at least one boundary site: a boundary lane redirects the
-// link by its precomputed code as in PushMixed (FP64: BFL links by BflGather).  A push and
+// Pushes of a warp that holds at least one boundary site: a boundary lane redirects a link
+// by its precomputed code: skip (the reference's rubbish site), bounce-back into its own
+// inverse slot, BFL eq. 5b (FP64: by BflGather), iolet (written by iolet_link).  A push and
 // a value sent back are two stores under two conditions, where one store of a selected
 // value to a selected address took twice the instructions; warps with boundary sites are
 // a third of all and the slowest.  BFL: the walls have interpolated links; without their
@@ -459,12 +462,8 @@ struct PushEachMixed<P, Q, XFACE, BFL> {
 // The pushes of one warp of one block b: this lane's site in slot j, local coordinates
 // x, y, z, post-collision values fpost, code as site_code (0: no site here; a zero goes
 // to its slot where row_fluid).  tabreg: the block's neighbour table in lanes 0..26.
-// Every lane of the warp takes part.  A monitored FP32 or FP16 update keeps the lookup of
-// each push: beside its accumulators the nine pointers cost more in registers than they
-// save (12 steps of a monitored 7.8M-site FP32 tree: 4764 us with the lookups, 4811 with
-// the pointers).
-// W: warps of the CTA.
-template <int P, bool MON, int W, class T>
+// Every lane of the warp takes part.  W: warps of the CTA.
+template <int P, int W, class T>
 __device__ __forceinline__ void push_warp(const StepArgs& a, int64_t b, int32_t tabreg, int x, int y, int z, int j,
                                           uint32_t code, bool row_fluid, const T* fpost) {
   using S = typename Store<P>::S;
@@ -477,41 +476,39 @@ __device__ __forceinline__ void push_warp(const StepArgs& a, int64_t b, int32_t 
   // write at all and stay untouched).
   const bool zero = code == 0 && row_fluid;
 #if HLBG_Z_COLUMNS
-  if constexpr (!MON || P == 0) {
-    if (!mixed) {
-      const PushTargets<P, false> t(fn, b, tabreg, x, y, z, j);
-      if (code == 1) {
-        if (t.xface) PushEach<P, 0, true>::run(t, a, fpost);
-        else PushEach<P, 0, false>::run(t, a, fpost);
-      }
-    } else {
-      const uint64_t links = bnd ? a.b_links[r] : 0ull;
-      const PushTargets<P, true> t(fn, b, tabreg, x, y, z, j);
-      if (P != 0 && a.wall == 1) {  // the only walls with interpolated links
-        if (t.xface) PushEachMixed<P, 0, true, true>::run(t, a, code != 0, zero, links, r, fpost);
-        else PushEachMixed<P, 0, false, true>::run(t, a, code != 0, zero, links, r, fpost);
-      } else {
-        if (t.xface) PushEachMixed<P, 0, true, false>::run(t, a, code != 0, zero, links, r, fpost);
-        else PushEachMixed<P, 0, false, false>::run(t, a, code != 0, zero, links, r, fpost);
-      }
-      if constexpr (P == 0) {
-        if (a.wall == 1) {
-          __shared__ BflQueue queue[W];
-          BflGather g{queue[threadIdx.x >> 5], static_cast<double*>(a.f_new) + b * (Q * kSites), a, 0};
-          BflEach<1>::run(g, links, j, r, fpost);
-          if (g.count) g.eval(0, g.count);
-        }
-      }
+  if (!mixed) {
+    const PushTargets<P, false> t(fn, b, tabreg, x, y, z, j);
+    if (code == 1) {
+      if (t.xface) PushEach<P, 0, true>::run(t, a, fpost);
+      else PushEach<P, 0, false>::run(t, a, fpost);
     }
     return;
   }
-#endif
+  const uint64_t links = bnd ? a.b_links[r] : 0ull;
+  const PushTargets<P, true> t(fn, b, tabreg, x, y, z, j);
+  if (P != 0 && a.wall == 1) {  // the only walls with interpolated links
+    if (t.xface) PushEachMixed<P, 0, true, true>::run(t, a, code != 0, zero, links, r, fpost);
+    else PushEachMixed<P, 0, false, true>::run(t, a, code != 0, zero, links, r, fpost);
+  } else {
+    if (t.xface) PushEachMixed<P, 0, true, false>::run(t, a, code != 0, zero, links, r, fpost);
+    else PushEachMixed<P, 0, false, false>::run(t, a, code != 0, zero, links, r, fpost);
+  }
+  if constexpr (P == 0) {
+    if (a.wall == 1) {
+      __shared__ BflQueue queue[W];
+      BflGather g{queue[threadIdx.x >> 5], static_cast<double*>(a.f_new) + b * (Q * kSites), a, 0};
+      BflEach<1>::run(g, links, j, r, fpost);
+      if (g.count) g.eval(0, g.count);
+    }
+  }
+#else
   if (!mixed) {
     PushBulk<P, 0>::run(fn, a, ShflBase{tabreg}, x, y, z, code == 1, fpost);
   } else {
     const uint64_t links = bnd ? a.b_links[r] : 0ull;
     PushMixed<P, 0>::run(fn, a, ShflBase{tabreg}, x, y, z, j, b * (Q * kSites), code != 0, zero, links, r, fpost);
   }
+#endif
 }
 
 // StabilityTester::PostSendToParent (Code/lb/StabilityTester.h:91-149) and
@@ -999,7 +996,7 @@ __device__ __forceinline__ void collide_slot(const StepArgs& a, int64_t s, MonAc
   if constexpr (MON) {
     if (code != 0) mon_site<P>(a, s, f, m0, mx, my, mz, acc, check, uo);
   }
-  push_warp<P, MON, W>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, row_fluid, fpost);
+  push_warp<P, W>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, row_fluid, fpost);
 }
 
 // One warp of the fluid list: 32 fluid sites of one block (or the zero-fill of its
@@ -1019,7 +1016,7 @@ __device__ __forceinline__ void collide_and_push(const StepArgs& a, int64_t b, i
   if constexpr (MON) {
     if (code != 0) mon_site<P>(a, s, f, m0, mx, my, mz, acc, check, uo);
   }
-  push_warp<P, MON, W>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, false, fpost);
+  push_warp<P, W>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, false, fpost);
 }
 
 // The unit's list entries (block e, this lane's slot js) are loaded by the caller.

@@ -585,8 +585,9 @@ __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamList a
   for (int k = 0; k < 4; ++k) {
     const int64_t i = i0 + k * 256;
     if (i >= n) break;
-    const float mn = b1 * mi[k] + (1.f - b1) * gi[k];
-    const float vn = b2 * vi[k] + (1.f - b2) * gi[k] * gi[k];
+    // fused as the compiler fused them in a kernel of one tensor: the same bits
+    const float mn = __fmaf_rn(1.f - b1, gi[k], b1 * mi[k]);
+    const float vn = __fmaf_rn((1.f - b2) * gi[k], gi[k], b2 * vi[k]);
     m[i] = mn;
     v[i] = vn;
     const float wn = wi[k] - lr * (mn * c1) / (sqrtf(vn * c2) + eps);
