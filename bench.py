@@ -340,9 +340,8 @@ def main():
     per_launch = kms / args.steps
     peak, peak_kind = measured_peak()
     achieved = B_ALG[prec] * n / (per_launch / 1e3) / 1e9
-    if prec == 0:  # FP64 runs two CTAs per SM in every shape, the fluid list from index 4 up
-        kname = ("k_stream_collide_listed<0, %d, 2>" % (64 if variant == 7 else 128)) if variant >= 4 \
-            else "k_stream_collide<0, 128, 2>"
+    if prec == 0:  # FP64: one shape for all slots, one-warp CTAs for the fluid list
+        kname = "k_stream_collide_listed<0, 32, 16>" if variant >= 4 else "k_stream_collide<0, 128, 2>"
     else:
         kname = KERNEL_OF_VARIANT.get(variant, "k_stream_collide").replace("<P", "<%d" % prec)
         kname = kname.replace(", S>", ", %d>" % (4 if prec == 1 else 8))
