@@ -41,13 +41,16 @@ const int HCY[19] = {0, 0, 0, 1, -1, 0, 0, 1, -1, -1, 1, 0, 0, 0, 0, 1, -1, 1, -
 const int HCZ[19] = {0, 0, 0, 0, 0, 1, -1, 0, 0, 0, 0, 1, -1, -1, 1, 1, -1, -1, 1};
 const int HINV[19] = {0, 2, 1, 4, 3, 6, 5, 8, 7, 10, 9, 12, 11, 14, 13, 16, 15, 18, 17};
 
-// Fluid list order within a block: its sites in slot order (HLBG_LIST_SPLIT=0);
-// its bulk sites first and then its boundary sites (1), which keeps most warps on
-// the bulk push path but leaves gaps in each warp's slots; or whole 8-site rows,
-// those without a boundary site first (2).  Measured on the vascular forest: 1 is
-// +4% to +9% for FP16 storage (instruction-bound) and -7% for FP32 deviations
-// (bandwidth-bound); 2 is +/-0 for FP32 and +8% for FP16.  The default (-1) is 1
-// for FP16 and 0 otherwise.
+// Fluid list order within a block: its sites in slot order (HLBG_LIST_SPLIT=0); its bulk
+// sites first and then its boundary sites (1), which keeps most warps on the bulk push
+// path but leaves gaps in each warp's slots; whole 8-site rows, those without a boundary
+// site first (2); or aligned groups of 32 slots that hold fluid (3), whose solid lanes
+// zero their slots, so that every warp reads and writes whole sectors of one 128-byte line
+// a direction and no warp is spent on zeros alone.  The default (-1): FP64, bound by its
+// arithmetic, takes 0, which has the fewest warps.  FP32 takes 3 (us a step against 0, at
+// 128 x 9: tree of 16.9M sites 512 / 569, of 7.8M 264 / 311, ensemble of 4.9M 171 / 179,
+// bifurcation of 1.5M 64.7 / 65.5; all slots 538, 282, 185, 67.9).  FP16 takes 1 (tree of
+// 7.8M 229 against 248 with 0 and 254 in all slots).
 #ifndef HLBG_LIST_SPLIT
 #define HLBG_LIST_SPLIT -1
 #endif
@@ -795,7 +798,7 @@ int build_layout(hlbg_ctx* ctx, const hlbg_geometry* g) {
       }
       tmp.clear();
     };
-    const int split = HLBG_LIST_SPLIT < 0 ? (ctx->prec == HLBG_FP16 ? 1 : 0) : HLBG_LIST_SPLIT;
+    const int split = HLBG_LIST_SPLIT < 0 ? (ctx->prec == HLBG_FP16 ? 1 : (ctx->prec == HLBG_FP64 ? 0 : 3)) : HLBG_LIST_SPLIT;
     // pipelined launch, per block: its first list warp (bits 0-31), the span of
     // rows from its first fluid row to its last (32-37: first, 38-44: end), its
     // fluid warps (45-50) and zero-fill warps (51-56)
@@ -810,7 +813,21 @@ int build_layout(hlbg_ctx* ctx, const hlbg_geometry* g) {
             rowe = row + 1;
           }
       if (rowe == 0) row0 = 0;
-      if (split == 1) {
+      if (split == 3) {
+        // aligned groups of 32 slots, each a warp of its own, where they hold fluid
+        for (int j0 = 0; j0 < 512; j0 += 32) {
+          bool any = false;
+          for (int j = j0; j < j0 + 32; ++j) any |= code[b * 512 + j] != 0;
+          if (!any) continue;
+          for (int j = j0; j < j0 + 32; ++j) {
+            const uint32_t c = code[b * 512 + j];
+            bool row = false;
+            for (int t = j & ~7; t < (j & ~7) + 8; ++t) row |= code[b * 512 + t] != 0;
+            tmp.push_back(c ? (uint16_t)(j | (c >= 2 ? kListBoundary : 0u))
+                            : (row ? (uint16_t)(j | kListSolid) : (uint16_t)0xffff));
+          }
+        }
+      } else if (split == 1) {
         // bulk sites first, then the boundary sites, so that most warps take the
         // bulk push path and only the warps holding boundary sites the mixed one
         for (int j = 0; j < 512; ++j)
@@ -836,7 +853,7 @@ int build_layout(hlbg_ctx* ctx, const hlbg_geometry* g) {
       }
       flush(b, false);
       const uint64_t nfw = wb.size() - first;
-      for (int sec = 0; sec < 64; ++sec) {
+      for (int sec = 0; sec < 64 && split != 3; ++sec) {
         bool any = false;
         for (int t = 0; t < 8; ++t) any |= code[b * 512 + sec * 8 + t] != 0;
         if (!any) continue;
@@ -1077,11 +1094,12 @@ int graph_steps(hlbg_ctx* ctx, int n, bool check) {
 
 namespace {
 
-// Launch shape of a new context: the fluid list, whose warps hold fluid sites only.
-// All slots (index 0) was the default before: on the 1.46M-site bifurcation, where 38 %
-// of the slots are solid, FP64 takes 670 us a step against 786, FP32 63 against 75.
-// FP16 takes 128 x 9 (its list keeps bulk and boundary sites apart).
-int default_variant(int prec) { return prec == HLBG_FP16 ? 5 : 6; }
+// Launch shape of a new context: the fluid list, which passes over what is solid.  FP64
+// (one shape of it): 670 us a step on the 1.46M-site bifurcation against 786 in all slots.
+// FP32 and FP16: 128 x 9, the fastest of the list's shapes on every vessel tried with the
+// orders above (FP32 tree of 16.9M sites 512, 128 x 8 528, 64 x 16 525; bifurcation 64.7,
+// 68.1, 67.7; FP16 tree of 7.8M 229, 236, 233).
+int default_variant(int prec) { return prec == HLBG_FP64 ? 6 : 5; }
 
 // Iolet parameters of a context: the models must match the streamers (Nash reads
 // a density, Ladd a velocity), and the warm-up start density is the smallest iolet

@@ -86,6 +86,9 @@ struct IoletDev {
 constexpr int32_t kPackedBit = 1 << 30;
 // Flag of a fluid-list entry whose site has a boundary record (site_code >= 2).
 constexpr unsigned kListBoundary = 1u << 14;
+// Flag of a solid slot in a fluid warp of the list, whose row of 8 slots holds fluid: its
+// lane writes zeros there.
+constexpr unsigned kListSolid = 1u << 13;
 // HLBG_PACK=1 builds the packed layout (fluid sites of partly fluid blocks in the
 // first slots; with HLBG_PACK_FILL=p only the blocks whose fluid fills less than
 // p % of the z-rows it touches).  It moves 5-12% fewer bytes but the packed code
@@ -180,7 +183,7 @@ struct StepArgs {
   int32_t mon_steady;  // count this check for steady-state detection
   // Fluid-list launch: warp w works on block warp_block[w] & 0x7fffffff, lane k on
   // its slot lane_slot[32 w + k] & 511 (0xffff: idle; kListBoundary set for a site
-  // with a boundary record); a negative warp_block marks a warp that only writes
+  // with a boundary record, kListSolid for a solid slot); a negative warp_block marks a warp that only writes
   // zeros into the solid slots sharing a 32-byte sector with fluid.
   const int32_t* warp_block;
   const uint16_t* lane_slot;

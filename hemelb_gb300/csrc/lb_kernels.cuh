@@ -1007,7 +1007,7 @@ __device__ __forceinline__ void collide_slot(const StepArgs& a, int64_t s, MonAc
 // 0..26.  Every lane of the warp must take part (shuffles, ballot).
 template <int P, bool MON, int W>
 __device__ __forceinline__ void collide_and_push(const StepArgs& a, int64_t b, int j, int64_t s, int l,
-                                                 uint32_t code, int32_t tabreg, typename Calc<P>::T* f,
+                                                 uint32_t code, bool zero, int32_t tabreg, typename Calc<P>::T* f,
                                                  MonAccT<P>& acc, bool check, const MonOld<P>& uo) {
   using T = typename Calc<P>::T;
   T fpost[Q];
@@ -1016,7 +1016,7 @@ __device__ __forceinline__ void collide_and_push(const StepArgs& a, int64_t b, i
   if constexpr (MON) {
     if (code != 0) mon_site<P>(a, s, f, m0, mx, my, mz, acc, check, uo);
   }
-  push_warp<P, W>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, false, fpost);
+  push_warp<P, W>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, zero, fpost);
 }
 
 // The unit's list entries (block e, this lane's slot js) are loaded by the caller.
@@ -1028,13 +1028,13 @@ __device__ __forceinline__ void collide_listed_unit(const StepArgs& a, int32_t e
   using T = typename Calc<P>::T;
   const int lane = threadIdx.x & 31;
   const int64_t b = e & 0x7fffffff;
-  const bool on = js != 0xffffu;
-  const int j = on ? (int)(js & (kSites - 1)) : 0;
+  const bool idle = js == 0xffffu, on = !idle && !(js & kListSolid);
+  const int j = idle ? 0 : (int)(js & (kSites - 1));
   const int64_t s = b * kSites + j;
   S* fn = static_cast<S*>(a.f_new);
   if (e < 0) {  // zero-fill warp: complete the sectors its slots share with fluid
     wait_for_previous();
-    if (on) {
+    if (!idle) {
 #pragma unroll
       for (int d = 0; d < Q; ++d) St::store(fn, fidx(s, d), (T)0, a);
     }
@@ -1042,11 +1042,11 @@ __device__ __forceinline__ void collide_listed_unit(const StepArgs& a, int32_t e
   }
   const int32_t* tab = a.block_nbr + b * 27;
   const int32_t tabreg = lane < 27 ? __ldg(tab + lane) : 0;
-  // every listed lane is a fluid site: its loads need not wait for its code, and
-  // only the boundary sites (flagged in the list) read one
+  // a lane knows from the list whether its slot is fluid: its loads need not wait for
+  // its code, and only the boundary sites (flagged in the list) read one
   const uint32_t code = on ? ((js & kListBoundary) ? a.site_code[s] : 1u) : 0u;
   const bool packed = (__shfl_sync(0xffffffffu, tabreg, 13) & kPackedBit) != 0;
-  const int l = on ? site_of_slot(a, s, packed) : 0;
+  const int l = idle ? 0 : site_of_slot(a, s, packed);
   const S* fo = static_cast<const S*>(a.f_old) + b * (Q * kSites) + j;
   wait_for_previous();
   MonOld<P> uo;
@@ -1060,7 +1060,7 @@ __device__ __forceinline__ void collide_listed_unit(const StepArgs& a, int32_t e
 #pragma unroll
     for (int i = 0; i < Q; ++i) f[i] = (T)(P == 0 ? weight_d(i) : 0.0);
   }
-  collide_and_push<P, MON, W>(a, b, j, s, l, code, tabreg, f, acc, check, uo);
+  collide_and_push<P, MON, W>(a, b, j, s, l, code, !idle && !on, tabreg, f, acc, check, uo);
 }
 
 template <int P, bool MON, int W>
@@ -1212,7 +1212,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_stream_collide_block(StepArgs
       else
         f[d] = on ? __half2float(stage[d * kSites + j]) * a.fp16_inv_scale : 0.f;
     }
-    collide_and_push<P, false, 1>(a, b, j, s, j, code, tabreg, f, acc, false, uo);
+    collide_and_push<P, false, 1>(a, b, j, s, j, code, false, tabreg, f, acc, false, uo);
   }
   // solid slots of the rows that hold fluid: zeros complete their sectors
   S* fn = static_cast<S*>(a.f_new);
@@ -1386,11 +1386,11 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) k_stream_collide_pipe(StepA
     const int32_t tabreg = lane < 27 && first < nfw ? __ldg(a.block_nbr + b * 27 + lane) : 0;
     for (int task = first; task < ntask; task += NCW) {  // warp-uniform trips
       const unsigned js = list[task * 32 + lane];
-      const bool on = js != 0xffffu;
-      const int j = on ? (int)(js & (kSites - 1)) : 0;
+      const bool idle = js == 0xffffu, on = !idle && !(js & kListSolid);
+      const int j = idle ? 0 : (int)(js & (kSites - 1));
       const int64_t s = b * kSites + j;
       if (task >= nfw) {  // zero-fill warp: complete the sectors its slots share with fluid
-        if (on) {
+        if (!idle) {
 #pragma unroll
           for (int d = 0; d < Q; ++d) Store<P>::store(fn, fidx(s, d), (T)0, a);
         }
@@ -1405,7 +1405,7 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) k_stream_collide_pipe(StepA
         else
           f[d] = on ? __half2float(stage[d * kSites + j]) * a.fp16_inv_scale : 0.f;
       }
-      collide_and_push<P, false, 1>(a, b, j, s, j, code, tabreg, f, acc, false, uo);
+      collide_and_push<P, false, 1>(a, b, j, s, j, code, !idle && !on, tabreg, f, acc, false, uo);
     }
     rot = (rot + ntask) % NCW;
     __syncwarp();
