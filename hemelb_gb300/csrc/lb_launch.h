@@ -11,7 +11,7 @@ struct StepArgs;
 
 // Launch variants of the stream-and-collide kernel (FP64: all slots for 0-3, the fluid
 // list with one warp per CTA from 4 up):
-// 0 default shape, 1: 128x8, 2: 256x4, 3: 512x2 threads x resident CTAs per SM,
+// 0: 128x10, 1: 128x8, 2: 256x4, 3: 512x2 threads x resident CTAs per SM,
 // 4: one CTA per block, staged by bulk copies; 5, 6, 7: the fluid-list launch;
 // 8: persistent, pipelined block staging (FP32 / FP16).
 constexpr int kSCVariants = 9;
