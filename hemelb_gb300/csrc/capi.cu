@@ -946,7 +946,6 @@ int build_layout(hlbg_ctx* ctx, const hlbg_geometry* g) {
 
 constexpr int kMonFields = 7;  // partials: mass, max |du|, min f, unstable, min rho, max rho, max |u|
 constexpr int kMonResult = 8;  // the same plus the valid flag
-constexpr int64_t kMonGroupCtas = 64;  // CTAs per group of the reduction (mon_finish)
 
 // Buffers of the fused StabilityTester, allocated on first use.
 int mon_prepare(hlbg_ctx* ctx) {
@@ -959,11 +958,10 @@ int mon_prepare(hlbg_ctx* ctx) {
   // one partial per CTA, for every launch shape: all slots in CTAs of 128 or more
   // threads, or the fluid list (FP64: one warp per CTA, else four)
   const int64_t max_ctas = std::max((ctx->nslot + 127) / 128, ctx->prec == 0 ? ctx->n_warps : (ctx->n_warps + 3) / 4);
-  const int64_t max_groups = (max_ctas + kMonGroupCtas - 1) / kMonGroupCtas;
   if ((rc = dev_alloc(ctx, &ctx->d_mon_part, kMonFields * (size_t)max_ctas))) return rc;
-  if ((rc = dev_alloc(ctx, &ctx->d_mon_part2, kMonFields * (size_t)max_groups))) return rc;
-  if ((rc = dev_alloc(ctx, &ctx->d_mon_tick, (size_t)max_groups + 1))) return rc;
-  CK(cudaMemsetAsync(ctx->d_mon_tick, 0, ((size_t)max_groups + 1) * sizeof(uint32_t), ctx->stream));
+  if ((rc = dev_alloc(ctx, &ctx->d_mon_part2, kMonFields * (size_t)((max_ctas + kMonFold - 1) / kMonFold)))) return rc;
+  if ((rc = dev_alloc(ctx, &ctx->d_mon_tick, 1))) return rc;
+  CK(cudaMemsetAsync(ctx->d_mon_tick, 0, sizeof(uint32_t), ctx->stream));
   if ((rc = dev_alloc(ctx, &ctx->d_mon_state, 1))) return rc;
   if ((rc = dev_alloc(ctx, &ctx->d_mon_result, kMonResult))) return rc;
   CK(cudaMemsetAsync(ctx->d_mon_result, 0, kMonResult * sizeof(double), ctx->stream));  // no check yet

@@ -167,10 +167,10 @@ struct StepArgs {
   const uint16_t* site2slot;  // [nslot] slot of each local site (packed blocks)
   // Fused StabilityTester (monitored steps only): each site's velocity at its last
   // update, u[(block * 3 + c) * 512 + slot] (double for FP64, float otherwise); the
-  // per-CTA partials (mon_finish, stride mon_nparts), those of groups of CTAs, and the
-  // arrival counters (groups arrived, then CTAs arrived per group; zero between
-  // launches); mon_state 0 while no velocity has been recorded since the state was
-  // set.  mon_fold 0: record the velocities only.
+  // per-CTA partials (mon_partial, stride mon_nparts), those of k_mon_fold's CTAs, and
+  // the counter of the CTAs that have arrived (zero between launches); mon_state 0 while
+  // no velocity has been recorded since the state was set.  mon_fold 0: record the
+  // velocities only.
   void* mon_u;
   double* mon_part;
   int64_t mon_nparts;
@@ -180,6 +180,7 @@ struct StepArgs {
   double* mon_result;
   SteadyArgs steady;
   int32_t mon_fold;
+  int32_t mon_apart;   // the partials are folded by a launch of their own
   int32_t mon_steady;  // count this check for steady-state detection
   // Fluid-list launch: warp w works on block warp_block[w] & 0x7fffffff, lane k on
   // its slot lane_slot[32 w + k] & 511 (0xffff: idle; kListBoundary set for a site

@@ -786,24 +786,10 @@ __device__ __forceinline__ MonAcc mon_load_cta(const StepArgs& a, int64_t i) {
   }
 }
 
-// End of a monitored CTA: its partial, and the reduction of all of them in the same
-// launch.  The CTAs form groups of kMonGroup; the last CTA of a group to arrive folds
-// the group's partials in index order, and the last group's folds the groups' -- a
-// fixed tree, so the result does not depend on the order of arrival -- and writes the
-// result [mass, max |du|, min f, unstable, valid, min rho, max rho, max |u|], where
-// valid is 0 for the first step after the state was set (it only recorded
-// velocities).  With mon_steady a valid check is also counted for steady-state
-// detection.  Every step then marks the recorded velocities as present.  As two
-// launches after the update this took 19 + 10 us beside 59 us of a 34k-site FP64
-// step (seven FP64 comparisons and additions per shuffle level in every thread); the
-// whole monitored step is 32 us now.
-constexpr int kMonGroup = 64;
+// A monitored CTA's partial.
 template <int P>
-__device__ __forceinline__ void mon_finish(const StepArgs& a, const MonAccT<P>& acc, unsigned cta) {
+__device__ __forceinline__ void mon_partial(const StepArgs& a, const MonAccT<P>& acc, unsigned cta) {
   const int64_t n = a.mon_nparts;
-  const unsigned groups = (unsigned)((n + kMonGroup - 1) / kMonGroup), g = cta / kMonGroup;
-  const int lane = threadIdx.x & 31;
-  int last = 0;
   wait_for_previous();  // its last CTAs may still read the partials
   if constexpr (P == 0) {
     const MonAcc r = mon_block(acc);
@@ -822,35 +808,15 @@ __device__ __forceinline__ void mon_finish(const StepArgs& a, const MonAccT<P>& 
       p[7 * n + cta] = __uint_as_float(r.bad);
     }
   }
-  if (threadIdx.x >= 32) return;
-  if (lane == 0) {
-    const unsigned size = (unsigned)(n - (int64_t)g * kMonGroup < kMonGroup ? n - (int64_t)g * kMonGroup : kMonGroup);
-    __threadfence();
-    last = atomicAdd(a.mon_tick + 1 + g, 1u) == size - 1;
-  }
-  if (!__shfl_sync(0xffffffffu, last, 0)) return;
-  __threadfence();
-  MonAcc v = mon_neutral();
-#pragma unroll
-  for (int k = 0; k < kMonGroup; k += 32) {
-    const int64_t i = (int64_t)g * kMonGroup + k + lane;
-    if (i < n) mon_combine(v, mon_load_cta<P>(a, i));
-  }
-  v = mon_warp(v);
-  if (lane == 0) {
-    mon_store(a.mon_part2, groups, g, v);
-    a.mon_tick[1 + g] = 0;
-    __threadfence();
-    last = atomicAdd(a.mon_tick, 1u) == groups - 1;
-  }
-  if (!__shfl_sync(0xffffffffu, last, 0)) return;
-  __threadfence();
-  v = mon_neutral();
-#pragma unroll 4
-  for (unsigned i = lane; i < groups; i += 32) mon_combine(v, mon_load(a.mon_part2, groups, i));
-  v = mon_warp(v);
-  if (lane != 0) return;
-  a.mon_tick[0] = 0;
+}
+
+// The step's result from the reduction of all partials (one thread): [mass, max |du|,
+// min f, unstable, valid, min rho, max rho, max |u|], where valid is 0 for the first
+// step after the state was set (it only recorded velocities).  With mon_steady a valid
+// check is also counted for steady-state detection.  Every step then marks the recorded
+// velocities as present.
+template <int P>
+__device__ __forceinline__ void mon_result(const StepArgs& a, const MonAcc& v) {
   const int valid = *a.mon_state != 0;
   double du = __longlong_as_double((long long)v.maxdu), um = __longlong_as_double((long long)v.umax);
   if constexpr (P == 0) {
@@ -874,6 +840,75 @@ __device__ __forceinline__ void mon_finish(const StepArgs& a, const MonAccT<P>& 
     if (du <= *a.steady.threshold && a.steady.counters[1] < 0) a.steady.counters[1] = k;
   }
   *a.mon_state = 1;
+}
+
+// The partials of a monitored update are folded by its last CTA to arrive (mon_finish),
+// or, from kMonFold CTAs on, by a launch of their own behind it (k_mon_fold).  Either
+// tree is fixed, so the result does not depend on the order of arrival.  In the launch
+// every CTA waits for its stores to reach L2 before it counts itself in, and holds its
+// registers meanwhile; a launch costs a call of one small step 1 us of host time.  Fold in
+// the launch against fold behind it, 128 x 8 list, us a checked step: FP32 forest of 223M
+// sites 9664 / 8704, tree of 16.9M 750 / 680, ensemble of 4.9M 249 / 228, pipe of 25k (250
+// CTAs) 10.1 / 9.2 in calls of many steps and 27.1 / 27.9 in calls of one; FP16 forest
+// 9114 / 7881; FP64 pipe (1,000 one-warp CTAs) 24.6 / 23.9 and 41.7 / 40.8.
+template <int P>
+__device__ __forceinline__ void mon_finish(const StepArgs& a, const MonAccT<P>& acc, unsigned cta) {
+  mon_partial<P>(a, acc, cta);
+  if (a.mon_apart || threadIdx.x >= 32) return;
+  const int64_t n = a.mon_nparts;
+  const int lane = threadIdx.x & 31;
+  int last = 0;
+  if (lane == 0) {
+    __threadfence();
+    last = atomicAdd(a.mon_tick, 1u) == (unsigned)n - 1;
+  }
+  if (!__shfl_sync(0xffffffffu, last, 0)) return;
+  __threadfence();
+  MonAcc v = mon_neutral();
+#pragma unroll 4
+  for (int64_t i = lane; i < n; i += 32) mon_combine(v, mon_load_cta<P>(a, i));
+  v = mon_warp(v);
+  if (lane != 0) return;
+  *a.mon_tick = 0;
+  mon_result<P>(a, v);
+}
+
+// A CTA folds kMonFold of the update's partials, the last one to arrive the CTAs'.
+constexpr int kMonFoldThreads = 256;
+template <int P>
+__global__ void __launch_bounds__(kMonFoldThreads) k_mon_fold(StepArgs a) {
+  __shared__ int last;
+  let_next_in();
+  wait_for_previous();
+  const int64_t n = a.mon_nparts;
+  MonAcc v = mon_neutral();
+#pragma unroll
+  for (int k = 0; k < kMonFold; k += kMonFoldThreads) {
+    const int64_t i = (int64_t)blockIdx.x * kMonFold + k + threadIdx.x;
+    if (i < n) mon_combine(v, mon_load_cta<P>(a, i));
+  }
+  v = mon_block(v);
+  if (threadIdx.x == 0) {
+    mon_store(a.mon_part2, gridDim.x, blockIdx.x, v);
+    __threadfence();
+    last = atomicAdd(a.mon_tick, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  v = mon_neutral();
+#pragma unroll 4
+  for (unsigned i = threadIdx.x; i < gridDim.x; i += kMonFoldThreads) mon_combine(v, mon_load(a.mon_part2, gridDim.x, i));
+  v = mon_block(v);
+  if (threadIdx.x == 0) {
+    *a.mon_tick = 0;
+    mon_result<P>(a, v);
+  }
+}
+
+template <int P>
+void launch_mon_fold(const StepArgs& a, cudaStream_t st) {
+  launch_overlapped(k_mon_fold<P>, (unsigned)((a.mon_nparts + kMonFold - 1) / kMonFold), kMonFoldThreads, 0, st, a);
 }
 
 // ---------------------------------------------------------------------------
@@ -1456,7 +1491,9 @@ void launch_listed(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
   StepArgs b = a;
   b.io_ctas = (uint32_t)((a.n_io_links + THREADS - 1) / THREADS);
   b.let_in = g >= 4 * 152 * MINB;
+  b.mon_apart = MON && a.mon_fold && g >= kMonFold;
   if (g) launch_overlapped(k_stream_collide_listed<P, THREADS, MINB, MON>, (unsigned)g + b.io_ctas, THREADS, 0, st, b, bxyz);
+  if (b.mon_apart) launch_mon_fold<P>(b, st);
 }
 
 template <int P>
@@ -1933,7 +1970,9 @@ void launch_sc(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
   StepArgs b = a;
   b.io_ctas = (uint32_t)((a.n_io_links + THREADS - 1) / THREADS);
   b.let_in = g >= 4 * 152 * MINB;
+  b.mon_apart = MON && a.mon_fold && g >= kMonFold;
   if (g) launch_overlapped(k_stream_collide<P, THREADS, MINB, MON>, g + b.io_ctas, THREADS, 0, st, b, bxyz);
+  if (b.mon_apart) launch_mon_fold<P>(b, st);
 }
 }  // namespace hlbg
 

@@ -16,6 +16,10 @@ struct StepArgs;
 // 8: persistent, pipelined block staging (FP32 / FP16).
 constexpr int kSCVariants = 9;
 
+// Partials of a monitored step one CTA of k_mon_fold folds; a launch of fewer CTAs folds
+// its own.
+constexpr int kMonFold = 512;
+
 struct PostArgs {
   void* f_new;
   int64_t stride;
