@@ -874,11 +874,27 @@ inline bool relu_bias(void* dy, const void* y, float* db, int64_t m, int32_t c, 
 
 inline unsigned blocks(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
 
+// Modelled microseconds of k_wgrad_brick, bpc bricks a CTA, for nbricks bricks of `shares`
+// channel blocks (as wgrad_tc_time): rounds of two CTAs an SM, which slow each other down,
+// and the additions to dw by their number and by the CTAs that meet at an address.
+inline double wgrad_mma_time(int cin, int cout, int nci, int64_t bpc, int64_t nbricks, int shares) {
+  const double gx = (double)((nbricks + bpc - 1) / bpc), ctas = gx * shares, per = ctas / 304.0;
+  const double rounds = per > 2 ? per : std::max(1.0, std::ceil(per)), resident = std::min(2.0, std::max(1.0, ctas / 152.0));
+  const double chain = rounds * ((double)bpc * (nci == 2 ? 1.5 : 0.93) * (1 + 2.4 * (resident - 1)) + (nci == 2 ? 1.5 : 0.2));
+  const double adds = gx * 27e-6 * cin * cout * 2.0, meet = 0.061 * gx;
+  return 3.5 + std::sqrt(std::sqrt(chain * chain * chain * chain + adds * adds * adds * adds + meet * meet * meet * meet));
+}
+
 int check_launch() { return cudaGetLastError() == cudaSuccess ? 0 : 3; }
 
 }  // namespace
 
 extern "C" {
+
+// hlbg_nn_conv3d_wgrad_tc where its modelled time is within `limit` microseconds
+// (nn_tc.cu; 1x1x1 has no model), else 1.
+int hlbg_nn_wgrad_tc_within(const void* x, int32_t cin, const void* dy, int32_t cout, float* dw, int32_t n, int32_t d,
+                            int32_t h, int32_t wd, int32_t taps, void* stream, double limit);
 
 int hlbg_nn_conv3d(const void* in, int32_t cin, const void* w, const float* bias, void* out, float* out_f32,
                    int32_t cout, int32_t n, int32_t d, int32_t h, int32_t wd, int32_t taps, int32_t relu,
@@ -922,21 +938,23 @@ int hlbg_nn_conv3d(const void* in, int32_t cin, const void* w, const float* bias
 int hlbg_nn_conv3d_wgrad(const void* x, int32_t cin, const void* dy, int32_t cout, float* dw, int32_t n,
                          int32_t d, int32_t h, int32_t wd, int32_t taps, void* stream) {
   if (!x || !dy || !dw || cin % 8 || cout <= 0) return 1;
-  // the tcgen05 kernel where it takes the shape, but for one block of 16 x 16 channels of a
-  // few thousand voxels, where its set-up is longer than the work (6^3: 9.9 us against 9.2)
-  if (cin % 16 == 0 && cout % 16 == 0 && aligned16(x, dy, dw) &&
-      (taps == 1 || cin * cout > 256 || (int64_t)n * d * h * wd >= 4096)) {
-    const int rc = hlbg_nn_conv3d_wgrad_tc(x, cin, dy, cout, dw, n, d, h, wd, taps, stream);
+  const bool by16 = cin % 16 == 0 && cout % 16 == 0;
+  const int nbz = (d + kBZ - 1) / kBZ, nby = (h + kBY - 1) / kBY, nbx = (wd + kBX - 1) / kBX;
+  const int64_t nbricks = (int64_t)n * nbz * nby * nbx;
+  const int nci = cin % 32 == 0 ? 2 : 1;
+  const int gy = cout / 16, gz = cin / (16 * nci);
+  // about four waves of 2 CTAs per SM over 152 SMs
+  const int64_t bpc = std::max<int64_t>(1, (nbricks * gy * gz + 1215) / 1216);
+  // The tcgen05 kernel where it is the faster one.  1x1x1: from 17 voxels on (us, mma.sync /
+  // tcgen05, 96 -> 96: 8 voxels 2.7 / 3.5, 27 5.2 / 3.5, 4096 440 / 4).  3x3x3: by the
+  // modelled times (96 -> 96: 96 x 3 x 3 voxels 17.0 / 25.0, 24^3 42 / 16).
+  const int64_t M = (int64_t)n * d * h * wd;
+  if (by16 && aligned16(x, dy, dw) && (taps == 27 || M > 16)) {
+    const double limit = taps == 27 ? wgrad_mma_time(cin, cout, nci, bpc, nbricks, gy * gz) : 0.0;
+    const int rc = hlbg_nn_wgrad_tc_within(x, cin, dy, cout, dw, n, d, h, wd, taps, stream, limit);
     if (rc != 1) return rc;
   }
-  if (taps == 27 && cin % 16 == 0 && cout % 16 == 0) {
-    const int nbz = (d + kBZ - 1) / kBZ, nby = (h + kBY - 1) / kBY, nbx = (wd + kBX - 1) / kBX;
-    const int64_t nbricks = (int64_t)n * nbz * nby * nbx;
-    const int nci = cin % 32 == 0 ? 2 : 1;
-    const int gy = cout / 16, gz = cin / (16 * nci);
-    // about four waves of 2 CTAs per SM over 152 SMs
-    int64_t bpc = (nbricks * gy * gz + 1215) / 1216;
-    if (bpc < 1) bpc = 1;
+  if (taps == 27 && by16) {
     dim3 grid((unsigned)((nbricks + bpc - 1) / bpc), (unsigned)gy, (unsigned)gz);
     auto X = (const __nv_bfloat16*)x;
     auto DY = (const __nv_bfloat16*)dy;
@@ -948,7 +966,6 @@ int hlbg_nn_conv3d_wgrad(const void* x, int32_t cin, const void* dy, int32_t cou
                                                                 nbricks, (int)bpc);
     return check_launch();
   }
-  const int64_t M = (int64_t)n * d * h * wd;
   const int64_t ntile = (int64_t)taps * ((cout + 15) / 16) * (cin / 8);
   const int64_t slice = 4096;
   dim3 grid((unsigned)((ntile + 3) / 4), (unsigned)((M + slice - 1) / slice));

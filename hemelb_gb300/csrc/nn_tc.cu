@@ -814,7 +814,14 @@ int hlbg_nn_conv3d_tc(const void* in, int32_t cin, const void* w, const float* b
 
 int hlbg_nn_conv3d_wgrad_tc(const void* x, int32_t cin, const void* dy, int32_t cout, float* dw, int32_t n, int32_t d,
                             int32_t h, int32_t wd, int32_t taps, void* stream) {
-  return wgrad_tc(x, cin, dy, cout, dw, n, d, h, wd, taps, static_cast<cudaStream_t>(stream));
+  return wgrad_tc(x, cin, dy, cout, dw, n, d, h, wd, taps, static_cast<cudaStream_t>(stream), INFINITY);
+}
+
+// (nn_kernels.cu)
+__attribute__((visibility("hidden"))) int hlbg_nn_wgrad_tc_within(const void* x, int32_t cin, const void* dy, int32_t cout,
+                                                                  float* dw, int32_t n, int32_t d, int32_t h, int32_t wd,
+                                                                  int32_t taps, void* stream, double limit) {
+  return wgrad_tc(x, cin, dy, cout, dw, n, d, h, wd, taps, static_cast<cudaStream_t>(stream), limit);
 }
 
 int hlbg_nn_tc_error(int32_t reset) {

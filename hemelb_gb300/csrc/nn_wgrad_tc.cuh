@@ -405,8 +405,30 @@ auto wg_kernel(int wb, int zg, int taps) {
   return wb == 16 ? wg_kernel<WA, 16>(zg, taps) : (wb == 32 ? wg_kernel<WA, 32>(zg, taps) : wg_kernel<WA, 64>(zg, taps));
 }
 
+// Modelled microseconds of a 3x3x3 gradient.  A CTA's units follow each other: a unit's
+// MMAs (issued one every 0.0394 us, or the SM's pipe shared by its CTAs) and its epilogue
+// (0.145 us a chunk of 16 columns), the two side by side where there are two sets.  The
+// additions to dw bound it from below where runs are short, by their number (those of dy's
+// rows, 16 bytes at a stride, cost twice those of x's) and by the runs that meet at an
+// address; a volume a few voxels wide or high is mostly padding of the 8 x 16 tiles, so
+// that its runs are many for what they add.  A 4-norm of the three over the launch's 2.77.
+// A fit to 742 shapes, 10 % in the mean; so is wgrad_mma_time's.  Of the two kernels the
+// faster one is chosen, or one within 5 %, for all but 25 of 754 other shapes (42 % at worst).
+double wgrad_tc_time(const WgPlan& pl, const WgParams& p, int64_t units, int64_t ctas) {
+  const double per_cta = (double)((units + ctas - 1) / ctas);
+  const double resident = std::min((double)pl.per_sm, std::max(1.0, (double)units / kSms));
+  const int n = 3 * pl.wb, sums = pl.zg * pl.groups;
+  const double mma = p.run * sums * 8.0 * std::max(0.0394, 0.00072 * mma_cost(n) * resident);
+  const double epi = 0.145 * (sums * n / 16);
+  const double chain = pl.sets == 2 && per_cta > 1 ? per_cta * std::max(mma, epi) + std::min(mma, epi)
+                                                   : per_cta * (mma + epi);
+  const double adds = p.runs * 27e-6 * p.Cin * p.Cout * (pl.a_is_dy ? 1.77 : 0.83), meet = 0.030 * p.runs;
+  return 2.77 + std::sqrt(std::sqrt(chain * chain * chain * chain + adds * adds * adds * adds + meet * meet * meet * meet));
+}
+
+// `limit`: modelled time (us) above which the shape is not taken (3x3x3).
 int wgrad_tc(const void* x, int cin, const void* dy, int cout, float* dw, int n, int d, int h, int wd, int taps,
-             cudaStream_t st) {
+             cudaStream_t st, double limit) {
   if (!x || !dy || !dw || cin <= 0 || cin % 16 || cout <= 0 || cout % 16 || n <= 0 || d <= 0 || h <= 0 || wd <= 0 ||
       (taps != 27 && taps != 1))
     return 1;
@@ -455,6 +477,7 @@ int wgrad_tc(const void* x, int cin, const void* dy, int cout, float* dw, int n,
   p.runs = (int)((tiles + run - 1) / run);
   const int64_t units = p.runs * blocks;
   if (units > 0x7fffffff) return 1;
+  if (taps == 27 && wgrad_tc_time(pl, p, units, std::min(units, ctas)) > limit) return 1;
   auto map = [&](CUtensorMap& m, const void* ptr, int c, int w, int bx, int by) {
     const cuuint64_t dims[5] = {(cuuint64_t)c, (cuuint64_t)wd, (cuuint64_t)h, (cuuint64_t)d, (cuuint64_t)n};
     const cuuint64_t strides[4] = {(cuuint64_t)c * 2, (cuuint64_t)c * 2 * wd, (cuuint64_t)c * 2 * wd * h,
