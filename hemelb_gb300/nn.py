@@ -61,6 +61,19 @@ def tc_faster(cin: int, cout: int, voxels: int, taps: int) -> bool:
     return voxels >= 1 << 15 or (taps == 27 and cin * cout > 256)
 
 
+def mostly_padding(cin: int, cout: int, n: int, d: int, h: int, w: int) -> bool:
+    """Volumes that fill less than a fifth of the tcgen05 convolution's 8 x 16 tiles and are
+    more of them than of the mma.sync kernel's bricks of 4 x 4 x 8, where that one is the
+    faster one: at 16 input channels (one slice of work a tile) and where it takes its 16
+    output channels a CTA (C_out no multiple of 32).  16 -> 48, us, mma.sync / tcgen05:
+    96 x 3 x 3 voxels 4.5 / 5.6, 48 x 1 x 48 6.1 / 8.0, 1 3.7 / 4.1, but 48 x 48 x 1 7.7 /
+    6.0.  Elsewhere tcgen05 is faster, or at most 5 % slower, for all but 19 of 1,447
+    shapes (31 % at worst)."""
+    tiles = n * d * -(-h // 16) * -(-w // 8)
+    bricks = n * -(-d // 4) * -(-h // 4) * -(-w // 8)
+    return cin == 16 and cout % 32 != 0 and 5 * n * d * h * w < 128 * tiles and (tiles > bricks or tiles <= 2)
+
+
 def conv3d(x, w, bias, out, out_f32=None, taps=27, relu=False, engine="auto"):
     """out[n,z,y,x,co] = act(sum_{tap,ci} x[n,(z,y,x)+off(tap),ci] w[tap,co,ci] + bias[co]).
 
@@ -80,7 +93,7 @@ def conv3d(x, w, bias, out, out_f32=None, taps=27, relu=False, engine="auto"):
         _need(out_f32, _F32, "conv3d FP32 output")
     if engine == "auto":
         engine = ("tc" if tc_eligible(cin, cout, x, w, out, out_f32) and tc_faster(cin, cout, n * d * h * wd, taps)
-                  else "mma")
+                  and not (taps == 27 and mostly_padding(cin, cout, n, d, h, wd)) else "mma")
     lib = _lib()
     fn = lib.hlbg_nn_conv3d_tc if engine == "tc" else lib.hlbg_nn_conv3d
     _ok(fn(_p(x), cin, _p(w), _p(bias), _p(out), _p(out_f32), cout, n, d, h, wd, taps, int(relu), _stream()),
