@@ -27,6 +27,7 @@
 
 #include "../../include/hemelb_gb300.h"
 #include "lb_device.cuh"
+#include "host_pages.h"
 #include "lb_launch.h"
 
 using namespace hlbg;
@@ -128,8 +129,11 @@ void parallel_for(int64_t n, F&& f) {
 // page in one after the other (1420 to 2870 us).  Four threads: each further one waits
 // for the others' faults when its stack is mapped (1.4 ms for six).  The pages' contents
 // do not change, and where the kernel refuses (an older one, memory that is not the
-// process's own) the copy faults them as before.  Small arrays and arrays that CUDA
-// knows (pinned, managed, device) are left alone.
+// process's own) the copy faults them as before.  Small arrays, arrays that CUDA knows
+// (pinned, managed, device) and arrays whose pages are all there are left alone: for those
+// the threads and the waits only cost time (density and velocity of 1.46M sites into
+// arrays in use 445 us by plain copies, 567 behind the threads; 223 MB of distributions
+// 1383 and 1834).
 class HostPages {
  public:
   static constexpr size_t kMin = 4u << 20, kChunk = 512u << 10;
@@ -138,7 +142,7 @@ class HostPages {
     const bool known = cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != cudaMemoryTypeUnregistered;
     if (known) cudaGetLastError();
     ranges_[n_ranges_++] = {static_cast<char*>(p), bytes, chunks_};
-    if (!known && bytes >= kMin) chunks_ += (bytes + kChunk - 1) / kChunk;
+    if (!known && bytes >= kMin && !hlbg::pages_present(p, bytes)) chunks_ += (bytes + kChunk - 1) / kChunk;
     else ranges_[n_ranges_ - 1].bytes = 0;
   }
   void start() {
