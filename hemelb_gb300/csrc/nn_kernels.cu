@@ -988,7 +988,12 @@ int hlbg_nn_relu_bwd(void* dy, const void* y, int64_t n, void* stream) {
 }
 
 int hlbg_nn_bias_grad(const void* dy, float* db, int64_t m, int32_t c, void* stream) {
-  if (relu_bias(const_cast<void*>(dy), nullptr, db, m, c, (cudaStream_t)stream)) return check_launch();  // reads dy
+  // A small tensor of few channels is done in the scalar kernel before a CTA of the vector
+  // kernel has added its rows, 256 for 8 channels (us, scalar / vector: 8 channels, 216
+  // voxels 1.4 / 2.3, 1,728 1.8 / 2.5, 6,912 3.6 / 2.3; 16 channels, 216 1.5 / 1.8, 1,728
+  // 2.1 / 1.7; 24 channels, 216 1.3 / 1.5; 48 the same in both).
+  const bool small = c < 48 && m <= (c <= 8 ? 2048 : 512);
+  if (!small && relu_bias(const_cast<void*>(dy), nullptr, db, m, c, (cudaStream_t)stream)) return check_launch();  // reads dy
   dim3 grid((unsigned)std::min<int64_t>((m + 255) / 256, 512), (unsigned)c);
   k_bias_grad<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)dy, db, m, c);
   return check_launch();
