@@ -982,7 +982,9 @@ int hlbg_nn_flip_transpose(const void* w, void* wt, int32_t cout, int32_t cin, i
 }
 
 int hlbg_nn_relu_bwd(void* dy, const void* y, int64_t n, void* stream) {
-  if (n % 8 == 0 && relu_bias(dy, y, nullptr, n / 8, 8, (cudaStream_t)stream)) return check_launch();
+  // From 2^18 values on in vectors (us, scalar / vector: 31,104 values 1.1 / 1.3, 110,592
+  // 1.2 / 1.3, 331,776 1.4 / 1.4, 663,552 2.2 / 1.5)
+  if (n >= 1 << 18 && n % 8 == 0 && relu_bias(dy, y, nullptr, n / 8, 8, (cudaStream_t)stream)) return check_launch();
   k_relu_bwd<<<blocks(n), 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)dy, (const __nv_bfloat16*)y, n);
   return check_launch();
 }
