@@ -809,26 +809,23 @@ int build_layout(hlbg_ctx* ctx, const hlbg_geometry* g) {
     std::vector<uint64_t> desc((size_t)nb, 0);
     for (int64_t b = 0; b < nb; ++b) {
       const uint64_t first = wb.size();
-      int row0 = 64, rowe = 0;
-      for (int row = 0; row < 64; ++row)
-        for (int t = 0; t < 8; ++t)
-          if (code[b * 512 + row * 8 + t]) {
-            row0 = std::min(row0, row);
-            rowe = row + 1;
-          }
-      if (rowe == 0) row0 = 0;
+      const uint32_t* cb = code.data() + b * 512;
+      uint64_t rows = 0;  // rows of 8 slots that hold fluid
+      for (int row = 0; row < 64; ++row) {
+        uint32_t any = 0;
+        for (int t = 0; t < 8; ++t) any |= cb[row * 8 + t];
+        rows |= (uint64_t)(any != 0) << row;
+      }
+      const int row0 = rows ? __builtin_ctzll(rows) : 0, rowe = rows ? 64 - __builtin_clzll(rows) : 0;
       if (split == 3) {
         // aligned groups of 32 slots, each a warp of its own, where they hold fluid
         for (int j0 = 0; j0 < 512; j0 += 32) {
-          bool any = false;
-          for (int j = j0; j < j0 + 32; ++j) any |= code[b * 512 + j] != 0;
-          if (!any) continue;
+          const uint32_t four = (uint32_t)(rows >> (j0 / 8)) & 15u;
+          if (!four) continue;
           for (int j = j0; j < j0 + 32; ++j) {
-            const uint32_t c = code[b * 512 + j];
-            bool row = false;
-            for (int t = j & ~7; t < (j & ~7) + 8; ++t) row |= code[b * 512 + t] != 0;
+            const uint32_t c = cb[j];
             tmp.push_back(c ? (uint16_t)(j | (c >= 2 ? kListBoundary : 0u))
-                            : (row ? (uint16_t)(j | kListSolid) : (uint16_t)0xffff));
+                            : ((four >> ((j - j0) / 8)) & 1u ? (uint16_t)(j | kListSolid) : (uint16_t)0xffff));
           }
         }
       } else if (split == 1) {
@@ -858,9 +855,7 @@ int build_layout(hlbg_ctx* ctx, const hlbg_geometry* g) {
       flush(b, false);
       const uint64_t nfw = wb.size() - first;
       for (int sec = 0; sec < 64 && split != 3; ++sec) {
-        bool any = false;
-        for (int t = 0; t < 8; ++t) any |= code[b * 512 + sec * 8 + t] != 0;
-        if (!any) continue;
+        if (!((rows >> sec) & 1u)) continue;
         for (int t = 0; t < 8; ++t)
           if (!code[b * 512 + sec * 8 + t]) tmp.push_back((uint16_t)(sec * 8 + t));
       }
@@ -929,7 +924,8 @@ int build_layout(hlbg_ctx* ctx, const hlbg_geometry* g) {
   {
     std::vector<int32_t> io_slot, io_meta;
     if (ctx->inlets.size() + ctx->outlets.size() >= (size_t)1 << 26) return fail(ctx, HLBG_ERR_INVAL, "too many iolets");
-    for (int64_t r = 0; r < ctx->nrec; ++r)
+    for (int64_t r = 0; r < ctx->nrec; ++r) {
+      if (rtype[r] < 2) continue;  // bulk and wall sites have none
       for (int d = 1; d < 19; ++d)
         if (((rlinks[r] >> (3 * d)) & 7u) == HLBG_LC_IOLET) {
           const bool inlet = rtype[r] == 2 || rtype[r] == 4;
@@ -937,6 +933,7 @@ int build_layout(hlbg_ctx* ctx, const hlbg_geometry* g) {
           io_slot.push_back(ctx->h_rec_slot[r]);
           io_meta.push_back((int32_t)((uint32_t)gi << 5) | d);
         }
+    }
     ctx->n_io_links = (int64_t)io_slot.size();
     if ((rc = upload(ctx, &ctx->d_io_slot, io_slot))) return rc;
     if ((rc = upload(ctx, &ctx->d_io_meta, io_meta))) return rc;
