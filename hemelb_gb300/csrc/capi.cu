@@ -42,20 +42,6 @@ const int HCY[19] = {0, 0, 0, 1, -1, 0, 0, 1, -1, -1, 1, 0, 0, 0, 0, 1, -1, 1, -
 const int HCZ[19] = {0, 0, 0, 0, 0, 1, -1, 0, 0, 0, 0, 1, -1, -1, 1, 1, -1, -1, 1};
 const int HINV[19] = {0, 2, 1, 4, 3, 6, 5, 8, 7, 10, 9, 12, 11, 14, 13, 16, 15, 18, 17};
 
-// Fluid list order within a block: its sites in slot order (HLBG_LIST_SPLIT=0); its bulk
-// sites first and then its boundary sites (1), which keeps most warps on the bulk push
-// path but leaves gaps in each warp's slots; whole 8-site rows, those without a boundary
-// site first (2); or aligned groups of 32 slots that hold fluid (3), whose solid lanes
-// zero their slots, so that every warp reads and writes whole sectors of one 128-byte line
-// a direction and no warp is spent on zeros alone.  The default (-1): FP64, bound by its
-// arithmetic, takes 0, which has the fewest warps.  FP32 takes 3 (us a step against 0, at
-// 128 x 9: tree of 16.9M sites 512 / 569, of 7.8M 264 / 311, ensemble of 4.9M 171 / 179,
-// bifurcation of 1.5M 64.7 / 65.5; all slots 538, 282, 185, 67.9).  FP16 takes 1 (tree of
-// 7.8M 229 against 248 with 0 and 254 in all slots).
-#ifndef HLBG_LIST_SPLIT
-#define HLBG_LIST_SPLIT -1
-#endif
-
 // Index of (x, y) along a 2-D Hilbert curve over an n x n grid (n a power of two):
 // the standard rotate-and-reflect walk from the top quadrant down.
 uint64_t hilbert2(uint32_t n, uint32_t x, uint32_t y) {
@@ -802,7 +788,7 @@ int build_layout(hlbg_ctx* ctx, const hlbg_geometry* g) {
       }
       tmp.clear();
     };
-    const int split = HLBG_LIST_SPLIT < 0 ? (ctx->prec == HLBG_FP16 ? 1 : (ctx->prec == HLBG_FP64 ? 0 : 3)) : HLBG_LIST_SPLIT;
+    const int split = list_order(ctx->prec);
     // pipelined launch, per block: its first list warp (bits 0-31), the span of
     // rows from its first fluid row to its last (32-37: first, 38-44: end), its
     // fluid warps (45-50) and zero-fill warps (51-56)

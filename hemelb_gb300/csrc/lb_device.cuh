@@ -89,6 +89,27 @@ constexpr unsigned kListBoundary = 1u << 14;
 // Flag of a solid slot in a fluid warp of the list, whose row of 8 slots holds fluid: its
 // lane writes zeros there.
 constexpr unsigned kListSolid = 1u << 13;
+// Fluid list order within a block: its sites in slot order (HLBG_LIST_SPLIT=0); its bulk
+// sites first and then its boundary sites (1), which keeps most warps on the bulk push
+// path but leaves gaps in each warp's slots; whole 8-site rows, those without a boundary
+// site first (2); or aligned groups of 32 slots that hold fluid (3), whose solid lanes
+// zero their slots, so that every warp reads and writes whole sectors of one 128-byte line
+// a direction and no warp is spent on zeros alone.  The default (-1): FP64, bound by its
+// arithmetic, takes 0, which has the fewest warps.  FP32 takes 3 (us a step against 0, at
+// 128 x 9: tree of 16.9M sites 512 / 569, of 7.8M 264 / 311, ensemble of 4.9M 171 / 179,
+// bifurcation of 1.5M 64.7 / 65.5; all slots 538, 282, 185, 67.9).  FP16 takes 1 (tree of
+// 7.8M 229 against 248 with 0, 243 with 3 and 254 in all slots; forest of 223M 5623 against
+// 5878 with 3, ensemble 152 against 161, bifurcation 57.4 against 70.7).
+#ifndef HLBG_LIST_SPLIT
+#define HLBG_LIST_SPLIT -1
+#endif
+__host__ __device__ constexpr int list_order(int prec) {
+  return HLBG_LIST_SPLIT >= 0 ? HLBG_LIST_SPLIT : (prec == 0 ? 0 : (prec == 1 ? 3 : 1));
+}
+// Whether a fluid warp of the list may hold solid slots; the other orders' kernels need no
+// code for them.
+template <int P>
+constexpr bool kSolidLanes = list_order(P) == 3;
 // HLBG_PACK=1 builds the packed layout (fluid sites of partly fluid blocks in the
 // first slots; with HLBG_PACK_FILL=p only the blocks whose fluid fills less than
 // p % of the z-rows it touches).  It moves 5-12% fewer bytes but the packed code
@@ -124,7 +145,7 @@ constexpr unsigned kListSolid = 1u << 13;
 #endif
 // In z-column order the non-empty blocks next to each other in z are consecutive, so a
 // push that crosses a z face moves by one whole block (PushTargets); the other build
-// options look every neighbour up.
+// options, and the pipelined launch, look every neighbour up.
 #define HLBG_Z_COLUMNS (!HLBG_PACK && !HLBG_BLOCK_ORDER && HLBG_BLOCK_SORT != 1)
 // bits 0, 1, 2 of v to bits 0, 3, 6 and back
 __host__ __device__ __forceinline__ int dilate3(int v) { return (v & 1) | ((v & 2) << 2) | ((v & 4) << 4); }

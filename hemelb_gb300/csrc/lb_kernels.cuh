@@ -223,9 +223,8 @@ __device__ __forceinline__ T bfl_value(T out, T back, T q) {
   return (out + ((T)2.0 * q - (T)1) * back) / ((T)2.0 * q);
 }
 
-#if !HLBG_Z_COLUMNS
-// Pushes of the all-slots kernel: every lane takes part in the shuffles, only
-// bulk sites store.
+// Pushes by lookup: the block of every push from the neighbour table, every lane taking
+// part in the shuffles, only bulk sites storing (push_warp says where).
 template <int P, int D>
 struct PushBulk {
   template <class S, class T, class B>
@@ -282,9 +281,7 @@ struct PushMixed<P, Q> {
   static __device__ __forceinline__ void run(S*, const StepArgs&, const B&, int, int, int, int,
                                              int64_t, bool, bool, uint64_t, int64_t, const T*) {}
 };
-#endif
 
-#if HLBG_Z_COLUMNS
 // Where a lane's site pushes to.  A site crosses at most one face per axis, so four
 // blocks are all it needs: its own, the one across its x face, across its y face, and
 // across both (three shuffles of the neighbour table); z-neighbours follow or precede
@@ -457,13 +454,13 @@ struct PushEachMixed<P, Q, XFACE, BFL> {
   static __device__ __forceinline__ void run(const PushTargets<P, true>&, const StepArgs&, bool, bool, uint64_t,
                                              int64_t, const T*) {}
 };
-#endif
 
 // The pushes of one warp of one block b: this lane's site in slot j, local coordinates
 // x, y, z, post-collision values fpost, code as site_code (0: no site here; a zero goes
 // to its slot where row_fluid).  tabreg: the block's neighbour table in lanes 0..26.
-// Every lane of the warp takes part.  W: warps of the CTA.
-template <int P, int W, class T>
+// Every lane of the warp takes part.  W: warps of the CTA.  COLUMNS: by pointers into the
+// blocks' z columns (PushTargets), else by lookup.
+template <int P, int W, bool COLUMNS, class T>
 __device__ __forceinline__ void push_warp(const StepArgs& a, int64_t b, int32_t tabreg, int x, int y, int z, int j,
                                           uint32_t code, bool row_fluid, const T* fpost) {
   using S = typename Store<P>::S;
@@ -475,40 +472,38 @@ __device__ __forceinline__ void push_warp(const StepArgs& a, int64_t b, int32_t 
   // 32-byte sector of slots it shares with fluid slots (sectors without any receive no
   // write at all and stay untouched).
   const bool zero = code == 0 && row_fluid;
-#if HLBG_Z_COLUMNS
-  if (!mixed) {
-    const PushTargets<P, false> t(fn, b, tabreg, x, y, z, j);
-    if (code == 1) {
-      if (t.xface) PushEach<P, 0, true>::run(t, a, fpost);
-      else PushEach<P, 0, false>::run(t, a, fpost);
+  if constexpr (COLUMNS) {
+    if (!mixed) {
+      const PushTargets<P, false> t(fn, b, tabreg, x, y, z, j);
+      if (code == 1) {
+        if (t.xface) PushEach<P, 0, true>::run(t, a, fpost);
+        else PushEach<P, 0, false>::run(t, a, fpost);
+      }
+      return;
     }
-    return;
-  }
-  const uint64_t links = bnd ? a.b_links[r] : 0ull;
-  const PushTargets<P, true> t(fn, b, tabreg, x, y, z, j);
-  if (P != 0 && a.wall == 1) {  // the only walls with interpolated links
-    if (t.xface) PushEachMixed<P, 0, true, true>::run(t, a, code != 0, zero, links, r, fpost);
-    else PushEachMixed<P, 0, false, true>::run(t, a, code != 0, zero, links, r, fpost);
-  } else {
-    if (t.xface) PushEachMixed<P, 0, true, false>::run(t, a, code != 0, zero, links, r, fpost);
-    else PushEachMixed<P, 0, false, false>::run(t, a, code != 0, zero, links, r, fpost);
-  }
-  if constexpr (P == 0) {
-    if (a.wall == 1) {
-      __shared__ BflQueue queue[W];
-      BflGather g{queue[threadIdx.x >> 5], static_cast<double*>(a.f_new) + b * (Q * kSites), a, 0};
-      BflEach<1>::run(g, links, j, r, fpost);
-      if (g.count) g.eval(0, g.count);
+    const uint64_t links = bnd ? a.b_links[r] : 0ull;
+    const PushTargets<P, true> t(fn, b, tabreg, x, y, z, j);
+    if (P != 0 && a.wall == 1) {  // the only walls with interpolated links
+      if (t.xface) PushEachMixed<P, 0, true, true>::run(t, a, code != 0, zero, links, r, fpost);
+      else PushEachMixed<P, 0, false, true>::run(t, a, code != 0, zero, links, r, fpost);
+    } else {
+      if (t.xface) PushEachMixed<P, 0, true, false>::run(t, a, code != 0, zero, links, r, fpost);
+      else PushEachMixed<P, 0, false, false>::run(t, a, code != 0, zero, links, r, fpost);
     }
-  }
-#else
-  if (!mixed) {
+    if constexpr (P == 0) {
+      if (a.wall == 1) {
+        __shared__ BflQueue queue[W];
+        BflGather g{queue[threadIdx.x >> 5], static_cast<double*>(a.f_new) + b * (Q * kSites), a, 0};
+        BflEach<1>::run(g, links, j, r, fpost);
+        if (g.count) g.eval(0, g.count);
+      }
+    }
+  } else if (!mixed) {
     PushBulk<P, 0>::run(fn, a, ShflBase{tabreg}, x, y, z, code == 1, fpost);
   } else {
     const uint64_t links = bnd ? a.b_links[r] : 0ull;
     PushMixed<P, 0>::run(fn, a, ShflBase{tabreg}, x, y, z, j, b * (Q * kSites), code != 0, zero, links, r, fpost);
   }
-#endif
 }
 
 // StabilityTester::PostSendToParent (Code/lb/StabilityTester.h:91-149) and
@@ -1031,7 +1026,7 @@ __device__ __forceinline__ void collide_slot(const StepArgs& a, int64_t s, MonAc
   if constexpr (MON) {
     if (code != 0) mon_site<P>(a, s, f, m0, mx, my, mz, acc, check, uo);
   }
-  push_warp<P, W>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, row_fluid, fpost);
+  push_warp<P, W, HLBG_Z_COLUMNS>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, row_fluid, fpost);
 }
 
 // One warp of the fluid list: 32 fluid sites of one block (or the zero-fill of its
@@ -1040,7 +1035,7 @@ __device__ __forceinline__ void collide_slot(const StepArgs& a, int64_t s, MonAc
 // stored nowhere) and push its post-collision values, on the warp's bulk path when
 // no lane has a boundary record.  tabreg: the block's neighbour table in lanes
 // 0..26.  Every lane of the warp must take part (shuffles, ballot).
-template <int P, bool MON, int W>
+template <int P, bool MON, int W, bool COLUMNS = HLBG_Z_COLUMNS>
 __device__ __forceinline__ void collide_and_push(const StepArgs& a, int64_t b, int j, int64_t s, int l,
                                                  uint32_t code, bool zero, int32_t tabreg, typename Calc<P>::T* f,
                                                  MonAccT<P>& acc, bool check, const MonOld<P>& uo) {
@@ -1051,7 +1046,7 @@ __device__ __forceinline__ void collide_and_push(const StepArgs& a, int64_t b, i
   if constexpr (MON) {
     if (code != 0) mon_site<P>(a, s, f, m0, mx, my, mz, acc, check, uo);
   }
-  push_warp<P, W>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, zero, fpost);
+  push_warp<P, W, COLUMNS>(a, b, tabreg, l >> 6, (l >> 3) & 7, l & 7, j, code, zero, fpost);
 }
 
 // The unit's list entries (block e, this lane's slot js) are loaded by the caller.
@@ -1063,7 +1058,7 @@ __device__ __forceinline__ void collide_listed_unit(const StepArgs& a, int32_t e
   using T = typename Calc<P>::T;
   const int lane = threadIdx.x & 31;
   const int64_t b = e & 0x7fffffff;
-  const bool idle = js == 0xffffu, on = !idle && !(js & kListSolid);
+  const bool idle = js == 0xffffu, on = !idle && !(kSolidLanes<P> && (js & kListSolid));
   const int j = idle ? 0 : (int)(js & (kSites - 1));
   const int64_t s = b * kSites + j;
   S* fn = static_cast<S*>(a.f_new);
@@ -1095,7 +1090,7 @@ __device__ __forceinline__ void collide_listed_unit(const StepArgs& a, int32_t e
 #pragma unroll
     for (int i = 0; i < Q; ++i) f[i] = (T)(P == 0 ? weight_d(i) : 0.0);
   }
-  collide_and_push<P, MON, W>(a, b, j, s, l, code, !idle && !on, tabreg, f, acc, check, uo);
+  collide_and_push<P, MON, W>(a, b, j, s, l, code, kSolidLanes<P> && !idle && !on, tabreg, f, acc, check, uo);
 }
 
 template <int P, bool MON, int W>
@@ -1421,7 +1416,7 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) k_stream_collide_pipe(StepA
     const int32_t tabreg = lane < 27 && first < nfw ? __ldg(a.block_nbr + b * 27 + lane) : 0;
     for (int task = first; task < ntask; task += NCW) {  // warp-uniform trips
       const unsigned js = list[task * 32 + lane];
-      const bool idle = js == 0xffffu, on = !idle && !(js & kListSolid);
+      const bool idle = js == 0xffffu, on = !idle && !(kSolidLanes<P> && (js & kListSolid));
       const int j = idle ? 0 : (int)(js & (kSites - 1));
       const int64_t s = b * kSites + j;
       if (task >= nfw) {  // zero-fill warp: complete the sectors its slots share with fluid
@@ -1440,7 +1435,10 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) k_stream_collide_pipe(StepA
         else
           f[d] = on ? __half2float(stage[d * kSites + j]) * a.fp16_inv_scale : 0.f;
       }
-      collide_and_push<P, false, 1>(a, b, j, s, j, code, !idle && !on, tabreg, f, acc, false, uo);
+      // by lookup: the pointers spill in the 64 registers of 1,024 threads (us a step, pointers /
+      // lookups: FP32 tree of 16.9M sites 662 / 639, forest of 223M 8347 / 8006; FP16 552 /
+      // 515 and 6842 / 6376)
+      collide_and_push<P, false, 1, false>(a, b, j, s, j, code, kSolidLanes<P> && !idle && !on, tabreg, f, acc, false, uo);
     }
     rot = (rot + ntask) % NCW;
     __syncwarp();
