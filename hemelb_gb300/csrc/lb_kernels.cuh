@@ -838,34 +838,35 @@ __device__ __forceinline__ void mon_result(const StepArgs& a, const MonAcc& v) {
 }
 
 // The partials of a monitored update are folded by its last CTA to arrive (mon_finish),
-// or, from kMonFold CTAs on, by a launch of their own behind it (k_mon_fold).  Either
+// or, from kMonApart CTAs on, by a launch of their own behind it (k_mon_fold).  Either
 // tree is fixed, so the result does not depend on the order of arrival.  In the launch
 // every CTA waits for its stores to reach L2 before it counts itself in, and holds its
 // registers meanwhile; a launch costs a call of one small step 1 us of host time.  Fold in
-// the launch against fold behind it, 128 x 8 list, us a checked step: FP32 forest of 223M
-// sites 9664 / 8704, tree of 16.9M 750 / 680, ensemble of 4.9M 249 / 228, pipe of 25k (250
-// CTAs) 10.1 / 9.2 in calls of many steps and 27.1 / 27.9 in calls of one; FP16 forest
-// 9114 / 7881; FP64 pipe (1,000 one-warp CTAs) 24.6 / 23.9 and 41.7 / 40.8.
+// the launch / behind it, us a checked step: FP32 forest of 223M sites 9664 / 8704, tree of
+// 16.9M 750 / 680, ensemble of 4.9M 249 / 228; FP16 forest 9114 / 7881; FP64 pipe of 25k
+// (1,000 one-warp CTAs) 24.6 / 23.9; FP32 pipe, 390 CTAs in all slots 11.7 / 10.4 in calls of
+// many steps and 27.4 / 27.6 in calls of one, 250 in the list 8.4 / 9.2 and 26.6 / 27.9.
 template <int P>
 __device__ __forceinline__ void mon_finish(const StepArgs& a, const MonAccT<P>& acc, unsigned cta) {
   mon_partial<P>(a, acc, cta);
-  if (a.mon_apart || threadIdx.x >= 32) return;
+  if (a.mon_apart) return;
+  __shared__ int last;
   const int64_t n = a.mon_nparts;
-  const int lane = threadIdx.x & 31;
-  int last = 0;
-  if (lane == 0) {
+  if (threadIdx.x == 0) {
     __threadfence();
     last = atomicAdd(a.mon_tick, 1u) == (unsigned)n - 1;
   }
-  if (!__shfl_sync(0xffffffffu, last, 0)) return;
+  __syncthreads();
+  if (!last) return;
   __threadfence();
   MonAcc v = mon_neutral();
-#pragma unroll 4
-  for (int64_t i = lane; i < n; i += 32) mon_combine(v, mon_load_cta<P>(a, i));
-  v = mon_warp(v);
-  if (lane != 0) return;
-  *a.mon_tick = 0;
-  mon_result<P>(a, v);
+#pragma unroll 2
+  for (unsigned i = threadIdx.x; i < (unsigned)n; i += blockDim.x) mon_combine(v, mon_load_cta<P>(a, i));
+  v = mon_block(v);
+  if (threadIdx.x == 0) {
+    *a.mon_tick = 0;
+    mon_result<P>(a, v);
+  }
 }
 
 // A CTA folds kMonFold of the update's partials, the last one to arrive the CTAs'.
@@ -1489,7 +1490,7 @@ void launch_listed(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
   StepArgs b = a;
   b.io_ctas = (uint32_t)((a.n_io_links + THREADS - 1) / THREADS);
   b.let_in = g >= 4 * 152 * MINB;
-  b.mon_apart = MON && a.mon_fold && g >= kMonFold;
+  b.mon_apart = MON && a.mon_fold && g >= kMonApart;
   if (g) launch_overlapped(k_stream_collide_listed<P, THREADS, MINB, MON>, (unsigned)g + b.io_ctas, THREADS, 0, st, b, bxyz);
   if (b.mon_apart) launch_mon_fold<P>(b, st);
 }
@@ -1968,7 +1969,7 @@ void launch_sc(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
   StepArgs b = a;
   b.io_ctas = (uint32_t)((a.n_io_links + THREADS - 1) / THREADS);
   b.let_in = g >= 4 * 152 * MINB;
-  b.mon_apart = MON && a.mon_fold && g >= kMonFold;
+  b.mon_apart = MON && a.mon_fold && g >= kMonApart;
   if (g) launch_overlapped(k_stream_collide<P, THREADS, MINB, MON>, g + b.io_ctas, THREADS, 0, st, b, bxyz);
   if (b.mon_apart) launch_mon_fold<P>(b, st);
 }

@@ -16,8 +16,9 @@ struct StepArgs;
 // 8: persistent, pipelined block staging (FP32 / FP16).
 constexpr int kSCVariants = 9;
 
-// Partials of a monitored step one CTA of k_mon_fold folds; a launch of fewer CTAs folds
-// its own.
+// CTAs from which on a monitored step's partials are folded by a launch of their own
+// (k_mon_fold), kMonFold of them by a CTA.
+constexpr int kMonApart = 256;
 constexpr int kMonFold = 512;
 
 struct PostArgs {

@@ -1,5 +1,5 @@
 """Where the fused StabilityTester's partials are folded: inside the update's launch, or,
-from 512 CTAs on, by a launch of their own behind it.  Boxes of full blocks give CTA
+from 256 CTAs on, by a launch of their own behind it.  Boxes of full blocks give CTA
 counts on both sides of the line and remainders of the fold's own CTAs; the stats of each
 step are compared with the separate reduction of a twin that makes plain steps."""
 import ctypes as C
@@ -52,9 +52,9 @@ def box(blocks, side=4):
 # CTAs of a full block: FP64 16 of one warp in the list (6) and 4 of 128 slots (1); FP32
 # and FP16 4 in either
 @pytest.mark.parametrize("precision,variant,blocks", [
-    (capi.FP64, 6, 31), (capi.FP64, 6, 32), (capi.FP64, 6, 33), (capi.FP64, 6, 70),
-    (capi.FP64, 1, 127), (capi.FP64, 1, 128),
-    (capi.FP32DEV, 6, 1), (capi.FP32DEV, 6, 127), (capi.FP32DEV, 6, 128), (capi.FP32DEV, 6, 129),
+    (capi.FP64, 6, 15), (capi.FP64, 6, 16), (capi.FP64, 6, 17), (capi.FP64, 6, 31), (capi.FP64, 6, 32), (capi.FP64, 6, 33), (capi.FP64, 6, 70),
+    (capi.FP64, 1, 63), (capi.FP64, 1, 64), (capi.FP64, 1, 127), (capi.FP64, 1, 128),
+    (capi.FP32DEV, 6, 1), (capi.FP32DEV, 6, 63), (capi.FP32DEV, 1, 64), (capi.FP32DEV, 6, 65), (capi.FP32DEV, 6, 127), (capi.FP32DEV, 6, 128), (capi.FP32DEV, 6, 129),
     (capi.FP32DEV, 3, 300), (capi.FP16, 2, 257), (capi.FP16, 5, 400)])
 def test_stats_of_every_step_on_both_sides_of_the_line(precision, variant, blocks):
     g = box(blocks)
