@@ -52,6 +52,11 @@ def tc_eligible(cin: int, cout: int, *tensors) -> bool:
     return True
 
 
+def tc_tiles(n: int, d: int, h: int, w: int) -> int:
+    """Tiles of 8 x 16 x 2 output voxels of a volume (ragged ones whole)."""
+    return n * -(-d // 2) * -(-h // 16) * -(-w // 8)
+
+
 def tc_faster(cin: int, cout: int, voxels: int, taps: int) -> bool:
     """Where the tcgen05 convolution is the faster one (the two give the same bits): all
     but small volumes at 16 -> 16 channels and of the 1x1x1 convolution, whose one slice
