@@ -931,8 +931,16 @@ int build_layout(hlbg_ctx* ctx, const hlbg_geometry* g) {
   return HLBG_OK;
 }
 
-constexpr int kMonFields = 7;  // partials: mass, max |du|, min f, unstable, min rho, max rho, max |u|
-constexpr int kMonResult = 8;  // the same plus the valid flag
+constexpr int kMonResult = 8;  // mass, max |du|, min f, unstable, valid, min rho, max rho, max |u|
+
+// CTAs, and partials, of a monitored step in launch shape `variant`.
+int64_t monitored_grid(const hlbg_ctx* ctx, int variant) {
+  switch (ctx->prec) {
+    case 0: return monitored_grid_0(ctx->nslot, variant, ctx->n_warps);
+    case 1: return monitored_grid_1(ctx->nslot, variant, ctx->n_warps);
+    default: return monitored_grid_2(ctx->nslot, variant, ctx->n_warps);
+  }
+}
 
 // Buffers of the fused StabilityTester, allocated on first use.
 int mon_prepare(hlbg_ctx* ctx) {
@@ -942,11 +950,11 @@ int mon_prepare(hlbg_ctx* ctx) {
   int rc = dev_alloc(ctx, &u, 3 * (size_t)ctx->nslot * es);
   if (rc) return rc;
   ctx->d_mon_u = u;
-  // one partial per CTA, for every launch shape: all slots in CTAs of 128 or more
-  // threads, or the fluid list (FP64: one warp per CTA, else four)
-  const int64_t max_ctas = std::max((ctx->nslot + 127) / 128, ctx->prec == 0 ? ctx->n_warps : (ctx->n_warps + 3) / 4);
-  if ((rc = dev_alloc(ctx, &ctx->d_mon_part, kMonFields * (size_t)max_ctas))) return rc;
-  if ((rc = dev_alloc(ctx, &ctx->d_mon_part2, kMonFields * (size_t)((max_ctas + kMonFold - 1) / kMonFold)))) return rc;
+  // one partial per CTA, for every launch shape
+  int64_t max_ctas = 0;
+  for (int v = 0; v < kSCVariants; ++v) max_ctas = std::max(max_ctas, monitored_grid(ctx, v));
+  if ((rc = dev_alloc(ctx, &ctx->d_mon_part, kMonWords * (size_t)max_ctas))) return rc;
+  if ((rc = dev_alloc(ctx, &ctx->d_mon_part2, kMonWords * (size_t)((max_ctas + kMonFold - 1) / kMonFold)))) return rc;
   if ((rc = dev_alloc(ctx, &ctx->d_mon_tick, 1))) return rc;
   CK(cudaMemsetAsync(ctx->d_mon_tick, 0, sizeof(uint32_t), ctx->stream));
   if ((rc = dev_alloc(ctx, &ctx->d_mon_state, 1))) return rc;
@@ -968,20 +976,12 @@ int mon_invalidate(hlbg_ctx* ctx) {
   return HLBG_OK;
 }
 
-int64_t monitored_grid(const hlbg_ctx* ctx) {
-  switch (ctx->prec) {
-    case 0: return monitored_grid_0(ctx->nslot, ctx->sc_variant, ctx->n_warps);
-    case 1: return monitored_grid_1(ctx->nslot, ctx->sc_variant, ctx->n_warps);
-    default: return monitored_grid_2(ctx->nslot, ctx->sc_variant, ctx->n_warps);
-  }
-}
-
 // Monitor fields of a step's arguments: the kernel records velocities and, with
 // `fold`, compares and reduces them (steady: counts the check).
 void mon_args(hlbg_ctx* ctx, StepArgs& a, bool fold, bool steady) {
   a.mon_u = ctx->d_mon_u;
   a.mon_part = ctx->d_mon_part;
-  a.mon_nparts = monitored_grid(ctx);
+  a.mon_nparts = monitored_grid(ctx, ctx->sc_variant);
   a.mon_part2 = ctx->d_mon_part2;
   a.mon_tick = ctx->d_mon_tick;
   a.mon_state = ctx->d_mon_state;

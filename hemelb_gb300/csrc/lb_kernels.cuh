@@ -737,7 +737,7 @@ __device__ __forceinline__ MonAccT<P> mon_neutral_t() {
 // One CTA's monitor partial: FP64 form as 7 64-bit words (the fields of MonAcc, stride
 // mon_nparts); FP32 forms as 8 32-bit words [sum (rho-1) | max |du|^2 | min f | min
 // (rho-1) | max (rho-1) | max |u|^2 | count | unstable] in the same buffer.
-constexpr int kMonWords = 7;
+static_assert(sizeof(MonAcc) == kMonWords * 8 && sizeof(MonAccF) <= kMonWords * 8, "the partials' buffers hold either form");
 __device__ __forceinline__ void mon_store(double* part, int64_t n, int64_t i, const MonAcc& r) {
   long long* p = reinterpret_cast<long long*>(part);
   part[i] = r.mass;
@@ -1484,6 +1484,9 @@ void launch_pipe(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
 // 25k-site pipe (5 warps a SM) 128-thread CTAs leave some SMs with 8.
 constexpr int kListThreads64 = 32, kListMinb64 = 16;
 
+// Monitored fluid list of the FP32 forms: the launch and the count of its partials.
+constexpr int kMonListThreads = 128, kMonListMinb = 8;
+
 template <int P, int THREADS, int MINB, bool MON>
 void launch_listed(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
   const int64_t g = (a.n_warps * 32 + THREADS - 1) / THREADS;
@@ -2034,7 +2037,7 @@ void launch_update(const StepArgs& a, const int32_t* bxyz, cudaStream_t st, int 
       case 1: launch_sc<P, 128, 8, true>(a, bxyz, st); break;
       case 2: launch_sc<P, 256, 4, true>(a, bxyz, st); break;
       case 3: launch_sc<P, 512, 2, true>(a, bxyz, st); break;
-      default: launch_listed<P, 128, 8, true>(a, bxyz, st); break;
+      default: launch_listed<P, kMonListThreads, kMonListMinb, true>(a, bxyz, st); break;
     }
   } else {
     // the staged shapes need the block tables (the default layout)
@@ -2063,7 +2066,8 @@ void launch_update(const StepArgs& a, const int32_t* bxyz, cudaStream_t st, int 
 // CTAs of a monitored step's update (one partial each).
 template <int P>
 int64_t monitored_ctas(int64_t nslot, int variant, int64_t n_warps) {
-  if (variant >= 4) return P == 0 ? (n_warps * 32 + kListThreads64 - 1) / kListThreads64 : (n_warps * 32 + 127) / 128;
+  constexpr int threads = P == 0 ? kListThreads64 : kMonListThreads;
+  if (variant >= 4) return (n_warps * 32 + threads - 1) / threads;
   if (P == 0 || variant < 2) return nslot / 128;
   return variant == 2 ? nslot / 256 : nslot / 512;
 }

@@ -20,6 +20,8 @@ constexpr int kSCVariants = 9;
 // (k_mon_fold), kMonFold of them by a CTA.
 constexpr int kMonApart = 256;
 constexpr int kMonFold = 512;
+// 64-bit words of a partial (hlbg_ctx's buffers, mon_store)
+constexpr int kMonWords = 7;
 
 struct PostArgs {
   void* f_new;
