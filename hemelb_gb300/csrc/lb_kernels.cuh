@@ -4,6 +4,7 @@
 
 #include "lb_device.cuh"
 #include "lb_launch.h"
+#include "sm_count.h"
 
 #include <algorithm>
 #include <atomic>
@@ -1492,7 +1493,7 @@ void launch_listed(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
   const int64_t g = (a.n_warps * 32 + THREADS - 1) / THREADS;
   StepArgs b = a;
   b.io_ctas = (uint32_t)((a.n_io_links + THREADS - 1) / THREADS);
-  b.let_in = g >= 4 * 152 * MINB;
+  b.let_in = g >= (int64_t)4 * sm_count() * MINB;
   b.mon_apart = MON && a.mon_fold && g >= kMonApart;
   if (g) launch_overlapped(k_stream_collide_listed<P, THREADS, MINB, MON>, (unsigned)g + b.io_ctas, THREADS, 0, st, b, bxyz);
   if (b.mon_apart) launch_mon_fold<P>(b, st);
@@ -1971,7 +1972,7 @@ void launch_sc(const StepArgs& a, const int32_t* bxyz, cudaStream_t st) {
   const unsigned g = (unsigned)(a.nslot / THREADS);
   StepArgs b = a;
   b.io_ctas = (uint32_t)((a.n_io_links + THREADS - 1) / THREADS);
-  b.let_in = g >= 4 * 152 * MINB;
+  b.let_in = g >= (int64_t)4 * sm_count() * MINB;
   b.mon_apart = MON && a.mon_fold && g >= kMonApart;
   if (g) launch_overlapped(k_stream_collide<P, THREADS, MINB, MON>, g + b.io_ctas, THREADS, 0, st, b, bxyz);
   if (b.mon_apart) launch_mon_fold<P>(b, st);

@@ -16,6 +16,7 @@
 
 #include "../../include/hemelb_gb300_nn.h"
 #include "overlap.cuh"
+#include "sm_count.h"
 
 namespace {
 
@@ -861,13 +862,13 @@ inline bool aligned16(const void* a, const void* b = nullptr, const void* c = nu
 inline bool vec8(int64_t elems, int64_t c) { return c > 0 && c % 8 == 0 && elems > 0 && elems / 8 < 0x7fff0000ll; }
 inline bool even3(int32_t d, int32_t h, int32_t w) { return d % 2 == 0 && h % 2 == 0 && w % 2 == 0; }
 
-// ReLU mask and bias sum in one pass: 8 CTAs of 256 threads a SM (152 SMs), at least
+// ReLU mask and bias sum in one pass: 8 CTAs of 256 threads a SM, at least
 // four rows a thread.  False: not a shape of the vector kernel.
 inline bool relu_bias(void* dy, const void* y, float* db, int64_t m, int32_t c, cudaStream_t st) {
   if (!vec8(m * c, c) || c > 2048 || m >= 0x7fff0000ll || !aligned16(dy, y)) return false;
   const uint32_t G = (uint32_t)c / 8, rows = 256 / G;
   const int64_t want = (m + 4 * rows - 1) / (4 * rows);
-  launch_overlapped(k_relu_bias_v8, (unsigned)std::min<int64_t>(want, 1216), 256, 0, st, (uint4*)dy, (const uint4*)y, db,
+  launch_overlapped(k_relu_bias_v8, (unsigned)std::min<int64_t>(want, 8 * hlbg::sm_count()), 256, 0, st, (uint4*)dy, (const uint4*)y, db,
                     (uint32_t)m, G);
   return true;
 }
@@ -877,9 +878,9 @@ inline unsigned blocks(int64_t n, int t = 256) { return (unsigned)((n + t - 1) /
 // Modelled microseconds of k_wgrad_brick, bpc bricks a CTA, for nbricks bricks of `shares`
 // channel blocks (as wgrad_tc_time): rounds of two CTAs an SM, which slow each other down,
 // and the additions to dw by their number and by the CTAs that meet at an address.
-inline double wgrad_mma_time(int cin, int cout, int nci, int64_t bpc, int64_t nbricks, int shares) {
-  const double gx = (double)((nbricks + bpc - 1) / bpc), ctas = gx * shares, per = ctas / 304.0;
-  const double rounds = per > 2 ? per : std::max(1.0, std::ceil(per)), resident = std::min(2.0, std::max(1.0, ctas / 152.0));
+inline double wgrad_mma_time(int cin, int cout, int nci, int64_t bpc, int64_t nbricks, int shares, int sms) {
+  const double gx = (double)((nbricks + bpc - 1) / bpc), ctas = gx * shares, per = ctas / (2.0 * sms);
+  const double rounds = per > 2 ? per : std::max(1.0, std::ceil(per)), resident = std::min(2.0, std::max(1.0, ctas / sms));
   const double chain = rounds * ((double)bpc * (nci == 2 ? 1.5 : 0.93) * (1 + 2.4 * (resident - 1)) + (nci == 2 ? 1.5 : 0.2));
   const double adds = gx * 27e-6 * cin * cout * 2.0, meet = 0.061 * gx;
   return 3.5 + std::sqrt(std::sqrt(chain * chain * chain * chain + adds * adds * adds * adds + meet * meet * meet * meet));
@@ -943,14 +944,15 @@ int hlbg_nn_conv3d_wgrad(const void* x, int32_t cin, const void* dy, int32_t cou
   const int64_t nbricks = (int64_t)n * nbz * nby * nbx;
   const int nci = cin % 32 == 0 ? 2 : 1;
   const int gy = cout / 16, gz = cin / (16 * nci);
-  // about four waves of 2 CTAs per SM over 152 SMs
-  const int64_t bpc = std::max<int64_t>(1, (nbricks * gy * gz + 1215) / 1216);
+  // about four waves of 2 CTAs per SM
+  const int sms = hlbg::sm_count();
+  const int64_t bpc = std::max<int64_t>(1, (nbricks * gy * gz + 8 * sms - 1) / (8 * sms));
   // The tcgen05 kernel where it is the faster one.  1x1x1: from 17 voxels on (us, mma.sync /
   // tcgen05, 96 -> 96: 8 voxels 2.7 / 3.5, 27 5.2 / 3.5, 4096 440 / 4).  3x3x3: by the
   // modelled times (96 -> 96: 96 x 3 x 3 voxels 17.0 / 25.0, 24^3 42 / 16).
   const int64_t M = (int64_t)n * d * h * wd;
   if (by16 && aligned16(x, dy, dw) && (taps == 27 || M > 16)) {
-    const double limit = taps == 27 ? wgrad_mma_time(cin, cout, nci, bpc, nbricks, gy * gz) : 0.0;
+    const double limit = taps == 27 ? wgrad_mma_time(cin, cout, nci, bpc, nbricks, gy * gz, sms) : 0.0;
     const int rc = hlbg_nn_wgrad_tc_within(x, cin, dy, cout, dw, n, d, h, wd, taps, stream, limit);
     if (rc != 1) return rc;
   }
@@ -1105,7 +1107,7 @@ int hlbg_nn_mse(const float* pred, const float* target, const float* mask, void*
                 int32_t c, float inv_count, void* stream) {
   if (c > 0 && c % 4 == 0 && m > 0 && m * c / 4 < 0x7fff0000ll && aligned16(pred, target, dpred)) {
     const uint32_t nv = (uint32_t)(m * c / 4);
-    const unsigned g = std::min(blocks((nv + 3) / 4), 1216u);  // 8 CTAs a SM; one atomic per CTA
+    const unsigned g = std::min(blocks((nv + 3) / 4), 8u * hlbg::sm_count());  // 8 CTAs a SM; one atomic per CTA
     launch_overlapped(k_mse_v4, g, 256, 0, (cudaStream_t)stream, (const float4*)pred, (const float4*)target, mask,
                       (uint2*)dpred, loss, nv, c / 4, inv_count);
     return check_launch();

@@ -65,6 +65,7 @@
 
 #include "../../include/hemelb_gb300_nn.h"
 #include "overlap.cuh"
+#include "sm_count.h"
 
 namespace {
 
@@ -599,7 +600,6 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 // Shared memory of an SM, what a CTA reserves and has as static arrays, and the most a
 // CTA may ask for on top of these.
 constexpr int kSmemSm = 233472, kSmemFixed = 1024 + 2048, kSmemDyn = 232448 - 2048;
-constexpr int kSms = 152;
 
 // Tile of a convolution (see TcParams) and the shared memory that goes with it.
 struct Plan {
@@ -635,15 +635,15 @@ bool conv_fit(int cin, int taps, int ct, int bz, int cols, int span, int tb, int
 // SM's TMA rows (kRow each) and bytes (loads and stores, kBytes a cycle) bound it from
 // below.  The constants are a fit to every plan of 37 layers (some 8,000 timings): the
 // plans it takes are 1 % slower than the best ones in the mean, 9 % at worst.
-double conv_time(int cin, int cout, int n, int d, int h, int wd, int taps, const Plan& pl) {
+double conv_time(int cin, int cout, int n, int d, int h, int wd, int taps, int sms, const Plan& pl) {
   constexpr double kIssue = 77.7, kTurn = 132.0, kLoad = 123.0, kLaunch = 11700.0, kStep = 258.0, kRow = 1.1,
                    kBytes = 27.0;
   const int slices = cin / 16, planes = pl.bz + (taps == 27 ? 2 : 0), per = 256 / pl.ct, k = taps == 27 ? 9 : 1;
   const int loads = (slices * 32 + pl.span - 1) / pl.span;
   const int columns = (d + pl.bz - 1) / pl.bz, ny = cout / pl.ct;
   const int64_t tiles = (int64_t)n * ((wd + 7) / 8) * ((h + 15) / 16) * ((columns + pl.cols - 1) / pl.cols);
-  const int64_t ctas = std::min<int64_t>(tiles, std::max(1, kSms * pl.per_sm / ny)) * ny;
-  const double resident = std::max(1.0, std::min((double)pl.per_sm, (double)ctas / kSms));
+  const int64_t ctas = std::min<int64_t>(tiles, std::max(1, sms * pl.per_sm / ny)) * ny;
+  const double resident = std::max(1.0, std::min((double)pl.per_sm, (double)ctas / sms));
   const double tiles_per_cta = std::ceil((double)(tiles * ny) / (double)ctas);
   double mma = 0, issue = 0;  // a column's planes, one slice
   for (int q = 0; q < planes; ++q) {
@@ -668,9 +668,9 @@ double conv_time(int cin, int cout, int n, int d, int h, int wd, int taps, const
 }
 
 // The tile with the smallest modelled time: output channels a multiple of 16 that
-// divides C_out (at most 256), every useful column height, one or two columns and sets
-// of accumulators, rows as wide as the channels allow or narrower (fewer bytes a plane).
-bool conv_plan(int cin, int cout, int n, int d, int h, int wd, int taps, Plan& best) {
+// divides C_out (at most 256), every useful column height, one to four columns, one
+// or two sets of accumulators, rows as wide as the channels allow or narrower (fewer bytes a plane).
+bool conv_plan(int cin, int cout, int n, int d, int h, int wd, int taps, int sms, Plan& best) {
   double best_t = 0;
   bool found = false;
   for (int ct = 16; ct <= std::min(cout, 256); ct += 16) {
@@ -685,7 +685,7 @@ bool conv_plan(int cin, int cout, int n, int d, int h, int wd, int taps, Plan& b
             for (int per_sm = 3; per_sm >= 1; --per_sm) {
               Plan pl;
               if (!conv_fit(cin, taps, ct, bz, cols, span, tb, per_sm, pl)) continue;
-              const double t = conv_time(cin, cout, n, d, h, wd, taps, pl);
+              const double t = conv_time(cin, cout, n, d, h, wd, taps, sms, pl);
               if (!found || t < best_t) {
                 found = true;
                 best_t = t;
@@ -699,21 +699,21 @@ bool conv_plan(int cin, int cout, int n, int d, int h, int wd, int taps, Plan& b
 }
 
 // conv_plan takes 10 to 40 us of host time, so each thread keeps the plans of the last
-// shapes it asked for (a fixed table, by the shape alone).
-bool planned(int cin, int cout, int n, int d, int h, int wd, int taps, Plan& pl) {
+// shapes it asked for (a fixed table, by the shape and the SMs).
+bool planned(int cin, int cout, int n, int d, int h, int wd, int taps, int sms, Plan& pl) {
   struct Entry {
-    int shape[7];
+    int shape[8];
     Plan plan;
   };
   static thread_local Entry table[64] = {};
-  const int shape[7] = {cin, cout, n, d, h, wd, taps};
+  const int shape[8] = {cin, cout, n, d, h, wd, taps, sms};
   uint32_t hash = 0;
   for (int v : shape) hash = hash * 2654435761u + (uint32_t)v;
   Entry& e = table[hash >> 26];
-  if (!std::equal(shape, shape + 7, e.shape)) {  // a zeroed entry has no valid shape
+  if (!std::equal(shape, shape + 8, e.shape)) {  // a zeroed entry has no valid shape
     Plan found;
-    if (!conv_plan(cin, cout, n, d, h, wd, taps, found)) return false;
-    std::copy(shape, shape + 7, e.shape);
+    if (!conv_plan(cin, cout, n, d, h, wd, taps, sms, found)) return false;
+    std::copy(shape, shape + 8, e.shape);
     e.plan = found;
   }
   pl = e.plan;
@@ -738,8 +738,9 @@ int hlbg_nn_conv3d_tc(const void* in, int32_t cin, const void* w, const float* b
     return 1;
   auto enc = encode_fn();
   if (!enc) return 3;
+  const int sms = hlbg::sm_count();
   Plan pl;
-  if (!planned(cin, cout, n, d, h, wd, taps, pl)) return 1;
+  if (!planned(cin, cout, n, d, h, wd, taps, sms, pl)) return 1;
   CUtensorMap tin, tw;
   {
     const cuuint64_t dims[5] = {(cuuint64_t)cin, (cuuint64_t)wd, (cuuint64_t)h, (cuuint64_t)d, (cuuint64_t)n};
@@ -806,7 +807,7 @@ int hlbg_nn_conv3d_tc(const void* in, int32_t cin, const void* w, const float* b
   }
   // persistent CTAs, as many as the SMs hold, over the tiles of each block of output channels
   const int ny = cout / pl.ct;
-  const unsigned gx = (unsigned)std::min<int64_t>(tiles, std::max(1, kSms * pl.per_sm / ny));
+  const unsigned gx = (unsigned)std::min<int64_t>(tiles, std::max(1, sms * pl.per_sm / ny));
   launch_overlapped(kernel, dim3(gx, (unsigned)ny), conv_threads(pl.cols), pl.smem, static_cast<cudaStream_t>(stream),
                     tin, tw, p);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;

@@ -414,9 +414,9 @@ auto wg_kernel(int wb, int zg, int taps) {
 // that its runs are many for what they add.  A 4-norm of the three over the launch's 2.77.
 // A fit to 742 shapes, 10 % in the mean; so is wgrad_mma_time's.  Of the two kernels the
 // faster one is chosen, or one within 5 %, for all but 25 of 754 other shapes (42 % at worst).
-double wgrad_tc_time(const WgPlan& pl, const WgParams& p, int64_t units, int64_t ctas) {
+double wgrad_tc_time(const WgPlan& pl, const WgParams& p, int64_t units, int64_t ctas, int sms) {
   const double per_cta = (double)((units + ctas - 1) / ctas);
-  const double resident = std::min((double)pl.per_sm, std::max(1.0, (double)units / kSms));
+  const double resident = std::min((double)pl.per_sm, std::max(1.0, (double)units / sms));
   const int n = 3 * pl.wb, sums = pl.zg * pl.groups;
   const double mma = p.run * sums * 8.0 * std::max(0.0394, 0.00072 * mma_cost(n) * resident);
   const double epi = 0.145 * (sums * n / 16);
@@ -435,6 +435,7 @@ int wgrad_tc(const void* x, int cin, const void* dy, int cout, float* dw, int n,
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dw)) & 15u) return 1;
   auto enc = encode_fn();
   if (!enc) return 3;
+  const int sms = hlbg::sm_count();
   WgPlan pl;
   if (!wg_plan(cin, cout, taps, pl)) return 1;
   WgParams p{};
@@ -465,10 +466,10 @@ int wgrad_tc(const void* x, int cin, const void* dy, int cout, float* dw, int n,
   // shared out evenly over whole waves of CTAs.  The tensor cores' sums lose about 2^-26
   // of themselves a step (16 -> 16 at 96^3, error against 64 bits: 184 steps 2.4e-6, 136
   // steps 1.6e-6, mma.sync's 184 2.2e-6), so the run decides the accuracy.
-  const int64_t blocks = (int64_t)p.na * p.nb * p.nzg, ctas = (int64_t)kSms * pl.per_sm;
+  const int64_t blocks = (int64_t)p.na * p.nb * p.nzg, ctas = (int64_t)sms * pl.per_sm;
   const int64_t bricks = (int64_t)n * ((d + 3) / 4) * ((h + 3) / 4) * ((wd + 7) / 8);
   const int64_t shares = (int64_t)(cout / 16) * (cin / (cin % 32 == 0 ? 32 : 16));
-  const int64_t theirs = taps == 27 ? (bricks * shares + 1215) / 1216 : 32;
+  const int64_t theirs = taps == 27 ? (bricks * shares + 8 * sms - 1) / (8 * sms) : 32;
   const int64_t most = theirs >= 16 ? theirs - theirs / 8 : std::max<int64_t>(1, theirs);
   const int64_t waves = std::max<int64_t>(1, (tiles * blocks + most * ctas - 1) / (most * ctas));
   int64_t run = (tiles * blocks + waves * ctas - 1) / (waves * ctas);
@@ -477,7 +478,7 @@ int wgrad_tc(const void* x, int cin, const void* dy, int cout, float* dw, int n,
   p.runs = (int)((tiles + run - 1) / run);
   const int64_t units = p.runs * blocks;
   if (units > 0x7fffffff) return 1;
-  if (taps == 27 && wgrad_tc_time(pl, p, units, std::min(units, ctas)) > limit) return 1;
+  if (taps == 27 && wgrad_tc_time(pl, p, units, std::min(units, ctas), sms) > limit) return 1;
   auto map = [&](CUtensorMap& m, const void* ptr, int c, int w, int bx, int by) {
     const cuuint64_t dims[5] = {(cuuint64_t)c, (cuuint64_t)wd, (cuuint64_t)h, (cuuint64_t)d, (cuuint64_t)n};
     const cuuint64_t strides[4] = {(cuuint64_t)c * 2, (cuuint64_t)c * 2 * wd, (cuuint64_t)c * 2 * wd * h,
