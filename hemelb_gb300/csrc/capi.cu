@@ -1080,7 +1080,7 @@ int graph_steps(hlbg_ctx* ctx, int n, bool check) {
 namespace {
 
 // Launch shape of a new context: the fluid list, which passes over what is solid.  FP64
-// (one shape of it): 670 us a step on the 1.46M-site bifurcation against 786 in all slots.
+// (one shape of it): 613 us a step on the 1.46M-site bifurcation against 701 in all slots.
 // FP32 and FP16: 128 x 9, the fastest of the list's shapes on every vessel tried with the
 // orders above (FP32 tree of 16.9M sites 512, 128 x 8 528, 64 x 16 525; bifurcation 64.7,
 // 68.1, 67.7; FP16 tree of 7.8M 229, 236, 233).

@@ -123,7 +123,7 @@ __device__ __forceinline__ int site_of_slot(const StepArgs& a, int64_t s, bool p
 }
 
 // HLBG_PUSH_FENCE=1: keep each push's lookup and store together (no hoisting of
-// the next direction's loads above this store).
+// the next direction's loads above this store), where pushes look their blocks up.
 #ifndef HLBG_PUSH_FENCE
 #define HLBG_PUSH_FENCE 0
 #endif

@@ -948,8 +948,8 @@ int hlbg_nn_conv3d_wgrad(const void* x, int32_t cin, const void* dy, int32_t cou
   const int sms = hlbg::sm_count();
   const int64_t bpc = std::max<int64_t>(1, (nbricks * gy * gz + 8 * sms - 1) / (8 * sms));
   // The tcgen05 kernel where it is the faster one.  1x1x1: from 17 voxels on (us, mma.sync /
-  // tcgen05, 96 -> 96: 8 voxels 2.7 / 3.5, 27 5.2 / 3.5, 4096 440 / 4).  3x3x3: by the
-  // modelled times (96 -> 96: 96 x 3 x 3 voxels 17.0 / 25.0, 24^3 42 / 16).
+  // tcgen05, 96 -> 96: 8 voxels 2.7 / 3.5, 27 5.2 / 3.5, 4,096 436 / 4).  3x3x3: by the
+  // modelled times (96 -> 96: 96 x 3 x 3 voxels 17.0 / 25.0, 24^3 50 / 25).
   const int64_t M = (int64_t)n * d * h * wd;
   if (by16 && aligned16(x, dy, dw) && (taps == 27 || M > 16)) {
     const double limit = taps == 27 ? wgrad_mma_time(cin, cout, nci, bpc, nbricks, gy * gz, sms) : 0.0;

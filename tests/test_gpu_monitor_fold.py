@@ -110,8 +110,8 @@ def test_nan_reaches_the_stats(blocks):
 def test_a_checked_step_of_a_large_run_costs_little_more_than_a_plain_one():
     """The velocities a check reads and writes are 24 bytes a site beside the update's
     152, and the step's time went from 7.55 to 9.51 ms with them on a vascular forest
-    (26 %) when the partials had launches of their own.  Folded by the update's CTAs they
-    took 42 % here; half way is the line."""
+    (26 %) when the partials had launches of their own.  Here it is 29 %, and was 45 % when
+    the update's CTAs folded them; half way is the line."""
     s = cases.tree(7, 512, 1, 6, 50.0, precision=capi.FP32DEV).solver()
     s.SetInitialConditions()
     s.SetLaunchVariant(6)
@@ -123,4 +123,4 @@ def test_a_checked_step_of_a_large_run_costs_little_more_than_a_plain_one():
         t = time.perf_counter()
         s.StepMonitored(40)
         checked.append((time.perf_counter() - t) / 40 * 1e3)
-    assert min(checked) < 1.34 * plain
+    assert min(checked) < 1.37 * plain
